@@ -22,20 +22,22 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
           "--expt-relaxed-constexpr", "-I" + INCLUDE]
 
-# translation unit -> extra flags
+# translation unit -> (source, extra flags); the stage kernels are compiled per reconstruction
+# (1 donor cell, 2 PLM, 3 PPM), so that no unit takes much longer than the others
 UNITS = {
-    "aph_capi.cu": [],
-    "aph_ghosts.cu": [],
-    "aph_fast.cu": [],
-    "aph_exact.cu": ["--fmad=false"],
-    "aph_stage_fast.cu": [],
-    "aph_stage_exact.cu": ["--fmad=false"],
-    "aph_stepper.cu": [],
-    "aph_adjoint.cu": [],
-    "aph_noalloc.cu": [],
-    "aph_history.cu": [],
-    "aph_diag.cu": ["--fmad=false"],
+    "aph_capi": ("aph_capi.cu", []),
+    "aph_ghosts": ("aph_ghosts.cu", []),
+    "aph_fast": ("aph_fast.cu", []),
+    "aph_exact": ("aph_exact.cu", ["--fmad=false"]),
+    "aph_stepper": ("aph_stepper.cu", []),
+    "aph_adjoint": ("aph_adjoint.cu", []),
+    "aph_noalloc": ("aph_noalloc.cu", []),
+    "aph_history": ("aph_history.cu", []),
+    "aph_diag": ("aph_diag.cu", ["--fmad=false"]),
 }
+for _r in (1, 2, 3):
+    UNITS["aph_stage_fast%d" % _r] = ("aph_stage_fast.cu", ["-DAPH_STAGE_RECON=%d" % _r])
+    UNITS["aph_stage_exact%d" % _r] = ("aph_stage_exact.cu", ["--fmad=false", "-DAPH_STAGE_RECON=%d" % _r])
 
 
 def nvcc():
@@ -57,9 +59,9 @@ def _sources_digest():
     return h.hexdigest()
 
 
-def _compile(unit, extra, verbose):
-    src = os.path.join(CSRC, unit)
-    obj = os.path.join(OBJDIR, unit.replace(".cu", ".o"))
+def _compile(unit, source, extra, verbose):
+    src = os.path.join(CSRC, source)
+    obj = os.path.join(OBJDIR, unit + ".o")
     cmd = [nvcc()] + ARCH + COMMON + extra + ["-c", src, "-o", obj]
     if verbose:
         cmd.insert(1, "-Xptxas=-v")
@@ -79,9 +81,9 @@ def build(force=False, verbose=False, jobs=None):
         with open(stamp) as f:
             if f.read().strip() == digest:
                 return LIB
-    units = [(u, e) for u, e in UNITS.items() if os.path.exists(os.path.join(CSRC, u))]
+    units = [(u, s, e) for u, (s, e) in UNITS.items()]
     with cf.ThreadPoolExecutor(max_workers=jobs or len(units)) as ex:
-        results = list(ex.map(lambda ue: _compile(ue[0], ue[1], verbose), units))
+        results = list(ex.map(lambda use: _compile(*use, verbose), units))
     if verbose:
         for obj, log in results:
             print(obj)

@@ -18,7 +18,7 @@ namespace aph {
 // The Jacobian depends on rho and v only, so it is evaluated from the primitives w.
 __device__ __forceinline__ void cons_to_prim_vjp(const double *w, const double *gw, double gm1,
                                                  double *gu) {
-  const double di = 1.0 / w[IDN];
+  const double di = rcp_x(w[IDN]);
   const double v1 = w[IV1], v2 = w[IV2], v3 = w[IV3];
   const double gp = gw[IPR];
   const double v2sum = v1 * v1 + v2 * v2 + v3 * v3;
@@ -38,7 +38,7 @@ __device__ __forceinline__ double plm_keep(double q_im1, double q_i, double q_ip
   const double dq2 = dql * dqr;
   double r = 0.0, dqm = 0.0;
   if (is_pos(dq2)) {
-    r = 1.0 / (dql + dqr);
+    r = rcp_x(dql + dqr);
     dqm = dq2 * r;
   }
   ql = q_i + dqm;
@@ -153,7 +153,7 @@ __device__ __forceinline__ void ppm_cell_code(double q_im2, double q_im1, double
     mx = a2 > mx ? a2 : mx;
     mx = a3 > mx ? a3 : mx;
     mx = a4 > mx ? a4 : mx;
-    if (mag(d2qf) > mag(1.0e-12 * from_bits(mx))) rho = qe / d2qf;
+    if (mag(d2qf) > mag(1.0e-12 * from_bits(mx))) rho = div_x(qe, d2qf);
     code |= src << 1;
     if (le(rho, 1.0 - 1.0e-12)) {
       qr = fma(-rho, dqf_minus, q_i);
@@ -190,7 +190,7 @@ __device__ __forceinline__ void ppm_cell_vjp(double q_i, double dph_lo, double d
       if (rho != 0.0 && src >= 1 && src <= 3) {  // rho = C2 d2(i + src - 2) / d2qf
         const double d2qf = 6.0 * (dph_lo + dph_hi - 2.0 * q_i);
         const double g_rho = gL * (dph_hi - q_i) - gR * (q_i - dph_lo);
-        const double g_qe = g_rho / d2qf;
+        const double g_qe = div_x(g_rho, d2qf);
         const double g_d2qf = -g_qe * rho;
         g_lo += 6.0 * g_d2qf;
         g_hi += 6.0 * g_d2qf;
@@ -266,7 +266,7 @@ __device__ __forceinline__ double side_flux_vjp(const double *w, double vx, doub
 __device__ void hlle_vjp(const double *wl, const double *wr, const GasConsts &gc, double ic2g,
                          const double *gf, double *gwl, double *gwr) {
   const double igm1 = gc.igm1;
-  const double ipl = 1.0 / wl[IPR], ipr = 1.0 / wr[IPR];
+  const double ipl = rcp_x(wl[IPR]), ipr = rcp_x(wr[IPR]);
   const SoundSpeed sl = sound_speed_d(wl[IDN], wl[IPR], ipl, gc, ic2g);
   const SoundSpeed sr = sound_speed_d(wr[IDN], wr[IPR], ipr, gc, ic2g);
   const double cl = sl.c, cr = sr.c;
@@ -299,7 +299,7 @@ __device__ void hlle_vjp(const double *wl, const double *wr, const GasConsts &gc
   fl[4] = el * vxl + wl[IPR] * wl[IV1];
   fr[4] = er * vxr + wr[IPR] * wr[IV1];
   const bool has = (mag(bp) | mag(bm)) != 0ULL;
-  const double ibpm = has ? 1.0 / (bp - bm) : 0.0;
+  const double ibpm = has ? rcp_x(bp - bm) : 0.0;
   const double tmp = has ? 0.5 * (bp + bm) * ibpm : 0.0;
   // reverse
   double gfl[5], gfr[5], gtmp = 0.0;
@@ -358,7 +358,7 @@ __device__ void hlle_vjp(const double *wl, const double *wr, const GasConsts &gc
 __device__ void hllc_vjp(const double *wl, const double *wr, const GasConsts &gc, double ic2g,
                          const double *gf, double *gwl, double *gwr) {
   const double igm1 = gc.igm1;
-  const double ipl = 1.0 / wl[IPR], ipr = 1.0 / wr[IPR];
+  const double ipl = rcp_x(wl[IPR]), ipr = rcp_x(wr[IPR]);
   const SoundSpeed sdl = sound_speed_d(wl[IDN], wl[IPR], ipl, gc, ic2g);
   const SoundSpeed sdr = sound_speed_d(wr[IDN], wr[IPR], ipr, gc, ic2g);
   const double cl = sdl.c, cr = sdr.c;
@@ -388,7 +388,7 @@ __device__ void hllc_vjp(const double *wl, const double *wr, const GasConsts &gc
   const double tr = pr + vxr * rr * ur;
   const double ml = rl * vxl;
   const double mr = -(rr * vxr);
-  const double imm = 1.0 / (ml + mr);
+  const double imm = rcp_x(ml + mr);
   const double sstar = (tl - tr) * imm;
   const double cp0 = (ml * tr + mr * tl) * imm;
   const bool cpos = is_pos(cp0);
@@ -410,7 +410,7 @@ __device__ void hllc_vjp(const double *wl, const double *wr, const GasConsts &gc
   fs[3] = ws[IDN] * ws[IV3] * wx;
   fs[4] = es * wx + ws[IPR] * ws[IV1];
   // c = sstar / (sstar - b), ustar = -b / (sstar - b)
-  const double idn = 1.0 / (sstar - b);
+  const double idn = rcp_x(sstar - b);
   const double cs = sstar * idn;
   const double ustar = -b * idn;
   double gfs[5], gcs = 0.0;

@@ -35,7 +35,9 @@ __global__ void k_exact_ops2(int op, const double *x, const double *y, double *o
     else if (op == 5) r = a / b;
     else if (op == 6) r = __drcp_rn(b);
     else if (op == 7) r = sqrt(a);
-    else r = div_rcp(a, b, __drcp_rn(b));
+    else if (op == 8) r = div_x(a, b);
+    else if (op == 9) r = rcp_x(b);
+    else r = sqrt_x(a);
     out[i] = r;
   }
 }
@@ -45,7 +47,7 @@ __global__ void k_exact_ops2(int op, const double *x, const double *y, double *o
 extern "C" aph_status aph_diag_exact_ops2(int op, const double *x, const double *y, double *out,
                                           long long n, void *stream) {
   clear_error();
-  if (op < 0 || op > 8) return fail(APH_ERR_INVALID, "op %d not in 0..8", op);
+  if (op < 0 || op > 10) return fail(APH_ERR_INVALID, "op %d not in 0..10", op);
   if (n < 0 || (n > 0 && (!x || !y || !out))) return fail(APH_ERR_INVALID, "NULL argument");
   if (n == 0) return APH_OK;
   const long long blocks = (n + 255) / 256;

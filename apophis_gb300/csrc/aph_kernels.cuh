@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kThreads) k_cons_to_prim(PackDev p, const Bloc
     B.gamma[nc + c] = g_e;
   }
   if (p.nvar > NHYDRO) {
-    const double di = 1.0 / u[IDN];
+    const double di = rcp_x(u[IDN]);
     for (int n = NHYDRO; n < p.nvar; ++n) B.prim[n * nc + c] = B.cons[n * nc + c] * di;
   }
   if (B.eos_lambda && B.eos_lambda[2 * nc + c] == 0.0) B.eos_lambda[2 * nc + c] = 7.0;  // hydro.cpp:491-493
@@ -169,8 +169,14 @@ __global__ void __launch_bounds__(kThreads) k_fluxes(PackDev p, const BlockDev *
     wl[IV3] = sL[ivz * vs + oL]; wl[IPR] = sL[IPR * vs + oL];
     wr[IDN] = sR[IDN * vs + oR]; wr[IV1] = sR[ivx * vs + oR]; wr[IV2] = sR[ivy * vs + oR];
     wr[IV3] = sR[ivz * vs + oR]; wr[IPR] = sR[IPR * vs + oR];
-    riemann<RS, false>(wl, wr, sL[nvar * vs + oL], sL[(nvar + 1) * vs + oL],
-                       sR[nvar * vs + oR], sR[(nvar + 1) * vs + oR], gc, flx);
+    const double glc = sL[nvar * vs + oL], gle = sL[(nvar + 1) * vs + oL];
+    const double grc = sR[nvar * vs + oR], gre = sR[(nvar + 1) * vs + oR];
+    IntOps o;
+    riemann<RS, false, false>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+    if (!o.ok()) {  // an operand outside the integer pipe's range
+      IeeeOps ieee;
+      riemann<RS, false, false>(wl, wr, glc, gle, grc, gre, gc, flx, ieee);
+    }
     flux[IDN * fn + fcell] = flx[IDN];
     flux[ivx * fn + fcell] = flx[IV1];
     flux[ivy * fn + fcell] = flx[IV2];
@@ -211,7 +217,7 @@ __global__ void __launch_bounds__(kThreads) k_update(PackDev p, const BlockDev *
   if (!interior_cell(B, p.ndim, p.ng, blockIdx.x * blockDim.x + threadIdx.x, c, ci, cj, ck)) return;
   const double beta_dt = dt_dev ? beta * dt_dev[0] : beta_dt_host;
   const double a1 = B.dx[1] * B.dx[2], a2 = B.dx[0] * B.dx[2], a3 = B.dx[0] * B.dx[1];
-  const double vol = B.dx[0] * B.dx[1] * B.dx[2];
+  const Den vol = den(B.dx[0] * B.dx[1] * B.dx[2]);
   const long long nc = B.ncell;
   for (int n = 0; n < p.nvar; ++n) {
     const long long q = n * nc + c;
@@ -225,7 +231,7 @@ __global__ void __launch_bounds__(kThreads) k_update(PackDev p, const BlockDev *
       const long long f3 = flux_index(B, 2, n, ck, cj, ci);
       du += (a3 * B.flux[2][f3 + B.fs[2][1]] - a3 * B.flux[2][f3]);
     }
-    const double div = -du / vol;
+    const double div = div_x(-du, vol);
     B.cons[q] = gam0 * B.cons[q] + gam1 * B.u1[q] + beta_dt * div;
   }
 }
@@ -250,7 +256,7 @@ __global__ void __launch_bounds__(kThreads) k_update_amr(PackDev p, const BlockD
   const int ii = idx % B.nx[0], jj = idx / B.nx[0];
   const double beta_dt = dt_dev ? beta * dt_dev[0] : beta_dt_host;
   const double a1 = B.dx[1] * B.dx[2], a2 = B.dx[0] * B.dx[2];
-  const double vol = B.dx[0] * B.dx[1] * B.dx[2];
+  const Den vol = den(B.dx[0] * B.dx[1] * B.dx[2]);
   const long long nc = B.ncell;
   for (int n = 0; n < p.nvar; ++n) {
     const long long q = n * nc + c;
@@ -274,7 +280,7 @@ __global__ void __launch_bounds__(kThreads) k_update_amr(PackDev p, const BlockD
       const double Fnew = 0.5 * (F.flux[d][g0] + F.flux[d][g1]);
       du = s == 0 ? du + (area * Fold - area * Fnew) : du + (area * Fnew - area * Fold);
     }
-    const double div = -du / vol;
+    const double div = div_x(-du, vol);
     B.cons[q] = gam0 * B.cons[q] + gam1 * B.u1[q] + beta_dt * div;
   }
 }

@@ -110,37 +110,25 @@ __device__ __forceinline__ double twice_x(double x) {
   const long long b = __double_as_longlong(x);
   return (b << 1) == 0 ? x : __longlong_as_double(b + (1LL << 52));
 }
-// x / 6.0 correctly rounded, on the integer pipe: with the significand M (leading 1 moved to
-// bit 63), floor(M / 3) is the high word of M * 0xAAAAAAAAAAAAAAAB shifted right once (the
-// exact quotient by an invariant divisor, Granlund and Montgomery), the remainder M - 3 floor
-// gives one more exact bit where the quotient is one bit short and a sticky bit, and the
-// quotient is rounded to nearest even (x / 6 is never a midpoint: a midpoint times 6 would need
-// more than 53 significant bits).  Valid for x zero or normal with 2^-1000 < |x| < 2^1000.
+// x / 6.0 correctly rounded, on the integer pipe: x / 6 = (x / 3) / 2, and with the significand
+// moved left by one or two bits to N, the quotient's significand is the integer nearest N / 3,
+// which is floor((N + 1) / 3) (N / 3 is never halfway).  2^30 is 1 modulo 3, so for
+// N + 1 = H 2^30 + L that is H (2^30 - 1) / 3 + floor((H + L) / 3).  Valid for x zero or normal with
+// 2^-1000 < |x| < 2^1000.  9 SM-cycles per warp on GB300 (26 in an earlier form built on
+// __umul64hi; a DADD takes 17).
 __device__ __forceinline__ double div6_x(double x) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const unsigned long long mg = u & 0x7fffffffffffffffULL;
-  if (mg == 0) return x;  // +-0 / 6 = +-0
-  const unsigned long long N = ((mg & 0xfffffffffffffULL) | 0x10000000000000ULL) << 11;
-  const unsigned long long Q = __umul64hi(N, 0xAAAAAAAAAAAAAAABULL) >> 1;  // floor(N / 3)
-  const unsigned long long R = N - 3ULL * Q;                                 // 0, 1 or 2
-  unsigned long long V;
-  long long e = (long long)(mg >> 52);
-  if (Q >> 62) {  // leading 1 at bit 62
-    V = Q;
-    e -= 2;
-  } else {        // at bit 61: append the next exact bit of N / 3
-    V = 2ULL * Q + (R == 2ULL ? 1ULL : 0ULL);
-    e -= 3;
-  }
-  unsigned long long m = V >> 10;
-  const unsigned long long r = V & 0x3ffULL;
-  if (r > 0x200ULL || (r == 0x200ULL && (R != 0ULL || (m & 1ULL)))) ++m;
-  if (m >> 53) {
-    m >>= 1;
-    ++e;
-  }
-  return __longlong_as_double(
-      (long long)((u & 0x8000000000000000ULL) | ((unsigned long long)e << 52) | (m & 0xfffffffffffffULL)));
+  const unsigned hi = (unsigned)(u >> 32);
+  const unsigned top = (hi >> 19) & 1u;  // the significand is 1.5 or more
+  const unsigned long long M = (u & 0xfffffffffffffULL) | 0x10000000000000ULL;
+  const unsigned long long N = (top ? M << 1 : M << 2) + 1;
+  const unsigned L = (unsigned)N & 0x3fffffffu, H = (unsigned)(N >> 30);
+  const unsigned long long m =
+      (unsigned long long)H * 0x15555555u + (__umulhi(H + L, 0xAAAAAAABu) >> 1);
+  // the exponent falls by 3 (2 if top), and m's leading bit adds one
+  const unsigned e = (hi & 0xfff00000u) - (4u - top) * 0x100000u;
+  const unsigned long long r = m + ((unsigned long long)e << 32);
+  return __longlong_as_double((long long)((u << 1) == 0 ? u : r));  // +-0 / 6 = +-0
 }
 
 // ---- IEEE double additions and small multiplications on the integer pipe ---------------
@@ -212,17 +200,184 @@ __device__ __forceinline__ double sub_x(double a, double b) {
   return add_x(a, __longlong_as_double(__double_as_longlong(b) ^ (long long)0x8000000000000000ULL));
 }
 
-// RN(k * x) for k = C * 2^S2 with a small odd integer C (3: k = 3 or 6; 5: k = 1.25)
+// RN(k * x) for k = C * 2^S2 with C = 3 (k = 3 or 6) or C = 5 (k = 1.25): the product of the
+// significand and C is one or two (C = 5: two or three) bits longer than a significand.
 template <int C, int S2>
 __device__ __forceinline__ double mulk_x(double x) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const unsigned long long m = u & 0x7fffffffffffffffULL;
-  if (m == 0) return x;  // k * +-0 = +-0
-  const unsigned long long P = ((m & 0xfffffffffffffULL) | 0x10000000000000ULL) * (unsigned long long)C;
-  const int sh = __clzll((long long)P) - 1;  // leading 1 to bit 62
-  // P << sh holds the value's significand in bits 62..10: exponent field E + 10 + S2 - sh
-  const long long e = (long long)(m >> 52) + 10 + S2 - sh;
-  return round_pack_x(u & 0x8000000000000000ULL, e, P << sh);
+  const unsigned hi = (unsigned)(u >> 32);
+  const unsigned long long P =
+      ((u & 0xfffffffffffffULL) | 0x10000000000000ULL) * (unsigned long long)C;
+  constexpr int s0 = C == 5 ? 2 : 1;
+  const unsigned longer = (unsigned)(P >> (53 + s0));  // 0 or 1
+  const unsigned sh = s0 + longer;
+  const unsigned long long m = (P + ((1ULL << (sh - 1)) - 1 + ((P >> sh) & 1))) >> sh;  // to even
+  const unsigned e = (hi & 0xfff00000u) + (unsigned)(s0 + S2 - 1 + (int)longer) * 0x100000u;
+  const unsigned long long r = m + ((unsigned long long)e << 32);
+  return __longlong_as_double((long long)((u << 1) == 0 ? u : r));  // k * +-0 = +-0
+}
+
+// ---- correctly rounded quotients, reciprocals and square roots on the integer pipe ------
+// GB300 spends 144 SM-cycles per warp on an IEEE double division and 151 on a square root (8-9
+// instructions of a pipe that takes 17 cycles each).  The digit recurrences below take 20 cycles
+// per warp in 32-bit integer instructions and give the same bits: a 32-bit reciprocal (or
+// reciprocal square root) word from the hardware's FP32 approximation and one Newton step, the
+// quotient's (root's) first ~30 bits by a multiplication with that word, the exact 64-bit
+// remainder, the remaining bits the same way, and one correction by the exact final remainder.
+// (Long division with an approximate reciprocal: D. E. Knuth, TAOCP 2, 4.3.1; Newton's iteration
+// for 1/b and 1/sqrt(x).)  54 bits come out, the last one being the round bit: a quotient or
+// root of doubles is never halfway between two doubles, so adding it rounds to nearest.
+__device__ __forceinline__ unsigned long long mulw(unsigned a, unsigned b) {
+  return (unsigned long long)a * (unsigned long long)b;
+}
+__device__ __forceinline__ unsigned long long significand(unsigned long long u) {
+  return (u & 0xfffffffffffffULL) | 0x10000000000000ULL;
+}
+
+// R = Y - d, 1 <= d < 5, for Y = 2^84 / B and a significand B.  With y = 2^52 / B (1/2 < y <= 1)
+// and f = B / 2^52 cut to 24 bits, the approximation (relative error 2^-23) lowered by 5 units of
+// 2^-24, and kept at or above 1/2, is y0 in [y - 7 2^-24, y]; the Newton step y0 (2 - y0 / y)
+// leaves (y - y0)^2 / y < 2^-41 plus at most two units of 2^-32 for B's dropped bits (upwards) and
+// one for the cut products (downwards); 3 is subtracted so that R < Y, also modulo 2^32.
+__device__ __forceinline__ unsigned rcp_word(unsigned long long B) {
+  const unsigned b1 = (unsigned)(B >> 21);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(0x3f800000u | ((b1 >> 8) & 0x7fffffu))));
+  const unsigned rb = max(__float_as_uint(r) - 5u, 0x3f000000u);
+  const unsigned R0 = (rb << 8) | 0x80000000u;
+  const unsigned eh = (unsigned)((0x8000000000000000ULL - mulw(R0, b1)) >> 16);
+  return R0 + (unsigned)(mulw(R0, eh) >> 47) - 3u;
+}
+
+// RN(a / b) from the bits of a and b, both normal with a normal quotient; R = rcp_word of b's
+// significand.  With A the numerator's significand moved so that B <= A < 2B, q1 is at most 7
+// below A 2^30 / B (cut operands 1 + 5, floor 1), so the remainder r1 < 7 B < 2^56, and q2 falls
+// short of the integer part of r1 2^23 / B by at most one (cut operands 0.2, floors 1), which the
+// remainder r2 shows.
+__device__ __forceinline__ double quot_bits(unsigned long long ua, unsigned long long ub, unsigned R) {
+  unsigned long long A = significand(ua);
+  const unsigned long long B = significand(ub);
+  const unsigned less = A < B ? 1u : 0u;
+  A <<= less;
+  const unsigned q1 = __umulhi((unsigned)(A >> 22), R);
+  const unsigned long long r1 = (A << 30) - (unsigned long long)q1 * B;
+  unsigned q2 = __umulhi((unsigned)(r1 >> 24), R) >> 5;
+  const unsigned long long r2 = (r1 << 23) - (unsigned long long)q2 * B;
+  q2 += r2 >= B ? 1u : 0u;
+  const unsigned long long m = (((unsigned long long)q1 << 23) + q2 + 1) >> 1;  // 53 bits, rounded
+  const unsigned e = ((unsigned)(ua >> 52) & 0x7ffu) - ((unsigned)(ub >> 52) & 0x7ffu) + 1022u - less;
+  return __longlong_as_double(
+      (long long)((m + ((unsigned long long)(e << 20) << 32)) | ((ua ^ ub) & 0x8000000000000000ULL)));
+}
+
+// RN(sqrt(x)) for x normal and positive.  With x = X 4^k, 1 <= X < 4, M = X 2^52 and y = 1/sqrt(X):
+// the approximation (relative error 2^-22.9) of X cut to 24 bits, lowered by 4 units of 2^-24, is
+// y0 in [y - 6.2 2^-24, y]; the Newton step y0 (3 - X y0^2) / 2 leaves 1.5 (y - y0)^2 / y < 2^-41, up to
+// 4 units of 2^-32 upwards for the cut products and one down, so R = Y - d, 1 <= d < 6.2, for
+// Y = y 2^32.  s1 is at most 8.1 below sqrt(X) 2^30, the remainder r1 = M 2^8 - s1^2 < 2^35.1, and s2
+// (ignoring s2^2: at most 0.3 low) at most 1.6 below the rest of the 54-bit root: r2, the remainder
+// of M 2^54, shows whether one more fits.
+__device__ __forceinline__ double sqrt_bits(unsigned long long u) {
+  const unsigned e = (unsigned)(u >> 52);
+  const unsigned odd = (e & 1u) ^ 1u;  // e - 1023 is odd
+  const unsigned long long M = significand(u) << odd;
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;"
+      : "=f"(r)
+      : "f"(__uint_as_float((odd ? 0x40000000u : 0x3f800000u) | ((unsigned)(u >> 29) & 0x7fffffu))));
+  const unsigned rb = max(__float_as_uint(r) - 4u, 0x3f000000u);
+  const unsigned R0 = (rb << 8) | 0x80000000u;
+  const unsigned x1 = (unsigned)(M >> 22);
+  const unsigned eh = (unsigned)((0x4000000000000000ULL - mulw(x1, __umulhi(R0, R0))) >> 16);
+  const unsigned R = R0 + (unsigned)(mulw(R0, eh) >> 47) - 5u;
+  const unsigned s1 = __umulhi(x1, R);
+  const unsigned long long r1 = (M << 8) - mulw(s1, s1);
+  const unsigned s2 = (unsigned)(mulw((unsigned)(r1 >> 4), R) >> 36);
+  const unsigned long long r2 = (((r1 << 22) - mulw(s1, s2)) << 24) - mulw(s2, s2);
+  const unsigned long long S = ((unsigned long long)s1 << 23) + s2;
+  const unsigned long long m = (S + 1 + (r2 > 2 * S ? 1u : 0u)) >> 1;
+  return __longlong_as_double((long long)(m + ((unsigned long long)((e + 1022u - odd) >> 1) << 52)));
+}
+
+// How far x's exponent field lies above 2^-400's; more than kFar above: x is outside
+// 2^-400 .. 2^401 (zero, infinite and NaN included; signed: also where x is negative).  Quotients,
+// products of two and roots of values inside are normal.
+constexpr unsigned kFar = 800u;
+__device__ __forceinline__ unsigned far_of(double x) {
+  return (((unsigned)__double2hiint(x) & 0x7fffffffu) >> 20) - 623u;
+}
+__device__ __forceinline__ unsigned far_of_signed(double x) {
+  return ((unsigned)__double2hiint(x) >> 20) - 623u;
+}
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+
+// A denominator and its reciprocal word, which several quotients may share.
+struct Den {
+  double b;
+  unsigned R;
+};
+
+// The operations of a Riemann solve on the integer pipe, unchecked and free of branches: far
+// collects the largest distance over all operands, and the caller takes the whole solve again
+// with IeeeOps where it exceeds kFar.  div0 allows a numerator of zero.
+struct IntOps {
+  unsigned far = 0;
+  __device__ __forceinline__ Den den(double b) {
+    far = max(far, far_of(b));
+    return Den{b, rcp_word(significand((unsigned long long)__double_as_longlong(b)))};
+  }
+  __device__ __forceinline__ double div(double a, const Den &d) {
+    far = max(far, far_of(a));
+    return quot_bits((unsigned long long)__double_as_longlong(a),
+                     (unsigned long long)__double_as_longlong(d.b), d.R);
+  }
+  __device__ __forceinline__ double div0(double a, const Den &d) {
+    const bool z = is_zero(a);
+    far = max(far, z ? 0u : far_of(a));
+    const unsigned long long ua = (unsigned long long)__double_as_longlong(a);
+    const unsigned long long ub = (unsigned long long)__double_as_longlong(d.b);
+    const double q = quot_bits(ua, ub, d.R);
+    return z ? __longlong_as_double((long long)((ua ^ ub) & 0x8000000000000000ULL)) : q;
+  }
+  __device__ __forceinline__ double div(double a, double b) { return div(a, den(b)); }
+  __device__ __forceinline__ double rcp(double b) { return div(1.0, den(b)); }
+  __device__ __forceinline__ double sqrt(double x) {
+    far = max(far, far_of_signed(x));
+    return sqrt_bits((unsigned long long)__double_as_longlong(x));
+  }
+  __device__ __forceinline__ bool ok() const { return far <= kFar; }
+};
+struct IeeeOps {
+  __device__ __forceinline__ Den den(double b) { return Den{b, 0u}; }
+  __device__ __forceinline__ double div(double a, const Den &d) { return __ddiv_rn(a, d.b); }
+  __device__ __forceinline__ double div0(double a, const Den &d) { return __ddiv_rn(a, d.b); }
+  __device__ __forceinline__ double div(double a, double b) { return __ddiv_rn(a, b); }
+  __device__ __forceinline__ double rcp(double b) { return __drcp_rn(b); }
+  __device__ __forceinline__ double sqrt(double x) { return __dsqrt_rn(x); }
+  __device__ __forceinline__ bool ok() const { return true; }
+};
+
+// Single operations for any operands: the digits, or the IEEE instruction where an operand is far
+// (a branch: predicating the instruction instead leaves its whole FP64 sequence in the path, which
+// cost the fast stage kernel 15 %).
+__device__ __forceinline__ Den den(double b) {
+  return Den{b, rcp_word(significand((unsigned long long)__double_as_longlong(b)))};
+}
+__device__ __forceinline__ double div_x(double a, const Den &d) {
+  IntOps o;
+  const double q = o.div0(a, d);
+  if (max(o.far, far_of(d.b)) > kFar) return __ddiv_rn(a, d.b);
+  return q;
+}
+__device__ __forceinline__ double div_x(double a, double b) { return div_x(a, den(b)); }
+__device__ __forceinline__ double rcp_x(double b) {
+  if (far_of(b) > kFar) return __drcp_rn(b);
+  return quot_bits(0x3ff0000000000000ULL, (unsigned long long)__double_as_longlong(b), den(b).R);
+}
+__device__ __forceinline__ double sqrt_x(double x) {
+  if (is_zero(x)) return x;
+  if (far_of_signed(x) > kFar) return __dsqrt_rn(x);
+  return sqrt_bits((unsigned long long)__double_as_longlong(x));
 }
 
 // ---- gamma-dependent constants of a pack (fast mode) ---------------------------
@@ -235,43 +390,10 @@ struct GasConsts {
 };
 
 // ---- ideal gas (singularity-eos IdealGas) ------------------------------------
-__device__ __forceinline__ double eos_pressure(double gm1, double rho, double sie) {
-  const double p = gm1 * rho * sie;
-  return is_neg(p) ? 0.0 : p;
-}
 __device__ __forceinline__ double eos_bulk_modulus(double gm1, double rho, double sie) {
   const double small = 10.0 * 2.2250738585072014e-308;
   const double b = gm1 * (gm1 + 1.0) * rho * sie;
   return lt(small, b) ? b : small;
-}
-
-// RN(a / b) given y = RN(1 / b), by Markstein's theorem (P. W. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Develop. 34(1),
-// 1990, Theorem 1): q = RN(a y) lies within one ulp of a / b, so the remainder a - b q is
-// exact (one fused multiply-add), and RN(q + (a - b q) y) is the correctly rounded quotient.
-// For a and b tame (b nonzero), where no product or remainder leaves the normal range; a zero
-// remainder means q = a / b exactly (and keeps the sign of a zero quotient).
-__device__ __forceinline__ double div_rcp(double a, double b, double y) {
-  const double q = __dmul_rn(a, y);
-  if ((((unsigned)__double2hiint(a) & 0x7fffffffu) | (unsigned)__double2loint(a)) == 0u) return q;
-  return __fma_rn(__fma_rn(-q, b, a), y, q);  // a nonzero: q nonzero, and q + (+-0) == q
-}
-
-// a / b correctly rounded, from y = RN(1 / b) where a and b allow it (the division otherwise).
-__device__ __forceinline__ double div_y(double a, double b, double y) {
-  return (tame(a) && tame_nz(b)) ? div_rcp(a, b, y) : a / b;
-}
-
-// a1 / b and a2 / b correctly rounded, sharing one reciprocal where the operands allow.
-__device__ __forceinline__ void div2(double a1, double a2, double b, double &q1, double &q2) {
-  if (tame(a1) && tame(a2) && tame_nz(b)) {
-    const double y = __drcp_rn(b);
-    q1 = div_rcp(a1, b, y);
-    q2 = div_rcp(a2, b, y);
-  } else {
-    q1 = a1 / b;
-    q2 = a2 / b;
-  }
 }
 
 // The reference's ConsToPrim arithmetic after the density floor (hydro.cpp:502-531), one
@@ -279,15 +401,16 @@ __device__ __forceinline__ void div2(double a1, double a2, double b, double &q1,
 // FMAs, and these values must match the reference bit for bit where they feed the
 // discontinuous PPM limiters (the adiabatic-index fields of blocks where a floor fired, which
 // the fast mode otherwise replaces by the constants) or the non-idempotent pressure floor.
-// u_d: the floored density, di = 1 / u_d.  Sets u[IEN], w[IPR], g_c, g_e; returns whether
-// the pressure floor fired.
+// u_d: the floored density (rho the same as a denominator), di = 1 / u_d.  Sets u[IEN], w[IPR],
+// g_c, g_e; returns whether the pressure floor fired.
 __device__ __forceinline__ bool cons_to_prim_tail(double *u, double *w, double &g_c, double &g_e,
-                                                  double u_d, double di, double gm1, double pfloor) {
+                                                  double u_d, const Den &rho, double di, double gm1,
+                                                  double pfloor) {
   const double m1 = u[IM1], m2 = u[IM2], m3 = u[IM3];
   const double e_k = __dmul_rn(__dmul_rn(0.5, di),
                                __dadd_rn(__dadd_rn(__dmul_rn(m1, m1), __dmul_rn(m2, m2)), __dmul_rn(m3, m3)));
   double u_e = u[IEN];
-  double sie = div_y(__dsub_rn(u_e, e_k), u_d, di);  // (u_e - e_k) / u_d
+  double sie = div_x(__dsub_rn(u_e, e_k), rho);
   double w_p = __dmul_rn(__dmul_rn(gm1, u_d), sie);
   w_p = is_neg(w_p) ? 0.0 : w_p;  // eos_pressure
   const bool floored = !gt(w_p, pfloor);
@@ -295,15 +418,15 @@ __device__ __forceinline__ bool cons_to_prim_tail(double *u, double *w, double &
     const double gm1q = __ddiv_rn(w_p, __dmul_rn(u_d, e_k));  // hydro.cpp:517
     u_e = __dadd_rn(__ddiv_rn(pfloor, gm1q), e_k);
     w_p = pfloor;
-    sie = div_y(__dsub_rn(u_e, e_k), u_d, di);  // of the floored energy (unchanged otherwise)
+    sie = div_x(__dsub_rn(u_e, e_k), rho);  // of the floored energy (unchanged otherwise)
   }
   u[IEN] = u_e;
   w[IPR] = w_p;
   const double small = 10.0 * 2.2250738585072014e-308;
   double b = __dmul_rn(__dmul_rn(__dmul_rn(gm1, __dadd_rn(gm1, 1.0)), u_d), sie);  // eos_bulk_modulus
   b = lt(small, b) ? b : small;
-  g_c = __ddiv_rn(b, w_p);
-  g_e = __dadd_rn(__ddiv_rn(w_p, __dsub_rn(u_e, e_k)), 1.0);
+  g_c = div_x(b, w_p);
+  g_e = __dadd_rn(div_x(w_p, __dsub_rn(u_e, e_k)), 1.0);
   return floored;
 }
 
@@ -316,7 +439,8 @@ __device__ __forceinline__ bool cons_to_prim_cell(double *u, double *w, double &
   const bool dens_ok = gt(u_d, dfloor);
   u_d = dens_ok ? u_d : dfloor;
   u[IDN] = u_d;
-  const double di = __drcp_rn(u_d);  // the correctly rounded 1.0 / u_d
+  const Den rho = den(u_d);
+  const double di = div_x(1.0, rho);
   w[IDN] = u_d;
   w[IV1] = u[IM1] * di;
   w[IV2] = u[IM2] * di;
@@ -326,8 +450,9 @@ __device__ __forceinline__ bool cons_to_prim_cell(double *u, double *w, double &
   // adiabatic indices are gamma (B / p = gm1 + 1 = p / (rho e) + 1), so one division per cell
   // (a floored density takes the reference's arithmetic below, whose indices are kept)
   if (dens_ok) {
-    const double e_k = 0.5 * di * (u[IM1] * u[IM1] + u[IM2] * u[IM2] + u[IM3] * u[IM3]);
-    const double pe = gm1 * (u[IEN] - e_k);
+    const double pe =
+        __dmul_rn(gm1, fma(-__dmul_rn(0.5, di),
+                           fma(u[IM3], u[IM3], fma(u[IM1], u[IM1], __dmul_rn(u[IM2], u[IM2]))), u[IEN]));
     const double wp = is_neg(pe) ? 0.0 : pe;
     if (gt(wp, pfloor)) {
       w[IPR] = wp;
@@ -337,14 +462,15 @@ __device__ __forceinline__ bool cons_to_prim_cell(double *u, double *w, double &
     }
   }
 #endif
-  return cons_to_prim_tail(u, w, g_c, g_e, u_d, di, gm1, pfloor);
+  return cons_to_prim_tail(u, w, g_c, g_e, u_d, rho, di, gm1, pfloor);
 }
 
 // The reference's adiabatic indices (gamma_c, gamma_e) of a cell whose floors did not fire,
 // from its conserved state after ConsToPrim (u: the cell's five values).
 __device__ __forceinline__ void gamma_ref(const double *u, double gm1, double &g_c, double &g_e) {
   double uu[NHYDRO] = {u[0], u[1], u[2], u[3], u[4]}, w[NHYDRO];
-  cons_to_prim_tail(uu, w, g_c, g_e, u[IDN], 1.0 / u[IDN], gm1, -1.0);
+  const Den rho = den(u[IDN]);
+  cons_to_prim_tail(uu, w, g_c, g_e, u[IDN], rho, div_x(1.0, rho), gm1, -1.0);
 }
 
 // ---- reconstruction (src/recon) --------------------------------------------------
@@ -354,7 +480,7 @@ __device__ __forceinline__ void plm(double q_im1, double q_i, double q_ip1, doub
   const double dqr = q_ip1 - q_i;
   const double dq2 = dql * dqr;
   double dqm = 0.0;
-  if (is_pos(dq2)) dqm = dq2 / (dql + dqr);
+  if (is_pos(dq2)) dqm = div_x(dq2, dql + dqr);
   ql_ip1 = q_i + dqm;
   qr_i = q_i - dqm;
 }
@@ -373,7 +499,7 @@ __device__ __forceinline__ void plm(double q_im1, double q_i, double q_ip1, doub
 template <bool TAME = false>
 __device__ __forceinline__ double ppm_dd(double qm1, double q0, double qp1) {
 #if APH_EXACT
-  if (TAME) return add_x(half_x(sub_x(qp1, q0)), half_x(sub_x(q0, qm1)));
+  if (TAME) return half_x(qp1 - q0) + half_x(q0 - qm1);
   return 0.5 * (qp1 - q0) + 0.5 * (q0 - qm1);
 #else
   return 0.5 * (qp1 - qm1);  // the same quantity with one rounding
@@ -381,7 +507,7 @@ __device__ __forceinline__ double ppm_dd(double qm1, double q0, double qp1) {
 }
 template <bool TAME = false>
 __device__ __forceinline__ double ppm_d2(double qm1, double q0, double qp1) {
-  if (APH_EXACT && TAME) return sub_x(add_x(qm1, qp1), twice_x(q0));
+  if (APH_EXACT && TAME) return (qm1 + qp1) - twice_x(q0);
   return (qm1 + qp1) - 2.0 * q0;
 }
 // Face between cells c-1 (value qm1) and c (value q0): ddm1 = dd(c-1), dd0 = dd(c),
@@ -391,20 +517,23 @@ __device__ __forceinline__ double ppm_face(double qm1, double q0, double ddm1, d
                                            double d2m1, double d20) {
 #if APH_EXACT
   if (TAME) {
-    const double s = add_x(qm1, q0);  // the additions and the x3, x5/4 scalings on the integer pipe
+    const double s = qm1 + q0;
     const double avg = half_x(s);
-    double dph = add_x(avg, div6_x(sub_x(ddm1, dd0)));
-    const double qa = mulk_x<3, 0>(sub_x(s, twice_x(dph)));
-    double qd = 0.0;
-    const bool sa = is_neg(qa);
-    if (sa == is_neg(d2m1) && sa == is_neg(d20)) {
-      const unsigned long long mb = mag(d2m1), mc = mag(d20);
-      const double m = mulk_x<5, -2>(from_bits(mc < mb ? mc : mb));  // PPM_C2 = 5/4
-      const unsigned long long mm = mag(m), ma = mag(qa);
-      qd = flip_if(from_bits(ma < mm ? ma : mm), sa);
+    double dph = avg + div6_x(ddm1 - dd0);
+    // (dph - qm1) * (q0 - dph) < 0, the differences being nonzero and their product normal; the
+    // limited value, which only such a face takes, is formed there
+    if (strictly_outside(dph, qm1, q0)) {
+      const double qa = mulk_x<3, 0>(s - twice_x(dph));
+      double qd = 0.0;
+      const bool sa = is_neg(qa);
+      if (sa == is_neg(d2m1) && sa == is_neg(d20)) {
+        const unsigned long long mb = mag(d2m1), mc = mag(d20);
+        const double m = mulk_x<5, -2>(from_bits(mc < mb ? mc : mb));  // PPM_C2 = 5/4
+        const unsigned long long mm = mag(m), ma = mag(qa);
+        qd = flip_if(from_bits(ma < mm ? ma : mm), sa);
+      }
+      dph = avg - div6_x(qd);
     }
-    // (dph - qm1) * (q0 - dph) < 0, the differences being nonzero and their product normal
-    if (strictly_outside(dph, qm1, q0)) dph = sub_x(avg, div6_x(qd));
     return dph;
   }
 #endif
@@ -445,11 +574,9 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
                                          double dph_lo, double dph_hi, double &ql_ip1,
                                          double &qr_i) {
   constexpr bool T = APH_EXACT && TAME;
-  const double d2qf = T ? mulk_x<3, 1>(sub_x(add_x(dph_lo, dph_hi), twice_x(q_i)))
-                        : 6.0 * (dph_lo + dph_hi - 2.0 * q_i);
   double qr = dph_lo, ql = dph_hi;
-  const double dqf_minus = T ? sub_x(q_i, qr) : q_i - qr;
-  const double dqf_plus = T ? sub_x(ql, q_i) : ql - q_i;
+  const double dqf_minus = q_i - qr;
+  const double dqf_plus = ql - q_i;
 #if APH_EXACT
   bool extremum;
   if (T) {  // the two products' signs, as in ppm_face
@@ -464,6 +591,7 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
   if (!strictly_between(qr, q_i, ql) || !strictly_between(q_im1, q_i, q_ip1)) {
 #endif
     // local extremum: limit with rho = qe/qd (CS eq 22-23, MC eq 27)
+    const double d2qf = T ? mulk_x<3, 1>((dph_lo + dph_hi) - twice_x(q_i)) : 6.0 * (dph_lo + dph_hi - 2.0 * q_i);
     double qe = 0.0;
     const bool sd = is_neg(d2qf);
     if (sd == is_neg(d2m1) && sd == is_neg(d20) && sd == is_neg(d2p1)) {
@@ -503,19 +631,19 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
                                     (long long)0x8000000000000000ULL) : 0LL;
       const double zm = __longlong_as_double(rs ^ (__double_as_longlong(dqf_minus) & (long long)0x8000000000000000ULL));
       const double zp = __longlong_as_double(rs ^ (__double_as_longlong(dqf_plus) & (long long)0x8000000000000000ULL));
-      qr = sub_x(q_i, zm);
-      ql = add_x(q_i, zp);
+      qr = q_i - zm;
+      ql = q_i + zp;
     } else if (T && __double_as_longlong(qe) == __double_as_longlong(d2qf)) {
       // rho = d2qf / d2qf = 1 > 1 - 1e-12: the face values stay
     } else {
-      if (guard) rho = qe / d2qf;
+      if (guard) rho = div_x(qe, d2qf);
       if (le(rho, 1.0 - 1.0e-12)) {
-        qr = T ? sub_x(q_i, rho * dqf_minus) : q_i - rho * dqf_minus;
-        ql = T ? add_x(q_i, rho * dqf_plus) : q_i + rho * dqf_plus;
+        qr = q_i - rho * dqf_minus;
+        ql = q_i + rho * dqf_plus;
       }
     }
 #else
-    if (guard) rho = qe / d2qf;
+    if (guard) rho = div_x(qe, d2qf);
     if (le(rho, 1.0 - 1.0e-12)) {
       qr = fma(-rho, dqf_minus, q_i);
       ql = fma(rho, dqf_plus, q_i);
@@ -523,9 +651,9 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
 #endif
   } else {
     if (mag(dqf_minus) >= twice_mag(dqf_plus))
-      qr = T ? sub_x(q_i, twice_x(dqf_plus)) : q_i - 2.0 * dqf_plus;
+      qr = T ? q_i - twice_x(dqf_plus) : q_i - 2.0 * dqf_plus;
     if (mag(dqf_plus) >= twice_mag(dqf_minus))
-      ql = T ? add_x(q_i, twice_x(dqf_minus)) : q_i + 2.0 * dqf_minus;
+      ql = T ? q_i + twice_x(dqf_minus) : q_i + 2.0 * dqf_minus;
   }
   ql_ip1 = ql;
   qr_i = qr;
@@ -545,6 +673,72 @@ __device__ __forceinline__ void ppm(double q_im2, double q_im1, double q_i, doub
   ppm_cell(q_im2, q_im1, q_i, q_ip1, q_ip2, d2_m1, d2_0, d2_p1, lo, hi, ql_ip1, qr_i);
 }
 
+#if APH_EXACT
+// ---- reconstruction of the adiabatic indices as small integers --------------------------
+// Where no floor fired, gamma_c = B / p and gamma_e = p / (rho e) + 1 are gamma up to a few
+// rounding errors.  A window whose indices all lie within kGamMax units u of the last place of
+// gamma = gm1 + 1 (M u, in one binade) is reconstructed on the offsets k = g / u - M: every sum,
+// difference and rounding of PPM and PLM on such values is a small integer operation with the
+// same result (a sum of two values of the binade is rounded to a multiple of 2 u, half to even;
+// a value added to such a mean is rounded to a multiple of u).  In PPM's extremum branch
+// |d2qf| <= 6 (2 (kGamMax + 41) + 2 kGamMax + 1) u stays below the roundoff guard's 1e-12 |q| (at least
+// 4503 u), so rho is 0 and both face values are the cell's.
+constexpr int kGamMax = 100;
+__device__ __forceinline__ int gam_round_half(int K, int odd) {  // RN((2 M + K) / 2) - M; odd: of M
+  const int h = K >> 1;
+  return h + (K & (h + odd) & 1);
+}
+__device__ __forceinline__ int gam_round_12(int j, int odd) {  // RN(M + j / 12) - M, |j| < 2000
+  const int t = j + 6 + 12 * 256;
+  const int q = (t * 5462) >> 16;  // floor(t / 12) for 0 <= t < 8160
+  return q - 256 - ((t - 12 * q == 0) & (q + odd) & 1);
+}
+// The limited value at the face between cells of offsets b and c (a, d: the next ones), as
+// ppm_face.  avg = M + h; the interpolation adds j / 12 with j the difference of the slopes;
+// qa = -6 m u, the second differences 2 e u, and the limited qd / 6 is (qd / u * 2) / 12 u.
+__device__ __forceinline__ int gam_face(int a, int b, int c, int d, int odd) {
+  const int h = gam_round_half(b + c, odd);
+  const int m = gam_round_12((c - a) - (d - b), odd + h);
+  int f = h + m;
+  if ((f > b && f > c) || (f < b && f < c)) {
+    const int eb = gam_round_half(a + c, odd) - b, ec = gam_round_half(b + d, odd) - c;
+    int q = 0;
+    if ((m > 0) == (eb < 0) && (m > 0) == (ec < 0)) {
+      const int lim = 5 * min(abs(eb), abs(ec));
+      q = min(12 * abs(m), lim);
+      if (m > 0) q = -q;
+    }
+    f = h + gam_round_12(-q, odd + h);
+  }
+  return f;
+}
+// ppm_cell: lo, hi the face values of cell q0 (qm, qp: its neighbours)
+__device__ __forceinline__ void gam_cell(int qm, int q0, int qp, int lo, int hi, int &ql, int &qr) {
+  const int dm = q0 - lo, dp = hi - q0;
+  const bool between = (dm > 0 && dp > 0) || (dm < 0 && dp < 0);
+  const bool monotone = (qm < q0 && q0 < qp) || (qm > q0 && q0 > qp);
+  if (!between || !monotone) {
+    ql = qr = q0;
+  } else {
+    qr = abs(dm) >= 2 * abs(dp) ? q0 - 2 * dp : lo;
+    ql = abs(dp) >= 2 * abs(dm) ? q0 + 2 * dm : hi;
+  }
+}
+// plm: q0 +- dl dr / (dl + dr), rounded half to even
+__device__ __forceinline__ void gam_plm(int qm, int q0, int qp, int odd, int &ql, int &qr) {
+  const int dl = q0 - qm, dr = qp - q0;
+  ql = qr = q0;
+  if (dl * dr <= 0) return;
+  const unsigned num = dl * dr, sum = abs(dl + dr);
+  const int x = (int)(num / sum);
+  const unsigned rest = 2 * (num - x * sum);
+  const int up = rest > sum || (rest == sum && ((q0 + x + odd) & 1));  // x or x + 1, either way
+  const int s = dl > 0 ? x + up : -(x + up);
+  ql = q0 + s;
+  qr = q0 - s;
+}
+#endif
+
 template <int RECON>
 __device__ __forceinline__ void reconstruct(const double *q, double &ql_ip1, double &qr_i) {
   // q[-2..2] addressable around q[0]
@@ -563,34 +757,20 @@ __device__ __forceinline__ void reconstruct(const double *q, double &ql_ip1, dou
 // flx: (mass, normal momentum, t1 momentum, t2 momentum, energy).
 
 // c-limited sound speed C*sqrt(gamma / (1 + (1/gm1 + rho C^2 / p))) (hydro_hlle.hpp:63-66)
-template <bool CONSTG>
-__device__ __forceinline__ double sound_speed(double rho, double p, double gamma, double igm1,
-                                              const GasConsts &gc) {
+
 #if APH_EXACT
-  return C_LIGHT * sqrt(gamma / (1 + (igm1 + rho * C_LIGHT2 / p)));
-#else
-  // same quantity as sqrt(C^2 gamma p / (p (1 + 1/gm1) + rho C^2))
-  const double num = (CONSTG ? gc.c2g : C_LIGHT2 * gamma) * p;
-  const double den = fma(p, CONSTG ? gc.one_igm1 : 1.0 + igm1, rho * C_LIGHT2);
-  return num * rsqrt(num * den);
-#endif
+template <class OPS>
+__device__ __forceinline__ double sound_speed(double rho, double p, double gamma, double igm1, OPS &o) {
+  return C_LIGHT * o.sqrt(o.div(gamma, 1 + (igm1 + o.div(rho * C_LIGHT2, p))));
 }
 
-template <bool CONSTG>
-__device__ __forceinline__ void solve_hlle(const double *wli, const double *wri, double glc,
-                                           double gle, double grc, double gre,
-                                           const GasConsts &gc, double *flxi) {
-  const double gammal = CONSTG ? gc.gamma : glc;
-  const double gammar = CONSTG ? gc.gamma : grc;
-  double igm1l, igm1r;
-  if (CONSTG) {
-    igm1l = igm1r = gc.igm1;
-  } else {
-    igm1l = __drcp_rn(gle - 1);  // the correctly rounded 1.0 / (gle - 1), cheaper than a division
-    igm1r = __drcp_rn(gre - 1);
-  }
-  const double cl = sound_speed<CONSTG>(wli[IDN], wli[IPR], gammal, igm1l, gc);
-  const double cr = sound_speed<CONSTG>(wri[IDN], wri[IPR], gammar, igm1r, gc);
+template <class OPS>
+__device__ __forceinline__ void solve_hlle_exact(const double *wli, const double *wri, double glc,
+                                                 double gle, double grc, double gre, double *flxi,
+                                                 OPS &o) {
+  const double igm1l = o.rcp(gle - 1), igm1r = o.rcp(gre - 1);
+  const double cl = sound_speed(wli[IDN], wli[IPR], glc, igm1l, o);
+  const double cr = sound_speed(wri[IDN], wri[IPR], grc, igm1r, o);
   const double el = wli[IPR] * igm1l +
                     0.5 * wli[IDN] * (wli[IV1] * wli[IV1] + wli[IV2] * wli[IV2] + wli[IV3] * wli[IV3]);
   const double er = wri[IPR] * igm1r +
@@ -599,21 +779,10 @@ __device__ __forceinline__ void solve_hlle(const double *wli, const double *wri,
   const double ca = .5 * (cl + cr);
   const double pmid = .5 * (wli[IPR] + wri[IPR] + (wli[IV1] - wri[IV1]) * rhoa * ca);
   double ql = 1.0, qr = 1.0;
-#if APH_EXACT
-  if (gt(pmid, wli[IPR])) ql = 1.0 + (gammal + 1) / sqrt(2 * gammal) * (pmid / wli[IPR] - 1.0);
-  if (gt(pmid, wri[IPR])) qr = 1.0 + (gammar + 1) / sqrt(2 * gammar) * (pmid / wri[IPR] - 1.0);
-#else
-  {
-    const bool bl = gt(pmid, wli[IPR]), br = gt(pmid, wri[IPR]);
-    if (bl || br) {
-      const double ipp = 1.0 / (wli[IPR] * wri[IPR]);  // shared reciprocal
-      const double kl = CONSTG ? gc.hlle_k : (gammal + 1) * rsqrt(2 * gammal);
-      const double kr = CONSTG ? gc.hlle_k : (gammar + 1) * rsqrt(2 * gammar);
-      if (bl) ql = fma(kl, fma(pmid * wri[IPR], ipp, -1.0), 1.0);
-      if (br) qr = fma(kr, fma(pmid * wli[IPR], ipp, -1.0), 1.0);
-    }
-  }
-#endif
+  if (gt(pmid, wli[IPR]))
+    ql = 1.0 + o.div(glc + 1, o.sqrt(2 * glc)) * (o.div(pmid, wli[IPR]) - 1.0);
+  if (gt(pmid, wri[IPR]))
+    qr = 1.0 + o.div(grc + 1, o.sqrt(2 * grc)) * (o.div(pmid, wri[IPR]) - 1.0);
   const double al = wli[IV1] - cl * ql;
   const double ar = wri[IV1] + cr * qr;
   const double bp = is_pos(ar) ? ar : 0.0;
@@ -635,10 +804,138 @@ __device__ __forceinline__ void solve_hlle(const double *wli, const double *wri,
   fr[IEN] = er * vxr + wri[IPR] * wri[IV1];
   double tmp = 0.0;
   if (__double_as_longlong(bp) != __double_as_longlong(bm) && (mag(bp) | mag(bm)) != 0ULL)
-    tmp = 0.5 * (bp + bm) / (bp - bm);
+    tmp = o.div0(0.5 * (bp + bm), o.den(bp - bm));
 #pragma unroll
   for (int n = 0; n < NHYDRO; ++n) flxi[n] = 0.5 * (fl[n] + fr[n]) + (fl[n] - fr[n]) * tmp;
 }
+
+#else
+// The fast solvers name every fused multiply-add themselves: left to the compiler, which products
+// are fused depends on how it splits the code into blocks, and PPM's discontinuous limiters turn
+// a difference of one rounding into a different flux, so that builds and launches would no
+// longer agree with one another.
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double square3(double a, double b, double c) {  // a^2 + b^2 + c^2
+  return fma(c, c, fma(a, a, mul(b, b)));
+}
+
+// the square of the sound speed as num / den
+template <bool CONSTG>
+__device__ __forceinline__ void sound_parts(double rho, double p, double gamma, double igm1,
+                                            const GasConsts &gc, double &num, double &root) {
+  num = CONSTG ? mul(gc.c2g, p) : mul(mul(C_LIGHT2, gamma), p);
+  const double den = fma(p, CONSTG ? gc.one_igm1 : add(1.0, igm1), mul(rho, C_LIGHT2));
+  root = rsqrt(mul(num, den));  // the speed is num * root
+}
+template <bool CONSTG>
+__device__ __forceinline__ double sound_speed(double rho, double p, double gamma, double igm1,
+                                              const GasConsts &gc) {
+  double num, root;
+  sound_parts<CONSTG>(rho, p, gamma, igm1, gc, num, root);
+  return mul(num, root);
+}
+
+template <bool CONSTG, class OPS>
+__device__ __forceinline__ void solve_hlle(const double *wl, const double *wr, double glc, double gle,
+                                           double grc, double gre, const GasConsts &gc, double *flx,
+                                           OPS &o) {
+  const double gl = CONSTG ? gc.gamma : glc, gr = CONSTG ? gc.gamma : grc;
+  const double il = CONSTG ? gc.igm1 : o.rcp(sub(gle, 1)), ir = CONSTG ? gc.igm1 : o.rcp(sub(gre, 1));
+  const double cl = sound_speed<CONSTG>(wl[IDN], wl[IPR], gl, il, gc);
+  const double cr = sound_speed<CONSTG>(wr[IDN], wr[IPR], gr, ir, gc);
+  const double el = fma(wl[IPR], il, mul(mul(0.5, wl[IDN]), square3(wl[IV1], wl[IV2], wl[IV3])));
+  const double er = fma(wr[IPR], ir, mul(mul(0.5, wr[IDN]), square3(wr[IV1], wr[IV2], wr[IV3])));
+  const double rhoa = mul(.5, add(wl[IDN], wr[IDN])), ca = mul(.5, add(cl, cr));
+  const double pmid = mul(.5, fma(mul(sub(wl[IV1], wr[IV1]), rhoa), ca, add(wl[IPR], wr[IPR])));
+  double ql = 1.0, qr = 1.0;
+  const bool bl = gt(pmid, wl[IPR]), br = gt(pmid, wr[IPR]);
+  if (bl || br) {
+    const double ipp = o.rcp(mul(wl[IPR], wr[IPR]));  // shared reciprocal
+    const double kl = CONSTG ? gc.hlle_k : mul(add(gl, 1), rsqrt(mul(2, gl)));
+    const double kr = CONSTG ? gc.hlle_k : mul(add(gr, 1), rsqrt(mul(2, gr)));
+    if (bl) ql = fma(kl, fma(mul(pmid, wr[IPR]), ipp, -1.0), 1.0);
+    if (br) qr = fma(kr, fma(mul(pmid, wl[IPR]), ipp, -1.0), 1.0);
+  }
+  const double al = fma(-cl, ql, wl[IV1]), ar = fma(cr, qr, wr[IV1]);
+  const double bp = is_pos(ar) ? ar : 0.0, bm = is_neg(al) ? al : 0.0;
+  const double vl = sub(wl[IV1], bm), vr = sub(wr[IV1], bp);
+  double fl[NHYDRO], fr[NHYDRO];
+  fl[IDN] = mul(wl[IDN], vl);
+  fr[IDN] = mul(wr[IDN], vr);
+  fl[IV1] = fma(mul(wl[IDN], wl[IV1]), vl, wl[IPR]);
+  fr[IV1] = fma(mul(wr[IDN], wr[IV1]), vr, wr[IPR]);
+  fl[IV2] = mul(mul(wl[IDN], wl[IV2]), vl);
+  fr[IV2] = mul(mul(wr[IDN], wr[IV2]), vr);
+  fl[IV3] = mul(mul(wl[IDN], wl[IV3]), vl);
+  fr[IV3] = mul(mul(wr[IDN], wr[IV3]), vr);
+  fl[IEN] = fma(el, vl, mul(wl[IPR], wl[IV1]));
+  fr[IEN] = fma(er, vr, mul(wr[IPR], wr[IV1]));
+  double t = 0.0;
+  if (__double_as_longlong(bp) != __double_as_longlong(bm) && (mag(bp) | mag(bm)) != 0ULL)
+    t = o.div0(mul(0.5, add(bp, bm)), o.den(sub(bp, bm)));
+#pragma unroll
+  for (int n = 0; n < NHYDRO; ++n) flx[n] = fma(0.5, add(fl[n], fr[n]), mul(sub(fl[n], fr[n]), t));
+}
+
+// HLLC; LOWMACH: the pstar of hydro_lhllc.hpp:71-79, whose "Mach" is the speed |v| itself
+template <bool CONSTG, bool LOWMACH, class OPS>
+__device__ __forceinline__ void solve_hllc(const double *wl, const double *wr, double glc, double gle,
+                                           double grc, double gre, const GasConsts &gc, double *flx,
+                                           OPS &o) {
+  const double gl = CONSTG ? gc.gamma : glc, gr = CONSTG ? gc.gamma : grc;
+  const double il = CONSTG ? gc.igm1 : o.rcp(sub(gle, 1)), ir = CONSTG ? gc.igm1 : o.rcp(sub(gre, 1));
+  const double cl = sound_speed<CONSTG>(wl[IDN], wl[IPR], gl, il, gc);
+  const double cr = sound_speed<CONSTG>(wr[IDN], wr[IPR], gr, ir, gc);
+  const double rhoa = mul(.5, add(wl[IDN], wr[IDN])), ca = mul(.5, add(cl, cr));
+  double x = mul(mul(mul(.5, sub(wr[IV1], wl[IV1])), rhoa), ca);
+  if (LOWMACH) {
+    auto root = [&](double q) { return is_zero(q) ? q : o.sqrt(is_zero(q) ? 1.0 : q); };
+    const double chi = smax(root(square3(wl[IV1], wl[IV2], wl[IV3])), root(square3(wr[IV1], wr[IV2], wr[IV3])));
+    x = mul(x, mul(chi, sub(2.0, chi)));
+  }
+  const double pstar = fma(.5, add(wl[IPR], wr[IPR]), -x);
+  double ql = 1.0, qr = 1.0;
+  const bool bl = gt(pstar, wl[IPR]), br = gt(pstar, wr[IPR]);
+  if (bl || br) {
+    const double ipp = o.rcp(mul(wl[IPR], wr[IPR]));
+    const double k = CONSTG ? gc.hllc_k : o.div(add(gl, 1), mul(2, gr));
+    if (bl) ql = o.sqrt(fma(k, fma(mul(pstar, wr[IPR]), ipp, -1.0), 1.0));
+    if (br) qr = o.sqrt(fma(k, fma(mul(pstar, wl[IPR]), ipp, -1.0), 1.0));
+  }
+  const double sl = fma(-cl, ql, wl[IV1]), sr = fma(cr, qr, wr[IV1]);
+  const double bp = is_pos(sr) ? sr : TINY_NUMBER;
+  const double bm = is_neg(sl) ? sl : -TINY_NUMBER;
+  const double vl = sub(wl[IV1], sl), vr = sub(wr[IV1], sr);
+  const double tl = fma(mul(vl, wl[IDN]), wl[IV1], wl[IPR]);
+  const double tr = fma(mul(vr, wr[IDN]), wr[IV1], wr[IPR]);
+  const double ml = mul(wl[IDN], vl), mr = -mul(wr[IDN], vr);
+  const double imm = o.rcp(add(ml, mr));
+  const double sstar = mul(sub(tl, tr), imm);
+  double cp = mul(fma(ml, tr, mul(mr, tl)), imm);
+  cp = is_pos(cp) ? cp : 0.0;
+  // one-sided: the flux is sstar/(sstar - b) times the physical flux of the upwind side of
+  // the contact (left with b = bm when sstar >= 0, else right with b = bp) plus the pressure
+  // terms; the other side's weight is exactly 0, so this is the two-sided sum of the reference
+  // with its zero term dropped
+  const bool L = !is_neg(sstar);
+  const double rho = L ? wl[IDN] : wr[IDN], u = L ? wl[IV1] : wr[IV1];
+  const double v = L ? wl[IV2] : wr[IV2], z = L ? wl[IV3] : wr[IV3];
+  const double p = L ? wl[IPR] : wr[IPR];
+  const double b = L ? bm : bp;
+  const double e = fma(p, L ? il : ir, mul(mul(0.5, rho), square3(u, v, z)));
+  const double id = o.rcp(sub(sstar, b));
+  const double coef = mul(sstar, id);
+  const double ustar = mul(-b, id);
+  const double vx = sub(u, b);
+  flx[IDN] = mul(coef, mul(rho, vx));
+  flx[IV1] = fma(coef, fma(mul(rho, u), vx, p), mul(ustar, cp));
+  flx[IV2] = mul(coef, mul(mul(rho, v), vx));
+  flx[IV3] = mul(coef, mul(mul(rho, z), vx));
+  flx[IEN] = fma(mul(ustar, cp), sstar, mul(coef, fma(p, u, mul(e, vx))));
+}
+#endif
 
 // x = 2^k with x and 1/x both normal: then y / x == y * (1/x) exactly for every y (both are
 // the correctly rounded y * 2^-k), so a division by x is a multiplication.
@@ -650,18 +947,20 @@ __device__ __forceinline__ bool pow2_normal(double x) {
 // y / vol, correctly rounded; ivol = 1 / vol, p2 = pow2_normal(vol) (uniform over a block)
 __device__ __forceinline__ double div_vol(double y, double vol, double ivol, bool p2) {
   if (p2) return y * ivol;
-  return y / vol;
+  return div_x(y, vol);
 }
 
+#if APH_EXACT
 // The reference's c-limited sound speed C sqrt(gamma / (1 + (igm1 + rho C^2 / p)))
 // (hydro_hllc.hpp:57-60) with its roundings.  Where X = rho C^2 / p is at least 2^55 times
 // both igm1 and 1 (always for non-relativistic gas: X ~ (c_light / c_sound)^2), each addition
 // adds less than a quarter ulp of X and returns X, so both are skipped.
-__device__ __forceinline__ double csound_exact(double rho, double p, double gamma, double igm1, double yp) {
-  const double X = div_y(rho * C_LIGHT2, p, yp);
+template <class OPS>
+__device__ __forceinline__ double csound_exact(double rho, const Den &p, double gamma, double igm1, OPS &o) {
+  const double X = o.div(rho * C_LIGHT2, p);
   const long long ex = (long long)(mag(X) >> 52), ei = (long long)(mag(igm1) >> 52);
-  const double den = (ex >= 1023 + 55 && ex >= ei + 55 && ex < 2047) ? X : 1 + (igm1 + X);
-  return C_LIGHT * sqrt(gamma / den);
+  const double d = (ex >= 1023 + 55 && ex >= ei + 55 && ex < 2047) ? X : 1 + (igm1 + X);
+  return C_LIGHT * o.sqrt(o.div(gamma, d));
 }
 
 // exponent field all ones: an infinity or a NaN
@@ -684,25 +983,26 @@ __device__ __forceinline__ bool nonfinite(double x) {
 //    term is zero and the sign of the zero sum depends on it, or where the other side is
 //    not finite.  The halvings and doublings run on the integer pipe (half_x, twice_x).
 //    Without TAME both sides' terms are always formed.
-template <bool LOWMACH, bool TAME>
+template <bool LOWMACH, bool TAME, class OPS>
 __device__ __forceinline__ void solve_hllc_exact(const double *wli, const double *wri, double glc,
-                                                 double gle, double grc, double gre, double *flxi) {
+                                                 double gle, double grc, double gre, double *flxi,
+                                                 OPS &o) {
   auto hlf = [](double x) { return TAME ? half_x(x) : 0.5 * x; };
   const double gammal = glc, gammar = grc;
-  const double igm1l = __drcp_rn(gle - 1), igm1r = __drcp_rn(gre - 1);  // == 1.0 / (g - 1)
-  // 1 / p of each side: the sound speed and the shock factor divide by p (div_y; unused
-  // where the operands leave the tame range and the divisions are made as such)
-  const double ypl = __drcp_rn(wli[IPR]), ypr = __drcp_rn(wri[IPR]);
-  const double cl = csound_exact(wli[IDN], wli[IPR], gammal, igm1l, ypl);
-  const double cr = csound_exact(wri[IDN], wri[IPR], gammar, igm1r, ypr);
+  const double igm1l = o.rcp(gle - 1), igm1r = o.rcp(gre - 1);
+  // the sound speed and the shock factor divide by the pressures
+  const Den pl = o.den(wli[IPR]), pr = o.den(wri[IPR]);
+  const double cl = csound_exact(wli[IDN], pl, gammal, igm1l, o);
+  const double cr = csound_exact(wri[IDN], pr, gammar, igm1r, o);
   const double rhoa = hlf(wli[IDN] + wri[IDN]);
   const double ca = hlf(cl + cr);
   double pstar;
   if (!LOWMACH) {
     pstar = hlf(wli[IPR] + wri[IPR]) - hlf(wri[IV1] - wli[IV1]) * rhoa * ca;
   } else {
-    const double machl = sqrt(wli[IV1] * wli[IV1] + wli[IV2] * wli[IV2] + wli[IV3] * wli[IV3]);
-    const double machr = sqrt(wri[IV1] * wri[IV1] + wri[IV2] * wri[IV2] + wri[IV3] * wri[IV3]);
+    auto root = [&](double x) { return is_zero(x) ? x : o.sqrt(is_zero(x) ? 1.0 : x); };
+    const double machl = root(wli[IV1] * wli[IV1] + wli[IV2] * wli[IV2] + wli[IV3] * wli[IV3]);
+    const double machr = root(wri[IV1] * wri[IV1] + wri[IV2] * wri[IV2] + wri[IV3] * wri[IV3]);
     const double chi = smax(machl, machr);
     const double phi = chi * (2.0 - chi);
     pstar = hlf(wli[IPR] + wri[IPR]) - hlf(wri[IV1] - wli[IV1]) * rhoa * ca * phi;
@@ -710,11 +1010,11 @@ __device__ __forceinline__ void solve_hllc_exact(const double *wli, const double
   double ql = 1.0, qr = 1.0;
   const bool bl = gt(pstar, wli[IPR]), br = gt(pstar, wri[IPR]);
   if (bl || br) {
-    const double k = (gammal + 1) / (TAME ? twice_x(gammar) : 2 * gammar);
-    const double q1 = sqrt(1.0 + k * (div_y(pstar, bl ? wli[IPR] : wri[IPR], bl ? ypl : ypr) - 1.0));
+    const double k = o.div(gammal + 1, TAME ? twice_x(gammar) : 2 * gammar);
+    const double q1 = o.sqrt(1.0 + k * (o.div(pstar, bl ? pl : pr) - 1.0));
     if (bl) ql = q1;
     else qr = q1;
-    if (bl && br) qr = sqrt(1.0 + k * (div_y(pstar, wri[IPR], ypr) - 1.0));
+    if (bl && br) qr = o.sqrt(1.0 + k * (o.div(pstar, pr) - 1.0));
   }
   const double sl = wli[IV1] - cl * ql;
   const double sr = wri[IV1] + cr * qr;
@@ -726,13 +1026,14 @@ __device__ __forceinline__ void solve_hllc_exact(const double *wli, const double
   const double tr = wri[IPR] + vxr0 * wri[IDN] * wri[IV1];
   const double ml = wli[IDN] * vxl0;
   const double mr = -(wri[IDN] * vxr0);
-  double sstar, cp;  // (tl - tr) / (ml + mr), (ml tr + mr tl) / (ml + mr)
-  div2(tl - tr, ml * tr + mr * tl, ml + mr, sstar, cp);
+  const Den m = o.den(ml + mr);
+  const double sstar = o.div0(tl - tr, m);
+  double cp = o.div0(ml * tr + mr * tl, m);
   cp = is_pos(cp) ? cp : 0.0;
   const bool L = !is_neg(sstar);  // sstar >= 0.0
-  const double den = L ? sstar - bm : bp - sstar;
-  double coef, ustar;  // ul (or ur) and ustar: (+-sstar) / den, (-bm or bp) / den
-  div2(L ? sstar : -sstar, L ? -bm : bp, den, coef, ustar);
+  const Den d = o.den(L ? sstar - bm : bp - sstar);
+  const double coef = o.div0(L ? sstar : -sstar, d);  // ul (or ur)
+  const double ustar = o.div(L ? -bm : bp, d);
   // the upwind side (U) and the other one (O)
   const double *wu = L ? wli : wri, *wo = L ? wri : wli;
   const double igu = L ? igm1l : igm1r;
@@ -775,157 +1076,24 @@ __device__ __forceinline__ void solve_hllc_exact(const double *wli, const double
   flxi[IEN] = t[IEN] + ustar * cp * sstar;
 }
 
-template <bool CONSTG, bool LOWMACH>
-__device__ __forceinline__ void solve_hllc(const double *wli, const double *wri, double glc,
-                                           double gle, double grc, double gre,
-                                           const GasConsts &gc, double *flxi) {
-  const double gammal = CONSTG ? gc.gamma : glc;
-  const double gammar = CONSTG ? gc.gamma : grc;
-  double igm1l, igm1r;
-  if (CONSTG) {
-    igm1l = igm1r = gc.igm1;
-  } else {
-    igm1l = __drcp_rn(gle - 1);  // the correctly rounded 1.0 / (gle - 1), cheaper than a division
-    igm1r = __drcp_rn(gre - 1);
-  }
-  const double cl = sound_speed<CONSTG>(wli[IDN], wli[IPR], gammal, igm1l, gc);
-  const double cr = sound_speed<CONSTG>(wri[IDN], wri[IPR], gammar, igm1r, gc);
-  const double el = wli[IPR] * igm1l +
-                    0.5 * wli[IDN] * (wli[IV1] * wli[IV1] + wli[IV2] * wli[IV2] + wli[IV3] * wli[IV3]);
-  const double er = wri[IPR] * igm1r +
-                    0.5 * wri[IDN] * (wri[IV1] * wri[IV1] + wri[IV2] * wri[IV2] + wri[IV3] * wri[IV3]);
-  const double rhoa = .5 * (wli[IDN] + wri[IDN]);
-  const double ca = .5 * (cl + cr);
-  double pstar;
-  if (!LOWMACH) {
-    pstar = .5 * (wli[IPR] + wri[IPR]) - .5 * (wri[IV1] - wli[IV1]) * rhoa * ca;
-  } else {
-    // hydro_lhllc.hpp:71-79: "Mach" is the speed |v| itself
-    const double machl = sqrt(wli[IV1] * wli[IV1] + wli[IV2] * wli[IV2] + wli[IV3] * wli[IV3]);
-    const double machr = sqrt(wri[IV1] * wri[IV1] + wri[IV2] * wri[IV2] + wri[IV3] * wri[IV3]);
-    const double chi = smax(machl, machr);
-    const double phi = chi * (2.0 - chi);
-    pstar = .5 * (wli[IPR] + wri[IPR]) - .5 * (wri[IV1] - wli[IV1]) * rhoa * ca * phi;
-  }
-  double ql = 1.0, qr = 1.0;
-#if APH_EXACT
-  if (gt(pstar, wli[IPR])) ql = sqrt(1.0 + (gammal + 1) / (2 * gammar) * (pstar / wli[IPR] - 1.0));
-  if (gt(pstar, wri[IPR])) qr = sqrt(1.0 + (gammal + 1) / (2 * gammar) * (pstar / wri[IPR] - 1.0));
-#else
-  {
-    const bool bl = gt(pstar, wli[IPR]), br = gt(pstar, wri[IPR]);
-    if (bl || br) {
-      const double ipp = 1.0 / (wli[IPR] * wri[IPR]);
-      const double k = CONSTG ? gc.hllc_k : (gammal + 1) / (2 * gammar);
-      if (bl) ql = sqrt(fma(k, fma(pstar * wri[IPR], ipp, -1.0), 1.0));
-      if (br) qr = sqrt(fma(k, fma(pstar * wli[IPR], ipp, -1.0), 1.0));
-    }
-  }
 #endif
-  const double sl = wli[IV1] - cl * ql;
-  const double sr = wri[IV1] + cr * qr;
-  const double bp = is_pos(sr) ? sr : TINY_NUMBER;
-  const double bm = is_neg(sl) ? sl : -TINY_NUMBER;
-  double vxl = wli[IV1] - sl;
-  double vxr = wri[IV1] - sr;
-  const double tl = wli[IPR] + vxl * wli[IDN] * wli[IV1];
-  const double tr = wri[IPR] + vxr * wri[IDN] * wri[IV1];
-  const double ml = wli[IDN] * vxl;
-  const double mr = -(wri[IDN] * vxr);
-#if APH_EXACT
-  const double sstar = (tl - tr) / (ml + mr);
-  double cp = (ml * tr + mr * tl) / (ml + mr);
-#else
-  const double imm = 1.0 / (ml + mr);
-  const double sstar = (tl - tr) * imm;
-  double cp = (ml * tr + mr * tl) * imm;
-#endif
-  cp = is_pos(cp) ? cp : 0.0;
-#if !APH_EXACT
-  {
-    // one-sided: the flux is sstar/(sstar - b) times the physical flux of the upwind side of
-    // the contact (left with b = bm when sstar >= 0, else right with b = bp) plus the
-    // pressure terms; the other side's weight is exactly 0, so this is the two-sided sum of
-    // the reference with its zero term dropped
-    const bool L = !is_neg(sstar);
-    const double rho = L ? wli[IDN] : wri[IDN], u = L ? wli[IV1] : wri[IV1];
-    const double v = L ? wli[IV2] : wri[IV2], z = L ? wli[IV3] : wri[IV3];
-    const double p = L ? wli[IPR] : wri[IPR];
-    const double b = L ? bm : bp;
-    const double e = p * (L ? igm1l : igm1r) + 0.5 * rho * (u * u + v * v + z * z);
-    const double id = 1.0 / (sstar - b);
-    const double coef = sstar * id;
-    const double ustar = -b * id;
-    const double vx = u - b;
-    flxi[IDN] = coef * (rho * vx);
-    flxi[IV1] = coef * (rho * u * vx + p) + ustar * cp;
-    flxi[IV2] = coef * (rho * v * vx);
-    flxi[IV3] = coef * (rho * z * vx);
-    flxi[IEN] = coef * (e * vx + p * u) + ustar * cp * sstar;
-    return;
-  }
-#endif
-  vxl = wli[IV1] - bm;
-  vxr = wri[IV1] - bp;
-  double fl[NHYDRO], fr[NHYDRO];
-  fl[IDN] = wli[IDN] * vxl;
-  fr[IDN] = wri[IDN] * vxr;
-  fl[IV1] = wli[IDN] * wli[IV1] * vxl + wli[IPR];
-  fr[IV1] = wri[IDN] * wri[IV1] * vxr + wri[IPR];
-  fl[IV2] = wli[IDN] * wli[IV2] * vxl;
-  fr[IV2] = wri[IDN] * wri[IV2] * vxr;
-  fl[IV3] = wli[IDN] * wli[IV3] * vxl;
-  fr[IV3] = wri[IDN] * wri[IV3] * vxr;
-  fl[IEN] = el * vxl + wli[IPR] * wli[IV1];
-  fr[IEN] = er * vxr + wri[IPR] * wri[IV1];
-  double ul, ur, ustar;
-  if (!is_neg(sstar)) {  // sstar >= 0.0
-#if APH_EXACT
-    ul = sstar / (sstar - bm);
-    ustar = -bm / (sstar - bm);
-#else
-    const double id = 1.0 / (sstar - bm);
-    ul = sstar * id;
-    ustar = -bm * id;
-#endif
-    ur = 0.0;
-  } else {
-#if APH_EXACT
-    ur = -sstar / (bp - sstar);
-    ustar = bp / (bp - sstar);
-#else
-    const double id = 1.0 / (bp - sstar);
-    ur = -sstar * id;
-    ustar = bp * id;
-#endif
-    ul = 0.0;
-  }
-  flxi[IDN] = ul * fl[IDN] + ur * fr[IDN];
-  flxi[IV1] = ul * fl[IV1] + ur * fr[IV1] + ustar * cp;
-  flxi[IV2] = ul * fl[IV2] + ur * fr[IV2];
-  flxi[IV3] = ul * fl[IV3] + ur * fr[IV3];
-  flxi[IEN] = ul * fl[IEN] + ur * fr[IEN] + ustar * cp * sstar;
-}
 
-template <int RS, bool CONSTG, bool TAME = false>
+// Fluxes of one face.  The caller checks o.ok() (IntOps), and takes the face again with IeeeOps
+// where it is false.
+template <int RS, bool CONSTG, bool TAME, class OPS>
 __device__ __forceinline__ void riemann(const double *wl, const double *wr, double glc, double gle,
-                                        double grc, double gre, const GasConsts &gc,
-                                        double *flx) {
-  if (RS == RS_HLLE) {
-    solve_hlle<CONSTG>(wl, wr, glc, gle, grc, gre, gc, flx);
-  } else if (RS == RS_HLLC) {
+                                        double grc, double gre, const GasConsts &gc, double *flx,
+                                        OPS &o) {
 #if APH_EXACT
-    solve_hllc_exact<false, TAME>(wl, wr, glc, gle, grc, gre, flx);
+  if (RS == RS_HLLE) solve_hlle_exact(wl, wr, glc, gle, grc, gre, flx, o);
+  else if (RS == RS_HLLC || RS == RS_LHLLC)
+    solve_hllc_exact<RS == RS_LHLLC, TAME>(wl, wr, glc, gle, grc, gre, flx, o);
 #else
-    solve_hllc<CONSTG, false>(wl, wr, glc, gle, grc, gre, gc, flx);
+  if (RS == RS_HLLE) solve_hlle<CONSTG>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+  else if (RS == RS_HLLC || RS == RS_LHLLC)
+    solve_hllc<CONSTG, RS == RS_LHLLC>(wl, wr, glc, gle, grc, gre, gc, flx, o);
 #endif
-  } else if (RS == RS_LHLLC) {
-#if APH_EXACT
-    solve_hllc_exact<true, TAME>(wl, wr, glc, gle, grc, gre, flx);
-#else
-    solve_hllc<CONSTG, true>(wl, wr, glc, gle, grc, gre, gc, flx);
-#endif
-  } else {
+  else {
 #pragma unroll
     for (int n = 0; n < NHYDRO; ++n) flx[n] = 0.0;
   }
@@ -935,19 +1103,31 @@ __device__ __forceinline__ void riemann(const double *wl, const double *wr, doub
 // of dx_d / (|v_d| + lambda).  dt_cell below is the form the stage kernel uses.
 __device__ __forceinline__ double dt_candidate(const double *w, double e_cons, const double *dx,
                                                int ndim, double gm1) {
-  const double e_internal =
-      (e_cons - 0.5 * w[IDN] * (w[IV1] * w[IV1] + w[IV2] * w[IV2] + w[IV3] * w[IV3])) / w[IDN];
+#if APH_EXACT
+  const double e_internal = div_x(
+      e_cons - 0.5 * w[IDN] * (w[IV1] * w[IV1] + w[IV2] * w[IV2] + w[IV3] * w[IV3]), w[IDN]);
+#else
+  const double e_internal = div_x(
+      fma(-mul(0.5, w[IDN]), square3(w[IV1], w[IV2], w[IV3]), e_cons), w[IDN]);
+#endif
   const double bulkmod = eos_bulk_modulus(gm1, w[IDN], e_internal);
-  double gamma_c, rat;  // bulkmod / p, (e_internal + c^2) rho / p
-  div2(bulkmod, (e_internal + C_LIGHT2) * w[IDN], w[IPR], gamma_c, rat);
-  const double lam = C_LIGHT * sqrt(gamma_c / (1 + rat));
-  double m = dx[0] / (dabs(w[IV1]) + lam);
+  const Den p = den(w[IPR]);
+  const double gamma_c = div_x(bulkmod, p);
+  const double rat = div_x((e_internal + C_LIGHT2) * w[IDN], p);
+  const double root = sqrt_x(div_x(gamma_c, 1 + rat));  // lambda is C times this
+#if APH_EXACT
+  const double lam = C_LIGHT * root;
+  auto rate = [&](int d) { return dabs(w[IV1 + d]) + lam; };
+#else
+  auto rate = [&](int d) { return fma(C_LIGHT, root, dabs(w[IV1 + d])); };
+#endif
+  double m = div_x(dx[0], rate(0));
   if (ndim > 1) {
-    const double c2 = dx[1] / (dabs(w[IV2]) + lam);
+    const double c2 = div_x(dx[1], rate(1));
     m = lt(c2, m) ? c2 : m;
   }
   if (ndim > 2) {
-    const double c3 = dx[2] / (dabs(w[IV3]) + lam);
+    const double c3 = div_x(dx[2], rate(2));
     m = lt(c3, m) ? c3 : m;
   }
   return m;
@@ -963,17 +1143,18 @@ __device__ __forceinline__ double dt_cell(const double *w, double e_cons, const 
   return dt_candidate(w, e_cons, dx, ndim, gc.gm1);
 #else
   if (floored) return dt_candidate(w, e_cons, dx, ndim, gc.gm1);
-  const double lam = sound_speed<true>(w[IDN], w[IPR], 0.0, 0.0, gc);
-  double r = (dabs(w[IV1]) + lam) / dx[0];
+  double num, root;
+  sound_parts<true>(w[IDN], w[IPR], 0.0, 0.0, gc, num, root);
+  double r = div_x(fma(num, root, dabs(w[IV1])), dx[0]);
   if (ndim > 1) {
-    const double r2 = (dabs(w[IV2]) + lam) / dx[1];
+    const double r2 = div_x(fma(num, root, dabs(w[IV2])), dx[1]);
     r = lt(r, r2) ? r2 : r;
   }
   if (ndim > 2) {
-    const double r3 = (dabs(w[IV3]) + lam) / dx[2];
+    const double r3 = div_x(fma(num, root, dabs(w[IV3])), dx[2]);
     r = lt(r, r3) ? r3 : r;
   }
-  return 1.0 / r;
+  return rcp_x(r);
 #endif
 }
 

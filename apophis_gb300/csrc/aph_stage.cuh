@@ -40,7 +40,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // Grid-wide barrier.  Every CTA of the launch is resident (the grid is sized from the
 // occupancy calculator, and launched cooperatively when possible); a wait that outlasts
 // timeout_ns records APH_ERR_TIMEOUT and the CTA leaves, so the launch always ends.
-__device__ __noinline__ bool grid_barrier(StepCtl *ctl, unsigned long long timeout_ns,
+static __device__ __noinline__ bool grid_barrier(StepCtl *ctl, unsigned long long timeout_ns,
                                           unsigned int expected) {
   __shared__ int s_ok;
   __syncthreads();
@@ -201,7 +201,7 @@ __device__ __forceinline__ void store_floored_energy(const StepBlock &X, long lo
   if (changed) X.eraw[c] = e_raw;
 }
 
-__device__ void ghost_cell(const StageArgs &a, const StepBlock &B, long long c) {
+static __device__ void ghost_cell(const StageArgs &a, const StepBlock &B, long long c) {
   const PackDev &p = a.p;
   const int idx[3] = {(int)(c % B.ni), (int)((c / B.ni) % B.nj), (int)(c / ((long long)B.ni * B.nj))};
   bool ghost = false;
@@ -445,38 +445,56 @@ __host__ __device__ constexpr size_t pass_smem_doubles(int recon, int n, int T, 
              : (size_t)V * T * ((n + 2 * (recon == RECON_PLM ? 2 : 1)) + 2 * (n + 2));
 }
 
-// Reconstructed slabs beyond the nvar primitives that shared memory is sized for: the exact
-// build always reconstructs the two adiabatic-index fields; the fast build sizes for
-// constant-gamma items and splits an item of a block where a floor fired (which needs the
-// two extra slabs) into chunks of fewer lines (split_lines).
-#if APH_EXACT
-constexpr int kGammaSlabs = 2;
-#else
-constexpr int kGammaSlabs = 0;
-#endif
+// The arithmetic of a pass item.
+//   ARITH_MAIN   quotients and roots on the integer pipe; exact build: tame windows whose
+//                adiabatic indices are gamma to within kGamMax units of the last place, which
+//                are reconstructed as small integers; fast build: blocks where no floor
+//                fired, with the constant gamma
+//   ARITH_SLABS  exact build only: the same with the indices reconstructed as doubles, two
+//                more slabs (a window near a floor, or gamma at a power of two)
+//   ARITH_IEEE   any window: the IEEE instructions
+// An item whose window or operands leave ARITH_MAIN's range is taken again with one of the
+// others, in chunks of lines that fit the two more slabs (split_lines).
+constexpr int ARITH_MAIN = 0, ARITH_SLABS = 1, ARITH_IEEE = 2;
+constexpr int ITEM_DONE = 0, ITEM_TIMEOUT = 1, ITEM_SLABS = 2, ITEM_IEEE = 3;
 
-// Lines of a chunk that fits the gamma slabs into the shared memory of T lines.
-__host__ __device__ constexpr int split_lines(int T, int nvar) {
-  return (nvar + kGammaSlabs) * T / (nvar + 2) > 1 ? (nvar + kGammaSlabs) * T / (nvar + 2) : 1;
+// The adiabatic-index offsets of an item (exact build), two 16-bit values a cell: the window,
+// the PPM face values, and the left and right states.
+__host__ __device__ constexpr size_t gamma_smem_doubles(int recon, int n, int T) {
+#if APH_EXACT
+  return ((size_t)T * ((n + 2 * (recon == RECON_PPM ? 3 : recon == RECON_PLM ? 2 : 1)) + 2 * (n + 2) +
+                       (recon == RECON_PPM ? n + 3 : 0)) +
+          1) / 2;
+#else
+  return 0;
+#endif
 }
 
-// Doubles between the window region and the TMA staging area: the window (nvar +
-// kGammaSlabs variables) is padded to a multiple of 16 doubles so that the staging area
-// starts 128-byte aligned.
+// What ARITH_MAIN needs for T lines.
+__host__ __device__ constexpr size_t main_smem_doubles(int recon, int n, int T, int nvar) {
+  return pass_smem_doubles(recon, n, T, nvar) + gamma_smem_doubles(recon, n, T);
+}
+
+// Lines of a chunk that fits the two gamma slabs into the shared memory of T lines.
+__host__ __device__ constexpr int split_lines(int T, int nvar) {
+  return nvar * T / (nvar + 2) > 1 ? nvar * T / (nvar + 2) : 1;
+}
+
+// Doubles between the window region and the TMA staging area: the window (nvar variables) is
+// padded to a multiple of 16 doubles so that the staging area starts 128-byte aligned.
 __host__ __device__ constexpr size_t tma_stage_offset(int recon, int n, int T, int nvar) {
-  return ((size_t)(nvar + kGammaSlabs) * T * (n + 2 * (recon == RECON_PPM ? 3 : recon == RECON_PLM ? 2 : 1)) +
-          15) /
-         16 * 16;
+  return ((size_t)nvar * T * (n + 2 * (recon == RECON_PPM ? 3 : recon == RECON_PLM ? 2 : 1)) + 15) / 16 * 16;
 }
 
 // PPM of a pass item's window: W holds V x T lines of cells -G..n+G-1 (row width n + 2G);
 // per cell the second differences D2 and centred differences DD (cells -2..n+1), per face
 // the limited value DPH once (faces -1..n+1), then per cell the parabola limiter writes the
 // left state of face c+1 to SL[c+1] and the right state of face c to SR[c+1] (cells -1..n).
-template <bool TAME>
+// also(0) and also(1) run beside the face and the cell phase (the adiabatic-index offsets).
+template <bool TAME, class ALSO>
 __device__ __forceinline__ void ppm_window(const double *W, double *D2, double *DD, double *DPH,
                                            double *SL, double *SR, int V, int nl, int T, int n,
-                                           int G) {
+                                           int G, ALSO also) {
   const int NW = n + 2 * G;
   const int tid = threadIdx.x, nth = blockDim.x;
   // row v * T + t of the slabs and position i in it, for element it of rows of width w (one
@@ -514,6 +532,7 @@ __device__ __forceinline__ void ppm_window(const double *W, double *D2, double *
         ppm_face<TAME>(w_at(row, f - 1), w_at(row, f), DD[o + f + 1], DD[o + f + 2],
                        D2[o + f + 1], D2[o + f + 2]);
   }
+  also(0);
   __syncthreads();
   const int w2 = n + 2;
   for (int it = tid; it < V * nl * w2; it += nth) {  // cells -1..n
@@ -528,21 +547,26 @@ __device__ __forceinline__ void ppm_window(const double *W, double *D2, double *
     SL[(size_t)row * w2 + c + 1] = ql;
     SR[(size_t)row * w2 + c + 1] = qr;
   }
+  also(1);
 }
 
-// One pass item: lines l0..l0+nl-1 of block B along DIR.  b: the block's index in the pack;
-// tma_phase: the parity of the CTA's next mbarrier phase (TMA items flip it).  Returns false
-// (the same in every thread of the CTA) when a TMA wait ran out: the window is then not used,
-// the item computes and writes nothing, and the caller leaves the launch, whose status is
-// already APH_ERR_TIMEOUT and whose results are invalid.
-template <int DIR, int RECON, int RS>
-__device__ bool pass_item(const StageArgs &a, const StepBlock &B, int b, int l0, int nl, int T,
-                          bool constg, bool deferred, bool first_pass, bool last_pass, double *sm,
-                          unsigned long long &dtmin, unsigned mbar, unsigned &tma_phase) {
+// One pass item: lines l0..l0+nl-1 of block B along DIR, T lines of shared memory.  b: the block's
+// index in the pack; tma_phase: the parity of the CTA's next mbarrier phase (TMA items flip it).
+// Returns ITEM_DONE; or (the same in every thread of the CTA, nothing written) ITEM_TIMEOUT when a
+// TMA wait ran out: the caller leaves the launch, whose status is already APH_ERR_TIMEOUT and
+// whose results are invalid; or ITEM_SLABS / ITEM_IEEE when the item needs that arithmetic.
+template <int DIR, int RECON, int RS, int ARITH>
+__device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B, int b, int l0, int nl, int T,
+                                         bool constg, bool deferred, bool first_pass, bool last_pass,
+                                         double *sm, unsigned long long &dtmin, unsigned mbar,
+                                         unsigned &tma_phase) {
   constexpr int G = Halo<RECON>::G;
+  constexpr bool kTame = APH_EXACT && ARITH != ARITH_IEEE;   // the window is tame
+  constexpr bool kOffsets = APH_EXACT && ARITH == ARITH_MAIN;  // gamma as small integers
   const int n = B.nx[DIR - 1];
   const int nv = a.p.nvar;  // 5 hydro variables, then the passive scalars
-  const int V = constg ? nv : nv + 2;  // with gamma_c, gamma_e where the gas is not ideal
+  // with gamma_c, gamma_e as doubles where they are neither constant nor offsets
+  const int V = (ARITH == ARITH_MAIN || constg) ? nv : nv + 2;
   const GasConsts gc = gas_of(a, B);
   const int NW = n + 2 * G;
   const long long nc = B.ncell;
@@ -556,11 +580,23 @@ __device__ bool pass_item(const StageArgs &a, const StepBlock &B, int b, int l0,
   double *SL = (RECON == RECON_PPM) ? DD : SR + (size_t)V * T * (n + 2);  // left states
   double *F = W;                                   // fluxes, after the window is dead
   auto w_at = [&](int v, int t, int c) -> double & { return W[((size_t)v * T + t) * NW + c + G]; };
+#if APH_EXACT
+  // offsets of gamma_c (low half) and gamma_e: window, PPM face values, states
+  int *GW = (int *)(sm + pass_smem_doubles(RECON, n, T, nv));
+  int *GL = GW + T * NW, *GR = GL + T * (n + 2), *GD = GR + T * (n + 2);
+  const long long gbase = __double_as_longlong(gc.gamma);
+  const int godd = (int)gbase & 1;
+  auto pack2 = [](int c, int e) { return (int)((unsigned)(c & 0xffff) | ((unsigned)e << 16)); };
+  auto low = [](int x) { return (int)(short)(x & 0xffff); };
+  auto high = [](int x) { return x >> 16; };
+#endif
 
   // A: load the window of prim (and gamma) along each line
-  bool tame_ok = true;  // exact mode: whether every window value is tame (aph_math.cuh)
+  bool tame_ok = true;    // exact: whether every window value is tame (aph_math.cuh)
+  bool offset_ok = true;  // and every adiabatic index near gamma, inside its binade
   (void)tame_ok;
-  if (a.tmaps && constg) {
+  (void)offset_ok;
+  if (!APH_EXACT && ARITH == ARITH_MAIN && a.tmaps) {
     // one tensor copy of the T lines' whole extent into the staging area, then the window
     // cells -G..n+G-1 into W (the staging layout is [v][t][i] along x, [v][w][t] along y, z)
     // 128-byte aligned staging area after the window region (the size reserves the slack)
@@ -591,7 +627,7 @@ __device__ bool pass_item(const StageArgs &a, const StepBlock &B, int b, int l0,
     }
     const bool arrived = mbar_wait_bounded(mbar, tma_phase, a.ctl, a.timeout_ns);
     tma_phase ^= 1u;
-    if (__syncthreads_or(!arrived)) return false;
+    if (__syncthreads_or(!arrived)) return ITEM_TIMEOUT;
     for (int it = tid; it < nv * nl * NW; it += nth) {
       const int v = it / (nl * NW);
       const int r = it - v * nl * NW;
@@ -620,16 +656,23 @@ __device__ bool pass_item(const StageArgs &a, const StepBlock &B, int b, int l0,
       for (int v = 0; v < nv; ++v) {
         const double x = flip_if(S->prim[v * snc + cell], v == flipv);
         W[((size_t)v * T + t) * NW + w] = x;
-#if APH_EXACT
-        tame_ok = tame_ok && tame(x);
-#endif
+        if (kTame) tame_ok = tame_ok && tame(x);
       }
+#if APH_EXACT
+      if (kOffsets) {
+        const long long kc = __double_as_longlong(S->gamma[cell]) - gbase;
+        const long long ke = __double_as_longlong(S->gamma[snc + cell]) - gbase;
+        offset_ok = offset_ok && (unsigned long long)(kc + kGamMax) <= 2u * kGamMax &&
+                    (unsigned long long)(ke + kGamMax) <= 2u * kGamMax;
+        GW[t * NW + w] = pack2((int)kc, (int)ke);
+      }
+#endif
       if (V > nv) {
         double g_c, g_e;
 #if APH_EXACT
         g_c = S->gamma[cell];
         g_e = S->gamma[snc + cell];
-        tame_ok = tame_ok && tame(g_c) && tame(g_e);
+        if (kTame) tame_ok = tame_ok && tame(g_c) && tame(g_e);
 #else
         // the fast ConsToPrim leaves the constants where no floor fired; the reference's
         // values (which the limiters see) are recomputed from the cell's state there (a
@@ -651,19 +694,43 @@ __device__ bool pass_item(const StageArgs &a, const StepBlock &B, int b, int l0,
     }
   }
 #if APH_EXACT
-  // every window value tame: the reconstruction takes the integer-pipe forms (same bits)
-  const bool tame_item = __syncthreads_and(tame_ok) != 0;
+  if (kOffsets) {
+    // gamma far enough from the ends of its binade for the offsets of all face values
+    const unsigned long long gm = (unsigned long long)gbase & 0xfffffffffffffULL;
+    if (!__syncthreads_and(tame_ok && offset_ok && gm >= 4096 && gm <= 0xfffffffffffffULL - 4096)) return ITEM_SLABS;
+  } else if (kTame) {
+    if (!__syncthreads_and(tame_ok)) return ITEM_IEEE;
+  } else {
+    __syncthreads();
+  }
 #else
   __syncthreads();
 #endif
   // B-D: reconstruction; left state of face c+1 -> SL[c+1], right state of face c -> SR[c+1]
   if (RECON == RECON_PPM) {
+    ppm_window<kTame>(W, D2, DD, DPH, SL, SR, V, nl, T, n, G, [&](int phase) {
 #if APH_EXACT
-    if (tame_item)
-      ppm_window<true>(W, D2, DD, DPH, SL, SR, V, nl, T, n, G);
-    else
+      if (!kOffsets) return;
+      if (phase == 0) {
+        for (int it = tid; it < nl * (n + 3); it += nth) {  // faces -1..n+1
+          const int t = it / (n + 3), f = it - t * (n + 3) - 1;
+          const int *g = GW + t * NW + f + G;
+          GD[it] = pack2(gam_face(low(g[-2]), low(g[-1]), low(g[0]), low(g[1]), godd),
+                         gam_face(high(g[-2]), high(g[-1]), high(g[0]), high(g[1]), godd));
+        }
+      } else {
+        for (int it = tid; it < nl * (n + 2); it += nth) {  // cells -1..n
+          const int t = it / (n + 2), c = it - t * (n + 2) - 1;
+          const int *g = GW + t * NW + c + G, *f = GD + t * (n + 3) + c + 1;
+          int lc, rc, le, re;
+          gam_cell(low(g[-1]), low(g[0]), low(g[1]), low(f[0]), low(f[1]), lc, rc);
+          gam_cell(high(g[-1]), high(g[0]), high(g[1]), high(f[0]), high(f[1]), le, re);
+          GL[it] = pack2(lc, le);
+          GR[it] = pack2(rc, re);
+        }
+      }
 #endif
-      ppm_window<false>(W, D2, DD, DPH, SL, SR, V, nl, T, n, G);
+    });
   } else {
     const int w2 = n + 2;
     for (int it = tid; it < V * nl * w2; it += nth) {
@@ -679,6 +746,21 @@ __device__ bool pass_item(const StageArgs &a, const StepBlock &B, int b, int l0,
       SL[((size_t)v * T + t) * w2 + c + 1] = ql;
       SR[((size_t)v * T + t) * w2 + c + 1] = qr;
     }
+#if APH_EXACT
+    if (kOffsets) {
+      for (int it = tid; it < nl * w2; it += nth) {
+        const int t = it / w2, c = it - t * w2 - 1;
+        const int *g = GW + t * NW + c + G;
+        int lc = low(g[0]), le = high(g[0]), rc = lc, re = le;
+        if (RECON == RECON_PLM) {
+          gam_plm(low(g[-1]), low(g[0]), low(g[1]), godd, lc, rc);
+          gam_plm(high(g[-1]), high(g[0]), high(g[1]), godd, le, re);
+        }
+        GL[it] = pack2(lc, le);
+        GR[it] = pack2(rc, re);
+      }
+    }
+#endif
   }
   __syncthreads();
   // E: Riemann solve on faces 0..n
@@ -688,6 +770,7 @@ __device__ bool pass_item(const StageArgs &a, const StepBlock &B, int b, int l0,
     constexpr int ivz = IV1 + ((ivx - IV1) + 2) % 3;
     const int w2 = n + 2, w1 = n + 1;
     const size_t vs = (size_t)T * w2;
+    bool in_range = true;
     for (int it = tid; it < nl * w1; it += nth) {
       const int t = it / w1, f = it - t * w1;
       const size_t oL = (size_t)t * w2 + f, oR = oL + 1;
@@ -696,21 +779,31 @@ __device__ bool pass_item(const StageArgs &a, const StepBlock &B, int b, int l0,
       wl[IV3] = SL[ivz * vs + oL]; wl[IPR] = SL[IPR * vs + oL];
       wr[IDN] = SR[IDN * vs + oR]; wr[IV1] = SR[ivx * vs + oR]; wr[IV2] = SR[ivy * vs + oR];
       wr[IV3] = SR[ivz * vs + oR]; wr[IPR] = SR[IPR * vs + oR];
+      double glc = 0.0, gle = 0.0, grc = 0.0, gre = 0.0;
 #if APH_EXACT
-      if (tame_item)
-        riemann<RS, false, true>(wl, wr, SL[nv * vs + oL], SL[(nv + 1) * vs + oL], SR[nv * vs + oR],
-                                 SR[(nv + 1) * vs + oR], gc, flx);
-      else
-        riemann<RS, false, false>(wl, wr, SL[nv * vs + oL], SL[(nv + 1) * vs + oL], SR[nv * vs + oR],
-                                  SR[(nv + 1) * vs + oR], gc, flx);
-#else
-      if (constg) {
-        riemann<RS, true>(wl, wr, 0.0, 0.0, 0.0, 0.0, gc, flx);
-      } else {
-        riemann<RS, false>(wl, wr, SL[nv * vs + oL], SL[(nv + 1) * vs + oL], SR[nv * vs + oR],
-                           SR[(nv + 1) * vs + oR], gc, flx);
+      if (kOffsets) {
+        const int gl = GL[oL], gr = GR[oR];
+        glc = __longlong_as_double(gbase + low(gl));
+        gle = __longlong_as_double(gbase + high(gl));
+        grc = __longlong_as_double(gbase + low(gr));
+        gre = __longlong_as_double(gbase + high(gr));
       }
 #endif
+      if (V > nv) {
+        glc = SL[nv * vs + oL];
+        gle = SL[(nv + 1) * vs + oL];
+        grc = SR[nv * vs + oR];
+        gre = SR[(nv + 1) * vs + oR];
+      }
+      if (ARITH == ARITH_IEEE) {
+        IeeeOps o;
+        if (!APH_EXACT && constg) riemann<RS, true, false>(wl, wr, 0.0, 0.0, 0.0, 0.0, gc, flx, o);
+        else riemann<RS, false, false>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+      } else {
+        IntOps o;
+        riemann<RS, !APH_EXACT, kTame>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+        in_range = in_range && o.ok();
+      }
       // store in cons order
       const size_t fs = (size_t)T * w1;
       const size_t of = (size_t)t * w1 + f;
@@ -723,8 +816,9 @@ __device__ bool pass_item(const StageArgs &a, const StepBlock &B, int b, int l0,
       for (int v = NHYDRO; v < nv; ++v)
         F[v * fs + of] = flx[IDN] * (!is_neg(flx[IDN]) ? SL[v * vs + oL] : SR[v * vs + oR]);
     }
+    if (ARITH == ARITH_IEEE) __syncthreads();
+    else if (!__syncthreads_and(in_range)) return ITEM_IEEE;
   }
-  __syncthreads();
   if (a.cf) {  // keep the boundary-face fluxes of every line for the coarse-fine correction
     const int w1 = n + 1;
     const size_t fs = (size_t)T * w1;
@@ -853,6 +947,51 @@ __device__ bool pass_item(const StageArgs &a, const StepBlock &B, int b, int l0,
     }
   }
   __syncthreads();
+  return ITEM_DONE;
+}
+
+// The rest of an item that left ARITH_MAIN's range: lines lfirst..lfirst+nl-1 in chunks that fit the
+// gamma slabs into the shared memory of T lines (out of line: it is rare).  Returns the least dt
+// candidate.
+template <int DIR, int RECON, int RS>
+static __device__ __noinline__ unsigned long long pass_general(const StageArgs &a, const StepBlock &B, int b,
+                                                               int lfirst, int nl, int T, int flags, double *sm) {
+  const bool constg = flags & 1, deferred = flags & 2, first_pass = flags & 4, last_pass = flags & 8;
+  unsigned long long dtmin = ~0ULL;
+  unsigned unused = 0;
+  const int Tc = constg ? T : split_lines(T, a.p.nvar);
+  for (int o = 0; o < nl; o += Tc) {
+    const int l0 = lfirst + o, n = min(Tc, nl - o);
+#if APH_EXACT
+    if (flags & 16)  // the window may be tame
+      if (pass_item<DIR, RECON, RS, ARITH_SLABS>(a, B, b, l0, n, Tc, false, deferred, first_pass, last_pass, sm,
+                                                 dtmin, 0, unused) == ITEM_DONE)
+        continue;
+#endif
+    __syncthreads();
+    pass_item<DIR, RECON, RS, ARITH_IEEE>(a, B, b, l0, n, Tc, constg, deferred, first_pass, last_pass, sm, dtmin, 0,
+                                          unused);
+  }
+  return dtmin;
+}
+
+// An item of any block: ARITH_MAIN where it applies, the rest otherwise.  False on a timeout.
+template <int DIR, int RECON, int RS>
+__device__ __forceinline__ bool pass_any(const StageArgs &a, const StepBlock &B, int b, int lfirst, int nl, int T,
+                                         bool constg, bool deferred, bool first_pass, bool last_pass, double *sm,
+                                         unsigned long long &dtmin, unsigned mbar, unsigned &tma_phase) {
+  int r = ITEM_IEEE;
+  if (APH_EXACT || constg) {
+    r = pass_item<DIR, RECON, RS, ARITH_MAIN>(a, B, b, lfirst, nl, T, constg, deferred, first_pass, last_pass, sm,
+                                              dtmin, mbar, tma_phase);
+    if (r == ITEM_DONE) return true;
+    if (r == ITEM_TIMEOUT) return false;
+    __syncthreads();
+  }
+  const int flags = (constg ? 1 : 0) | (deferred ? 2 : 0) | (first_pass ? 4 : 0) | (last_pass ? 8 : 0) |
+                    (r == ITEM_SLABS ? 16 : 0);
+  const unsigned long long m = pass_general<DIR, RECON, RS>(a, B, b, lfirst, nl, T, flags, sm);
+  dtmin = m < dtmin ? m : dtmin;
   return true;
 }
 
@@ -882,7 +1021,7 @@ __device__ __forceinline__ double amr_fixed_du(const StageArgs &a, const StepBlo
   return x;
 }
 
-__device__ void amr_fix(const StageArgs &a, const Sched &sched, unsigned int *ctr,
+static __device__ void amr_fix(const StageArgs &a, const Sched &sched, unsigned int *ctr,
                         unsigned long long &dtmin) {
   const PackDev &p = a.p;
   for (int it = sched.first(ctr, a.nfix_items); it < a.nfix_items; it = sched.next(ctr, a.nfix_items, it)) {
@@ -952,7 +1091,7 @@ __device__ void amr_fix(const StageArgs &a, const Sched &sched, unsigned int *ct
 // MINB: resident CTAs per SM the registers are budgeted for (1: as many registers as the code
 // wants; 3: capped near 80 per thread for 256-thread CTAs, trading a few spills for occupancy).
 template <int RECON, int RS, int MINB>
-__global__ void __launch_bounds__(kStageThreads, MINB) k_stage(StageArgs a) {
+__global__ void __launch_bounds__(kStageThreads, MINB) k_stage(const __grid_constant__ StageArgs a) {
   extern __shared__ __align__(128) double sm[];
   __shared__ __align__(8) unsigned long long s_mbar;
   const unsigned mbar = smem_addr(&s_mbar);
@@ -1043,7 +1182,7 @@ __global__ void __launch_bounds__(kStageThreads, MINB) k_stage(StageArgs a) {
     B.gamma[c] = g_c;
     B.gamma[nc + c] = g_e;
     if (p.nvar > NHYDRO) {  // passive scalars: concentration = cons / floored density
-      const double di = 1.0 / u[IDN];
+      const double di = rcp_x(u[IDN]);
       for (int n = NHYDRO; n < p.nvar; ++n) {
         const double q = B.u0[n * nc + c];
         B.prim[n * nc + c] = q * di;
@@ -1083,22 +1222,17 @@ __global__ void __launch_bounds__(kStageThreads, MINB) k_stage(StageArgs a) {
       const bool constg = a.block_flags[2 * w.x] != epoch;
 #endif
       const bool deferred = first_pass && a.block_flags[2 * w.x + 1] == epoch;
-      // the item's lines, in chunks that fit the gamma slabs where they are reconstructed
-      const int Tc = constg ? Ti : split_lines(Ti, p.nvar);
-      for (int o = 0; o < nl; o += Tc) {
-        const int l0 = lfirst + o, nc = min(Tc, nl - o);
-        bool ok;
-        if (dir == 1)
-          ok = pass_item<1, RECON, RS>(a, B, w.x, l0, nc, Tc, constg, deferred, first_pass, last_pass, sm, dtmin,
-                                       mbar, tma_phase);
-        else if (dir == 2)
-          ok = pass_item<2, RECON, RS>(a, B, w.x, l0, nc, Tc, constg, deferred, first_pass, last_pass, sm, dtmin,
-                                       mbar, tma_phase);
-        else
-          ok = pass_item<3, RECON, RS>(a, B, w.x, l0, nc, Tc, constg, deferred, first_pass, last_pass, sm, dtmin,
-                                       mbar, tma_phase);
-        if (!ok) return;  // a TMA wait ran out (APH_ERR_TIMEOUT is recorded)
-      }
+      bool ok;
+      if (dir == 1)
+        ok = pass_any<1, RECON, RS>(a, B, w.x, lfirst, nl, Ti, constg, deferred, first_pass, last_pass, sm, dtmin,
+                                    mbar, tma_phase);
+      else if (dir == 2)
+        ok = pass_any<2, RECON, RS>(a, B, w.x, lfirst, nl, Ti, constg, deferred, first_pass, last_pass, sm, dtmin,
+                                    mbar, tma_phase);
+      else
+        ok = pass_any<3, RECON, RS>(a, B, w.x, lfirst, nl, Ti, constg, deferred, first_pass, last_pass, sm, dtmin,
+                                    mbar, tma_phase);
+      if (!ok) return;  // a TMA wait ran out (APH_ERR_TIMEOUT is recorded)
     }
     if (!last_pass && !grid_barrier(a.ctl, a.timeout_ns, gridDim.x)) return;
   }
@@ -1114,20 +1248,49 @@ __global__ void __launch_bounds__(kStageThreads, MINB) k_stage(StageArgs a) {
 
 // Failure-path probe: one CTA waits at a grid barrier for one more CTA than the launch has,
 // so the wait runs out after timeout_ns and records APH_ERR_TIMEOUT in ctl.
-__global__ void k_barrier_probe(StepCtl *ctl, unsigned long long timeout_ns) {
+static __global__ void k_barrier_probe(StepCtl *ctl, unsigned long long timeout_ns) {
   grid_barrier(ctl, timeout_ns, gridDim.x + 1);
 }
 
 // ---- host side ---------------------------------------------------------------------------
+// The kernels of one reconstruction, instantiated in a translation unit of their own (each
+// takes a good part of a minute to compile).
+template <int RECON>
+const void *stage_kernel_of(int rs, int reg_cap);
+
+template <int RECON, int MINB>
+static const void *kernel_for_rs(int rs) {
+  if constexpr (RECON == RECON_DC)
+    if (rs == RS_NONE) return (const void *)k_stage<RECON_DC, RS_NONE, MINB>;
+  switch (rs) {
+    case RS_HLLE: return (const void *)k_stage<RECON, RS_HLLE, MINB>;
+    case RS_HLLC: return (const void *)k_stage<RECON, RS_HLLC, MINB>;
+    case RS_LHLLC: return (const void *)k_stage<RECON, RS_LHLLC, MINB>;
+    default: return nullptr;
+  }
+}
+
+template <>
+const void *stage_kernel_of<APH_STAGE_RECON>(int rs, int reg_cap) {
+  return reg_cap ? kernel_for_rs<APH_STAGE_RECON, 3>(rs) : kernel_for_rs<APH_STAGE_RECON, 1>(rs);
+}
+
+// What the launches share is compiled with the donor-cell kernels.
+#if APH_STAGE_RECON == 1
+template <>
+const void *stage_kernel_of<RECON_PLM>(int rs, int reg_cap);
+template <>
+const void *stage_kernel_of<RECON_PPM>(int rs, int reg_cap);
+
 cudaError_t launch_barrier_probe(StepCtl *ctl, unsigned long long timeout_ns, cudaStream_t s) {
   k_barrier_probe<<<1, 32, 0, s>>>(ctl, timeout_ns);
   return cudaGetLastError();
 }
 
-// Items of T lines with nvar + kGammaSlabs slabs, and single-line chunks with the gamma slabs
-// (split_lines never returns less than one line).
+// Items of T lines, and single-line chunks with the gamma slabs (split_lines never returns less
+// than one line).
 size_t stage_smem_bytes(int recon, int n, int T, int nvar) {
-  const size_t a = pass_smem_doubles(recon, n, T, nvar + kGammaSlabs);
+  const size_t a = main_smem_doubles(recon, n, T, nvar);
   const size_t b = pass_smem_doubles(recon, n, 1, nvar + 2);
   return (a > b ? a : b) * sizeof(double);
 }
@@ -1135,36 +1298,19 @@ size_t stage_smem_bytes(int recon, int n, int T, int nvar) {
 // With TMA staging: the window region padded to 128 bytes, then the larger of the remaining
 // pass regions and the staging area (nvar variables x T lines x the line's entire extent L).
 size_t stage_smem_bytes_tma(int recon, int n, int T, int L, int nvar) {
-  const int V = nvar + kGammaSlabs;
-  const size_t rest = pass_smem_doubles(recon, n, T, V) -
-                      (size_t)V * T * (n + 2 * (recon == RECON_PPM ? 3 : recon == RECON_PLM ? 2 : 1));
+  const size_t rest = pass_smem_doubles(recon, n, T, nvar) -
+                      (size_t)nvar * T * (n + 2 * (recon == RECON_PPM ? 3 : recon == RECON_PLM ? 2 : 1));
   const size_t stage = (size_t)2 * nvar * T * L;  // two boxes for items that cross a plane
   const size_t tma = (tma_stage_offset(recon, n, T, nvar) + 16 + (rest > stage ? rest : stage)) * sizeof(double);
   const size_t plain = stage_smem_bytes(recon, n, T, nvar);
   return tma > plain ? tma : plain;
 }
 
-template <int RECON, int MINB>
-static const void *kernel_for_rs(int rs) {
-  switch (rs) {
-    case RS_HLLE: return (const void *)k_stage<RECON, RS_HLLE, MINB>;
-    case RS_HLLC: return (const void *)k_stage<RECON, RS_HLLC, MINB>;
-    case RS_LHLLC: return (const void *)k_stage<RECON, RS_LHLLC, MINB>;
-    case RS_NONE: return RECON == RECON_DC ? (const void *)k_stage<RECON_DC, RS_NONE, MINB> : nullptr;
-    default: return nullptr;
-  }
-}
-
-template <int MINB>
-static const void *stage_kernel_t(int recon, int rsolver) {
-  if (recon == RECON_PPM) return kernel_for_rs<RECON_PPM, MINB>(rsolver);
-  if (recon == RECON_PLM) return kernel_for_rs<RECON_PLM, MINB>(rsolver);
-  if (recon == RECON_DC) return kernel_for_rs<RECON_DC, MINB>(rsolver);
-  return nullptr;
-}
-
 const void *stage_kernel(int recon, int rsolver, int reg_cap) {
-  return reg_cap ? stage_kernel_t<3>(recon, rsolver) : stage_kernel_t<1>(recon, rsolver);
+  if (recon == RECON_PPM) return stage_kernel_of<RECON_PPM>(rsolver, reg_cap);
+  if (recon == RECON_PLM) return stage_kernel_of<RECON_PLM>(rsolver, reg_cap);
+  if (recon == RECON_DC) return stage_kernel_of<RECON_DC>(rsolver, reg_cap);
+  return nullptr;
 }
 
 cudaError_t stage_occupancy(int recon, int rsolver, int threads, size_t smem, int reg_cap, int *blocks) {
@@ -1192,5 +1338,6 @@ cudaError_t launch_stage(const StageArgs &a, int recon, int rsolver, int grid, i
   void *args[] = {(void *)&a};
   return cudaLaunchKernelExC(&cfg, k, args);
 }
+#endif
 
 }  // namespace APH_NS

@@ -1,0 +1,80 @@
+"""Quotients, reciprocals and square roots on the integer pipe against IEEE arithmetic, and the
+exact stepper where a pass item leaves that arithmetic's range (far operands, a gamma at a power of
+two), against the oracle: equality of every bit, so no tolerance."""
+import ctypes
+import dataclasses
+
+import numpy as np
+import pytest
+import torch
+
+from apophis_gb300 import _capi, hydro, problems
+from apophis_gb300.stepper import Stepper
+
+pytestmark = pytest.mark.gpu
+SIG = [0, 1, 2, 3, (1 << 52) - 1, (1 << 52) - 2, (1 << 51), (1 << 51) - 1, (1 << 51) + 1, (1 << 29) - 1, 1 << 29]
+DIV, RCP, SQRT = 8, 9, 10
+
+
+def _values(rng, n, lo, hi):
+    """n values of either sign with exponents in lo..hi, a third of them with edge significands."""
+    m = rng.integers(0, 1 << 52, n, dtype=np.uint64)
+    edge = rng.integers(0, 3, n) == 0
+    m[edge] = np.array(SIG, np.uint64)[rng.integers(0, len(SIG), int(edge.sum()))]
+    e = rng.integers(lo + 1023, hi + 1024, n).astype(np.uint64)
+    s = rng.integers(0, 2, n).astype(np.uint64)
+    return (m | (e << np.uint64(52)) | (s << np.uint64(63))).view(np.float64)
+
+
+def _run(op, x, y):
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    out = torch.empty_like(xd)
+    _capi.call("aph_diag_exact_ops2", op, ctypes.c_void_p(xd.data_ptr()), ctypes.c_void_p(yd.data_ptr()),
+               ctypes.c_void_p(out.data_ptr()), x.size, hydro.stream_handle())
+    return out.cpu().numpy()
+
+
+def _same(got, want):
+    bad = (got.view(np.uint64) != want.view(np.uint64)) & ~(np.isnan(got) & np.isnan(want))
+    assert not bad.any(), (int(bad.sum()), got[bad][:3], want[bad][:3])
+
+
+@pytest.mark.parametrize("lo,hi", [(-1, 1), (-400, 400), (-405, -395), (395, 405), (-1022, 1023)])
+def test_quotients_and_roots_are_ieee(lo, hi):
+    rng = np.random.default_rng(10_000 + lo * 7 + hi)
+    special = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, -2.2e-308, 1.7e308, 1.0, 3.0])
+    a, b = (np.concatenate([_values(rng, 400_000, lo, hi), v]) for v in
+            (np.repeat(special, special.size), np.tile(special, special.size)))
+    # quotients next to representable numbers: b * q rounded, and its neighbours
+    q = _values(rng, 100_000, 0, 0)
+    c = _values(rng, 100_000, max(lo, -400), min(hi, 400))
+    near = np.nextafter(c * q, np.where(rng.integers(0, 2, q.size) == 0, np.inf, -np.inf))
+    a, b = np.concatenate([a, near, c * q]), np.concatenate([b, c, c])
+    with np.errstate(all="ignore"):
+        _same(_run(DIV, a, b), a / b)
+        _same(_run(RCP, a, b), 1.0 / b)
+        _same(_run(SQRT, a, b), np.sqrt(a))
+        r = _values(rng, 100_000, 0, 1)  # roots next to representable numbers
+        _same(_run(SQRT, r * r, r), np.sqrt(r * r))
+
+
+@pytest.mark.parametrize("recon,rsolver", [("ppm", "hllc"), ("plm", "hlle"), ("ppm", "lhllc"), ("dc", "hllc")])
+@pytest.mark.parametrize("gamma,scale", [(2.0, 0), (1.5, 0), (1.0 + 2.0 ** -9, 0), (5.0 / 3.0, -150),
+                                         (5.0 / 3.0, 190), (1.4, -260)])
+def test_exact_stepper_outside_the_main_path(recon, rsolver, gamma, scale):
+    """One RK2 step equals the oracle: gamma at and near powers of two (no small-integer indices),
+    densities and energies far from 1 (2^scale: products and quotients beyond the integer pipe's
+    range, then windows that are not tame)."""
+    from oracle import oracle as O
+    cfg, cons = problems.kh2d(n=32, block=16, ng=3, recon=recon, rsolver=rsolver, gamma=gamma)
+    cfg = dataclasses.replace(cfg, dfloor=0.0, pfloor=0.0)
+    cons = cons * 2.0 ** scale
+    ref = O.Mesh(cfg)
+    ref.set_cons(cons)
+    ref.run(nsteps=2)
+    st = Stepper(cfg, cons, exact=True)
+    st.step(2)
+    sk, sj, si = cfg.interior
+    _same(np.ascontiguousarray(st.state()[:, :, sk, sj, si]), np.ascontiguousarray(ref.get()[:, :, sk, sj, si]))
+    assert st.status()["dt"] == ref.state()["dt"]
+    st.close()
