@@ -68,6 +68,8 @@ struct StepBlock {
   long long ncell, nint;
   long long ipre;     // interior cells of the blocks before this one (packed interiors)
   double dx[3];
+  double area[3];     // of a face across each dimension: dx1 dx2, dx0 dx2, dx0 dx1
+  double vol, ivol;   // dx0 dx1 dx2 and its reciprocal
   AmrFaces amr;
 };
 

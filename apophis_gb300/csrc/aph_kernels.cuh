@@ -172,10 +172,15 @@ __global__ void __launch_bounds__(kThreads) k_fluxes(PackDev p, const BlockDev *
     const double glc = sL[nvar * vs + oL], gle = sL[(nvar + 1) * vs + oL];
     const double grc = sR[nvar * vs + oR], gre = sR[(nvar + 1) * vs + oR];
     IntOps o;
-    riemann<RS, false, false>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+#pragma unroll
+    for (int k = 0; k < NHYDRO; ++k) {
+      o.see(wl[k]);
+      o.see(wr[k]);
+    }
+    riemann<RS, false>(wl, wr, glc, gle, grc, gre, gc, flx, o);
     if (!o.ok()) {  // an operand outside the integer pipe's range
       IeeeOps ieee;
-      riemann<RS, false, false>(wl, wr, glc, gle, grc, gre, gc, flx, ieee);
+      riemann<RS, false>(wl, wr, glc, gle, grc, gre, gc, flx, ieee);
     }
     flux[IDN * fn + fcell] = flx[IDN];
     flux[ivx * fn + fcell] = flx[IV1];

@@ -35,11 +35,11 @@ constexpr double PPM_C2 = 1.25;                  // ppm_simple.hpp:36
 // ---- integer-pipe predicates ------------------------------------------------
 __device__ __forceinline__ bool is_neg(double x) {  // x < 0.0
   const int hi = __double2hiint(x), lo = __double2loint(x);
-  return hi < 0 && ((((unsigned)hi) << 1) | (unsigned)lo) != 0u;
+  return (hi < 0) & (((((unsigned)hi) << 1) | (unsigned)lo) != 0u);
 }
 __device__ __forceinline__ bool is_pos(double x) {  // x > 0.0
   const int hi = __double2hiint(x), lo = __double2loint(x);
-  return hi >= 0 && (hi | lo) != 0;
+  return (hi >= 0) & ((hi | lo) != 0);
 }
 // monotone integer key: a < b  <=>  okey(a) < okey(b)  (-0.0 and +0.0 share key 0)
 __device__ __forceinline__ long long okey(double x) {
@@ -52,10 +52,19 @@ __device__ __forceinline__ bool gt(double a, double b) { return okey(a) > okey(b
 // std::min / std::max tie rules (the first argument wins when neither is smaller)
 __device__ __forceinline__ double smin(double a, double b) { return lt(b, a) ? b : a; }
 __device__ __forceinline__ double smax(double a, double b) { return lt(a, b) ? b : a; }
-__device__ __forceinline__ unsigned long long mag(double x) {
-  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+// The sign bit is masked and flipped in PTX, out of the compiler's sight: it would make an FP64
+// instruction (a DADD with an absolute or negated operand) of it.
+__device__ __forceinline__ unsigned abs_hi(double x) {
+  unsigned r;
+  asm("and.b32 %0, %1, 0x7fffffff;" : "=r"(r) : "r"(__double2hiint(x)));
+  return r;
 }
-__device__ __forceinline__ double dabs(double x) { return __longlong_as_double((long long)mag(x)); }
+__device__ __forceinline__ unsigned long long mag(double x) {
+  return ((unsigned long long)abs_hi(x) << 32) | (unsigned)__double2loint(x);
+}
+__device__ __forceinline__ double dabs(double x) {
+  return __hiloint2double((int)abs_hi(x), __double2loint(x));
+}
 // bits of 2*|x| (exact doubling: exponent +1, or a shift for subnormals; overflow -> inf)
 __device__ __forceinline__ unsigned long long twice_mag(double x) {
   const unsigned long long m = mag(x);
@@ -66,7 +75,9 @@ __device__ __forceinline__ unsigned long long twice_mag(double x) {
 }
 // v with its sign flipped when neg (SIGN(s) * v for SIGN in {-1, +1})
 __device__ __forceinline__ double flip_if(double v, bool neg) {
-  return neg ? __longlong_as_double(__double_as_longlong(v) ^ (long long)0x8000000000000000ULL) : v;
+  int hi;
+  asm("xor.b32 %0, %1, %2;" : "=r"(hi) : "r"(__double2hiint(v)), "r"(neg ? 0x80000000u : 0u));
+  return __hiloint2double(hi, __double2loint(v));
 }
 __device__ __forceinline__ double from_bits(unsigned long long b) { return __longlong_as_double((long long)b); }
 // b strictly between a and c: the reference's sign test (b - a) * (c - b) > 0 without the FP64
@@ -75,12 +86,12 @@ __device__ __forceinline__ double from_bits(unsigned long long b) { return __lon
 // order 1e-162).  Fast mode.
 __device__ __forceinline__ bool strictly_between(double a, double b, double c) {
   const long long ka = okey(a), kb = okey(b), kc = okey(c);
-  return (ka < kb && kb < kc) || (ka > kb && kb > kc);
+  return ((ka < kb) & (kb < kc)) | ((ka > kb) & (kb > kc));
 }
 // x beyond both a and b on the same side: the sign test (x - a) * (b - x) < 0.  Fast mode.
 __device__ __forceinline__ bool strictly_outside(double x, double a, double b) {
   const long long kx = okey(x), ka = okey(a), kb = okey(b);
-  return (kx > ka && kx > kb) || (kx < ka && kx < kb);
+  return ((kx > ka) & (kx > kb)) | ((kx < ka) & (kx < kb));
 }
 
 // ---- exact operations on the integer pipe for tame operands -------------------------
@@ -96,19 +107,23 @@ __device__ __forceinline__ bool strictly_outside(double x, double a, double b) {
 __device__ __forceinline__ bool tame(double x) {
   const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
   const unsigned e = hi >> 20;  // biased exponent
-  return (e - (1023u - 200u) <= 400u) || ((hi | (unsigned)__double2loint(x)) == 0u);
+  return (e - (1023u - 200u) <= 400u) | ((hi | (unsigned)__double2loint(x)) == 0u);
 }
 __device__ __forceinline__ bool tame_nz(double x) {  // tame and nonzero
   const unsigned e = ((unsigned)__double2hiint(x) & 0x7fffffffu) >> 20;
   return e - (1023u - 200u) <= 400u;
 }
+// (word by word: from a test of all 64 bits the compiler makes a DSETP, an FP64 instruction)
+__device__ __forceinline__ bool is_zero(double x) {
+  return ((((unsigned)__double2hiint(x)) << 1) | (unsigned)__double2loint(x)) == 0u;
+}
 __device__ __forceinline__ double half_x(double x) {
-  const long long b = __double_as_longlong(x);
-  return (b << 1) == 0 ? x : __longlong_as_double(b - (1LL << 52));
+  const int hi = __double2hiint(x);
+  return __hiloint2double(is_zero(x) ? hi : hi - 0x100000, __double2loint(x));
 }
 __device__ __forceinline__ double twice_x(double x) {
-  const long long b = __double_as_longlong(x);
-  return (b << 1) == 0 ? x : __longlong_as_double(b + (1LL << 52));
+  const int hi = __double2hiint(x);
+  return __hiloint2double(is_zero(x) ? hi : hi + 0x100000, __double2loint(x));
 }
 // x / 6.0 correctly rounded, on the integer pipe: x / 6 = (x / 3) / 2, and with the significand
 // moved left by one or two bits to N, the quotient's significand is the integer nearest N / 3,
@@ -128,7 +143,7 @@ __device__ __forceinline__ double div6_x(double x) {
   // the exponent falls by 3 (2 if top), and m's leading bit adds one
   const unsigned e = (hi & 0xfff00000u) - (4u - top) * 0x100000u;
   const unsigned long long r = m + ((unsigned long long)e << 32);
-  return __longlong_as_double((long long)((u << 1) == 0 ? u : r));  // +-0 / 6 = +-0
+  return is_zero(x) ? x : __longlong_as_double((long long)r);  // +-0 / 6 = +-0
 }
 
 // ---- IEEE double additions and small multiplications on the integer pipe ---------------
@@ -214,7 +229,7 @@ __device__ __forceinline__ double mulk_x(double x) {
   const unsigned long long m = (P + ((1ULL << (sh - 1)) - 1 + ((P >> sh) & 1))) >> sh;  // to even
   const unsigned e = (hi & 0xfff00000u) + (unsigned)(s0 + S2 - 1 + (int)longer) * 0x100000u;
   const unsigned long long r = m + ((unsigned long long)e << 32);
-  return __longlong_as_double((long long)((u << 1) == 0 ? u : r));  // k * +-0 = +-0
+  return is_zero(x) ? x : __longlong_as_double((long long)r);  // k * +-0 = +-0
 }
 
 // ---- correctly rounded quotients, reciprocals and square roots on the integer pipe ------
@@ -309,7 +324,6 @@ __device__ __forceinline__ unsigned far_of(double x) {
 __device__ __forceinline__ unsigned far_of_signed(double x) {
   return ((unsigned)__double2hiint(x) >> 20) - 623u;
 }
-__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
 
 // A denominator and its reciprocal word, which several quotients may share.
 struct Den {
@@ -321,6 +335,7 @@ struct Den {
 // collects the largest distance over all operands, and the caller takes the whole solve again
 // with IeeeOps where it exceeds kFar.  div0 allows a numerator of zero.
 struct IntOps {
+  static constexpr bool kInt = true;
   unsigned far = 0;
   __device__ __forceinline__ Den den(double b) {
     far = max(far, far_of(b));
@@ -345,15 +360,41 @@ struct IntOps {
     far = max(far, far_of_signed(x));
     return sqrt_bits((unsigned long long)__double_as_longlong(x));
   }
+  // RN(a b), a and b zero or normal: the 106-bit product of the significands, rounded by a carry
+  // chain.  13 SM-cycles per warp on pipes of its own, where a DMUL holds the FP64 pipe for 17.
+  __device__ __forceinline__ double mul(double a, double b) {
+    const unsigned long long ua = (unsigned long long)__double_as_longlong(a);
+    const unsigned long long ub = (unsigned long long)__double_as_longlong(b);
+    const unsigned ea = (unsigned)(ua >> 52) & 0x7ffu, eb = (unsigned)(ub >> 52) & 0x7ffu;
+    unsigned __int128 P = (unsigned __int128)significand(ua) * (significand(ub) << 11);
+    const unsigned low = (unsigned)((unsigned long long)(P >> 64) >> 52) ^ 1u;  // 1: below 2^116
+    P <<= low;
+    P += 0x7fffffffffffffffULL + ((unsigned)(unsigned long long)(P >> 64) & 1u);  // to even
+    const unsigned e = ea + eb - 1023u - low;  // the leading bit of the significand adds one
+    const unsigned long long sg = (ua ^ ub) & 0x8000000000000000ULL;
+    const bool z = min(ea, eb) == 0u;
+    far = max(far, z ? 0u : e - 622u);
+    return __longlong_as_double(
+        (long long)(z ? sg : (((unsigned long long)(P >> 64) + ((unsigned long long)(e << 20) << 32)) | sg)));
+  }
+  __device__ __forceinline__ double half(double x) { return half_x(x); }
+  // an input: zero or inside the range
+  __device__ __forceinline__ void see(double x) { far = max(far, is_zero(x) ? 0u : far_of(x)); }
+  __device__ __forceinline__ void give_up() { far = ~0u; }
   __device__ __forceinline__ bool ok() const { return far <= kFar; }
 };
 struct IeeeOps {
+  static constexpr bool kInt = false;
   __device__ __forceinline__ Den den(double b) { return Den{b, 0u}; }
   __device__ __forceinline__ double div(double a, const Den &d) { return __ddiv_rn(a, d.b); }
   __device__ __forceinline__ double div0(double a, const Den &d) { return __ddiv_rn(a, d.b); }
   __device__ __forceinline__ double div(double a, double b) { return __ddiv_rn(a, b); }
   __device__ __forceinline__ double rcp(double b) { return __drcp_rn(b); }
   __device__ __forceinline__ double sqrt(double x) { return __dsqrt_rn(x); }
+  __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+  __device__ __forceinline__ double half(double x) { return __dmul_rn(0.5, x); }
+  __device__ __forceinline__ void see(double) {}
+  __device__ __forceinline__ void give_up() {}
   __device__ __forceinline__ bool ok() const { return true; }
 };
 
@@ -374,6 +415,14 @@ __device__ __forceinline__ double rcp_x(double b) {
   if (far_of(b) > kFar) return __drcp_rn(b);
   return quot_bits(0x3ff0000000000000ULL, (unsigned long long)__double_as_longlong(b), den(b).R);
 }
+__device__ __forceinline__ double mul_x(double a, double b) {
+  IntOps o;
+  o.see(a);
+  o.see(b);
+  const double r = o.mul(a, b);
+  if (!o.ok()) return __dmul_rn(a, b);
+  return r;
+}
 __device__ __forceinline__ double sqrt_x(double x) {
   if (is_zero(x)) return x;
   if (far_of_signed(x) > kFar) return __dsqrt_rn(x);
@@ -390,44 +439,66 @@ struct GasConsts {
 };
 
 // ---- ideal gas (singularity-eos IdealGas) ------------------------------------
-__device__ __forceinline__ double eos_bulk_modulus(double gm1, double rho, double sie) {
-  const double small = 10.0 * 2.2250738585072014e-308;
-  const double b = gm1 * (gm1 + 1.0) * rho * sie;
-  return lt(small, b) ? b : small;
-}
-
 // The reference's ConsToPrim arithmetic after the density floor (hydro.cpp:502-531), one
 // rounded operation at a time in its order: the fast build contracts products and sums into
 // FMAs, and these values must match the reference bit for bit where they feed the
 // discontinuous PPM limiters (the adiabatic-index fields of blocks where a floor fired, which
 // the fast mode otherwise replaces by the constants) or the non-idempotent pressure floor.
-// u_d: the floored density (rho the same as a denominator), di = 1 / u_d.  Sets u[IEN], w[IPR],
-// g_c, g_e; returns whether the pressure floor fired.
+// u_d: the floored density.  Sets w, g_c, g_e and u[IEN]; returns whether the pressure floor
+// fired (with IntOps, which gives up there, at a zero internal energy and on far operands: not
+// valid then).
+template <class OPS>
 __device__ __forceinline__ bool cons_to_prim_tail(double *u, double *w, double &g_c, double &g_e,
-                                                  double u_d, const Den &rho, double di, double gm1,
-                                                  double pfloor) {
+                                                  double u_d, double gm1, double pfloor, OPS &o) {
+  const Den rho = o.den(u_d);
+  const double di = o.div(1.0, rho);
   const double m1 = u[IM1], m2 = u[IM2], m3 = u[IM3];
-  const double e_k = __dmul_rn(__dmul_rn(0.5, di),
-                               __dadd_rn(__dadd_rn(__dmul_rn(m1, m1), __dmul_rn(m2, m2)), __dmul_rn(m3, m3)));
   double u_e = u[IEN];
-  double sie = div_x(__dsub_rn(u_e, e_k), rho);
-  double w_p = __dmul_rn(__dmul_rn(gm1, u_d), sie);
+  o.see(m1);
+  o.see(m2);
+  o.see(m3);
+  o.see(u_e);
+  w[IDN] = u_d;
+  w[IV1] = o.mul(m1, di);
+  w[IV2] = o.mul(m2, di);
+  w[IV3] = o.mul(m3, di);
+  const double e_k =
+      o.mul(o.half(di), __dadd_rn(__dadd_rn(o.mul(m1, m1), o.mul(m2, m2)), o.mul(m3, m3)));
+  double e_i = __dsub_rn(u_e, e_k);
+  double sie = o.div0(e_i, rho);
+  double w_p = o.mul(o.mul(gm1, u_d), sie);
   w_p = is_neg(w_p) ? 0.0 : w_p;  // eos_pressure
   const bool floored = !gt(w_p, pfloor);
   if (floored) {
-    const double gm1q = __ddiv_rn(w_p, __dmul_rn(u_d, e_k));  // hydro.cpp:517
-    u_e = __dadd_rn(__ddiv_rn(pfloor, gm1q), e_k);
-    w_p = pfloor;
-    sie = div_x(__dsub_rn(u_e, e_k), rho);  // of the floored energy (unchanged otherwise)
+    if (OPS::kInt) {
+      o.give_up();
+    } else {
+      const double gm1q = __ddiv_rn(w_p, __dmul_rn(u_d, e_k));  // hydro.cpp:517
+      u_e = __dadd_rn(__ddiv_rn(pfloor, gm1q), e_k);
+      w_p = pfloor;
+      e_i = __dsub_rn(u_e, e_k);
+      sie = o.div0(e_i, rho);  // of the floored energy (unchanged otherwise)
+    }
   }
   u[IEN] = u_e;
   w[IPR] = w_p;
   const double small = 10.0 * 2.2250738585072014e-308;
-  double b = __dmul_rn(__dmul_rn(__dmul_rn(gm1, __dadd_rn(gm1, 1.0)), u_d), sie);  // eos_bulk_modulus
+  double b = o.mul(o.mul(__dmul_rn(gm1, __dadd_rn(gm1, 1.0)), u_d), sie);  // eos_bulk_modulus
   b = lt(small, b) ? b : small;
-  g_c = div_x(b, w_p);
-  g_e = __dadd_rn(div_x(w_p, __dsub_rn(u_e, e_k)), 1.0);
+  g_c = o.div(b, o.den(w_p));
+  g_e = __dadd_rn(o.div(w_p, o.den(e_i)), 1.0);
   return floored;
+}
+// The same for any state: on the integer pipe, or again with the IEEE instructions.
+__device__ __forceinline__ bool cons_to_prim_any(double *u, double *w, double &g_c, double &g_e,
+                                                 double u_d, double gm1, double pfloor) {
+  IntOps o;
+  const double e = u[IEN];
+  cons_to_prim_tail(u, w, g_c, g_e, u_d, gm1, pfloor, o);
+  if (o.ok()) return false;
+  IeeeOps ieee;
+  u[IEN] = e;
+  return cons_to_prim_tail(u, w, g_c, g_e, u_d, gm1, pfloor, ieee);
 }
 
 // ConsToPrim for one cell (hydro.cpp:459-531, ideal gas).  u[] is updated in place
@@ -439,17 +510,16 @@ __device__ __forceinline__ bool cons_to_prim_cell(double *u, double *w, double &
   const bool dens_ok = gt(u_d, dfloor);
   u_d = dens_ok ? u_d : dfloor;
   u[IDN] = u_d;
-  const Den rho = den(u_d);
-  const double di = div_x(1.0, rho);
-  w[IDN] = u_d;
-  w[IV1] = u[IM1] * di;
-  w[IV2] = u[IM2] * di;
-  w[IV3] = u[IM3] * di;
 #if !APH_EXACT
   // fast: p = gm1 rho ((E - e_k) / rho) = gm1 (E - e_k), and with the floors inactive both
   // adiabatic indices are gamma (B / p = gm1 + 1 = p / (rho e) + 1), so one division per cell
   // (a floored density takes the reference's arithmetic below, whose indices are kept)
   if (dens_ok) {
+    const double di = rcp_x(u_d);
+    w[IDN] = u_d;
+    w[IV1] = __dmul_rn(u[IM1], di);
+    w[IV2] = __dmul_rn(u[IM2], di);
+    w[IV3] = __dmul_rn(u[IM3], di);
     const double pe =
         __dmul_rn(gm1, fma(-__dmul_rn(0.5, di),
                            fma(u[IM3], u[IM3], fma(u[IM1], u[IM1], __dmul_rn(u[IM2], u[IM2]))), u[IEN]));
@@ -462,15 +532,14 @@ __device__ __forceinline__ bool cons_to_prim_cell(double *u, double *w, double &
     }
   }
 #endif
-  return cons_to_prim_tail(u, w, g_c, g_e, u_d, rho, di, gm1, pfloor);
+  return cons_to_prim_any(u, w, g_c, g_e, u_d, gm1, pfloor);
 }
 
 // The reference's adiabatic indices (gamma_c, gamma_e) of a cell whose floors did not fire,
 // from its conserved state after ConsToPrim (u: the cell's five values).
 __device__ __forceinline__ void gamma_ref(const double *u, double gm1, double &g_c, double &g_e) {
   double uu[NHYDRO] = {u[0], u[1], u[2], u[3], u[4]}, w[NHYDRO];
-  const Den rho = den(u[IDN]);
-  cons_to_prim_tail(uu, w, g_c, g_e, u[IDN], rho, div_x(1.0, rho), gm1, -1.0);
+  cons_to_prim_any(uu, w, g_c, g_e, u[IDN], gm1, -1.0);
 }
 
 // ---- reconstruction (src/recon) --------------------------------------------------
@@ -522,17 +591,16 @@ __device__ __forceinline__ double ppm_face(double qm1, double q0, double ddm1, d
     double dph = avg + div6_x(ddm1 - dd0);
     // (dph - qm1) * (q0 - dph) < 0, the differences being nonzero and their product normal; the
     // limited value, which only such a face takes, is formed there
+    // (selects inside: lanes that part in a nested branch would take the last addition one
+    // group after the other)
     if (strictly_outside(dph, qm1, q0)) {
       const double qa = mulk_x<3, 0>(s - twice_x(dph));
-      double qd = 0.0;
       const bool sa = is_neg(qa);
-      if (sa == is_neg(d2m1) && sa == is_neg(d20)) {
-        const unsigned long long mb = mag(d2m1), mc = mag(d20);
-        const double m = mulk_x<5, -2>(from_bits(mc < mb ? mc : mb));  // PPM_C2 = 5/4
-        const unsigned long long mm = mag(m), ma = mag(qa);
-        qd = flip_if(from_bits(ma < mm ? ma : mm), sa);
-      }
-      dph = avg - div6_x(qd);
+      const unsigned long long mb = mag(d2m1), mc = mag(d20), ma = mag(qa);
+      const unsigned long long mm = mag(mulk_x<5, -2>(from_bits(mc < mb ? mc : mb)));  // PPM_C2 = 5/4
+      const bool same = (sa == is_neg(d2m1)) & (sa == is_neg(d20));
+      const double qd = flip_if(from_bits(ma < mm ? ma : mm), sa);
+      dph = avg - div6_x(same ? qd : 0.0);
     }
     return dph;
   }
@@ -573,25 +641,69 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
                                          double q_ip2, double d2m1, double d20, double d2p1,
                                          double dph_lo, double dph_hi, double &ql_ip1,
                                          double &qr_i) {
-  constexpr bool T = APH_EXACT && TAME;
   double qr = dph_lo, ql = dph_hi;
   const double dqf_minus = q_i - qr;
   const double dqf_plus = ql - q_i;
 #if APH_EXACT
-  bool extremum;
-  if (T) {  // the two products' signs, as in ppm_face
-    extremum = !strictly_between(qr, q_i, ql) || !strictly_between(q_im1, q_i, q_ip1);
-  } else {
-    const double qa_tmp = dqf_minus * dqf_plus;
-    const double qb_tmp = (q_ip1 - q_i) * (q_i - q_im1);
-    extremum = !is_pos(qa_tmp) || !is_pos(qb_tmp);
+  if (TAME) {
+    // the states are qr = q_i - xm where sub_m, ql = q_i + xp where add_p: one addition each
+    // for all lanes whatever branch formed the steps
+    double xm = 0.0, xp = 0.0;
+    bool sub_m, add_p;
+    // the signs of the two products of differences, as in ppm_face
+    if (!strictly_between(qr, q_i, ql) | !strictly_between(q_im1, q_i, q_ip1)) {
+      const double d2qf = mulk_x<3, 1>((dph_lo + dph_hi) - twice_x(q_i));
+      const bool sd = is_neg(d2qf);
+      unsigned long long m = mag(d2m1);
+      const unsigned long long m0 = mag(d20), m1 = mag(d2p1), md = mag(d2qf);
+      m = m0 < m ? m0 : m;
+      m = m1 < m ? m1 : m;
+      const unsigned long long ms = mag(mulk_x<5, -2>(from_bits(m)));
+      const bool same = (sd == is_neg(d2m1)) & (sd == is_neg(d20)) & (sd == is_neg(d2p1));
+      const double qe = same ? flip_if(from_bits(md < ms ? md : ms), sd) : 0.0;
+      unsigned long long mx = mag(q_im2);
+      const unsigned long long a1 = mag(q_im1), a2 = mag(q_i), a3 = mag(q_ip1), a4 = mag(q_ip2);
+      mx = a1 > mx ? a1 : mx;
+      mx = a2 > mx ? a2 : mx;
+      mx = a3 > mx ? a3 : mx;
+      mx = a4 > mx ? a4 : mx;
+      // the roundoff guard |d2qf| > 1e-12 * max|q| (ppm_simple.hpp:132): RN(1e-12 * mx), mx tame,
+      // from the product of the significands; 0 > anything is false, a nonzero value over 0 true
+      IntOps o;  // (tame operands: all in range)
+      const bool guard = md > mag(o.mul(1.0e-12, from_bits(mx)));
+      // rho = qe / d2qf with the guard, else +0.  Where it is a zero (of qe's and d2qf's signs with
+      // the guard) the steps are signed zeros; where qe is d2qf it is 1 > 1 - 1e-12: the face
+      // values stay
+      const bool none = is_zero(qe) | !guard;
+      const double rho = o.div(qe, o.den(d2qf));
+      const unsigned rs = guard ? (unsigned)(__double2hiint(qe) ^ __double2hiint(d2qf)) & 0x80000000u : 0u;
+      auto step = [&](double dqf) {
+        const double z = __hiloint2double((int)(rs ^ ((unsigned)__double2hiint(dqf) & 0x80000000u)), 0);
+        const double r = o.mul(rho, dqf);
+        return none ? z : r;
+      };
+      xm = step(dqf_minus);
+      xp = step(dqf_plus);
+      sub_m = add_p = none | le(rho, 1.0 - 1.0e-12);
+    } else {
+      sub_m = mag(dqf_minus) >= twice_mag(dqf_plus);
+      add_p = mag(dqf_plus) >= twice_mag(dqf_minus);
+      xm = twice_x(dqf_plus);
+      xp = twice_x(dqf_minus);
+    }
+    const double rm = q_i - xm, lp = q_i + xp;
+    qr_i = sub_m ? rm : qr;
+    ql_ip1 = add_p ? lp : ql;
+    return;
   }
-  if (extremum) {
+  const double qa_tmp = dqf_minus * dqf_plus;
+  const double qb_tmp = (q_ip1 - q_i) * (q_i - q_im1);
+  if (!is_pos(qa_tmp) || !is_pos(qb_tmp)) {
 #else
   if (!strictly_between(qr, q_i, ql) || !strictly_between(q_im1, q_i, q_ip1)) {
 #endif
     // local extremum: limit with rho = qe/qd (CS eq 22-23, MC eq 27)
-    const double d2qf = T ? mulk_x<3, 1>((dph_lo + dph_hi) - twice_x(q_i)) : 6.0 * (dph_lo + dph_hi - 2.0 * q_i);
+    const double d2qf = 6.0 * (dph_lo + dph_hi - 2.0 * q_i);
     double qe = 0.0;
     const bool sd = is_neg(d2qf);
     if (sd == is_neg(d2m1) && sd == is_neg(d20) && sd == is_neg(d2p1)) {
@@ -599,7 +711,7 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
       const unsigned long long m0 = mag(d20), m1 = mag(d2p1);
       m = m0 < m ? m0 : m;
       m = m1 < m ? m1 : m;
-      const unsigned long long ms = mag(T ? mulk_x<5, -2>(from_bits(m)) : PPM_C2 * from_bits(m));
+      const unsigned long long ms = mag(PPM_C2 * from_bits(m));
       const unsigned long long md = mag(d2qf);
       qe = flip_if(from_bits(md < ms ? md : ms), sd);
     }
@@ -610,50 +722,19 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
     mx = a3 > mx ? a3 : mx;
     mx = a4 > mx ? a4 : mx;
     double rho = 0.0;
-    // the roundoff guard |d2qf| > 1e-12 * max|q| (ppm_simple.hpp:132); RN(1e-12 * mx) lies in
-    // [2^-40, 2^-38) times mx's binade, so the exponents decide it except within two binades
-    bool guard;
-    if (T) {
-      const long long ed = (long long)(mag(d2qf) >> 52), em = (long long)(mx >> 52);
-      if (mag(d2qf) == 0) guard = false;  // 0 > anything is false
-      else if (mx == 0) guard = true;      // a nonzero value over 1e-12 * 0
-      else if (ed >= em - 38) guard = true;
-      else if (ed <= em - 41) guard = false;
-      else guard = mag(d2qf) > mag(1.0e-12 * from_bits(mx));
-    } else {
-      guard = mag(d2qf) > mag(1.0e-12 * from_bits(mx));
-    }
-#if APH_EXACT
-    if (T && ((__double_as_longlong(qe) << 1) == 0 || !guard)) {
-      // rho is a zero (+0 without the guard, else qe / d2qf = +-0 by the signs): the products
-      // rho * dqf are zeros with the product of the signs, and no division is needed
-      const long long rs = guard ? ((__double_as_longlong(qe) ^ __double_as_longlong(d2qf)) &
-                                    (long long)0x8000000000000000ULL) : 0LL;
-      const double zm = __longlong_as_double(rs ^ (__double_as_longlong(dqf_minus) & (long long)0x8000000000000000ULL));
-      const double zp = __longlong_as_double(rs ^ (__double_as_longlong(dqf_plus) & (long long)0x8000000000000000ULL));
-      qr = q_i - zm;
-      ql = q_i + zp;
-    } else if (T && __double_as_longlong(qe) == __double_as_longlong(d2qf)) {
-      // rho = d2qf / d2qf = 1 > 1 - 1e-12: the face values stay
-    } else {
-      if (guard) rho = div_x(qe, d2qf);
-      if (le(rho, 1.0 - 1.0e-12)) {
-        qr = q_i - rho * dqf_minus;
-        ql = q_i + rho * dqf_plus;
-      }
-    }
-#else
-    if (guard) rho = div_x(qe, d2qf);
+    if (mag(d2qf) > mag(1.0e-12 * from_bits(mx))) rho = div_x(qe, d2qf);
     if (le(rho, 1.0 - 1.0e-12)) {
+#if APH_EXACT
+      qr = q_i - rho * dqf_minus;
+      ql = q_i + rho * dqf_plus;
+#else
       qr = fma(-rho, dqf_minus, q_i);
       ql = fma(rho, dqf_plus, q_i);
-    }
 #endif
+    }
   } else {
-    if (mag(dqf_minus) >= twice_mag(dqf_plus))
-      qr = T ? q_i - twice_x(dqf_plus) : q_i - 2.0 * dqf_plus;
-    if (mag(dqf_plus) >= twice_mag(dqf_minus))
-      ql = T ? q_i + twice_x(dqf_minus) : q_i + 2.0 * dqf_minus;
+    if (mag(dqf_minus) >= twice_mag(dqf_plus)) qr = q_i - 2.0 * dqf_plus;
+    if (mag(dqf_plus) >= twice_mag(dqf_minus)) ql = q_i + 2.0 * dqf_minus;
   }
   ql_ip1 = ql;
   qr_i = qr;
@@ -761,7 +842,7 @@ __device__ __forceinline__ void reconstruct(const double *q, double &ql_ip1, dou
 #if APH_EXACT
 template <class OPS>
 __device__ __forceinline__ double sound_speed(double rho, double p, double gamma, double igm1, OPS &o) {
-  return C_LIGHT * o.sqrt(o.div(gamma, 1 + (igm1 + o.div(rho * C_LIGHT2, p))));
+  return o.mul(C_LIGHT, o.sqrt(o.div(gamma, 1 + (igm1 + o.div(o.mul(rho, C_LIGHT2), o.den(p))))));
 }
 
 template <class OPS>
@@ -771,42 +852,39 @@ __device__ __forceinline__ void solve_hlle_exact(const double *wli, const double
   const double igm1l = o.rcp(gle - 1), igm1r = o.rcp(gre - 1);
   const double cl = sound_speed(wli[IDN], wli[IPR], glc, igm1l, o);
   const double cr = sound_speed(wri[IDN], wri[IPR], grc, igm1r, o);
-  const double el = wli[IPR] * igm1l +
-                    0.5 * wli[IDN] * (wli[IV1] * wli[IV1] + wli[IV2] * wli[IV2] + wli[IV3] * wli[IV3]);
-  const double er = wri[IPR] * igm1r +
-                    0.5 * wri[IDN] * (wri[IV1] * wri[IV1] + wri[IV2] * wri[IV2] + wri[IV3] * wri[IV3]);
-  const double rhoa = .5 * (wli[IDN] + wri[IDN]);
-  const double ca = .5 * (cl + cr);
-  const double pmid = .5 * (wli[IPR] + wri[IPR] + (wli[IV1] - wri[IV1]) * rhoa * ca);
+  auto energy = [&](const double *w, double igm1) {
+    return o.mul(w[IPR], igm1) +
+           o.mul(o.half(w[IDN]), o.mul(w[IV1], w[IV1]) + o.mul(w[IV2], w[IV2]) + o.mul(w[IV3], w[IV3]));
+  };
+  const double el = energy(wli, igm1l), er = energy(wri, igm1r);
+  const double rhoa = o.half(wli[IDN] + wri[IDN]);
+  const double ca = o.half(cl + cr);
+  const double pmid = o.half(wli[IPR] + wri[IPR] + o.mul(o.mul(wli[IV1] - wri[IV1], rhoa), ca));
   double ql = 1.0, qr = 1.0;
   if (gt(pmid, wli[IPR]))
-    ql = 1.0 + o.div(glc + 1, o.sqrt(2 * glc)) * (o.div(pmid, wli[IPR]) - 1.0);
+    ql = 1.0 + o.mul(o.div(glc + 1, o.den(o.sqrt(2 * glc))), o.div(pmid, o.den(wli[IPR])) - 1.0);
   if (gt(pmid, wri[IPR]))
-    qr = 1.0 + o.div(grc + 1, o.sqrt(2 * grc)) * (o.div(pmid, wri[IPR]) - 1.0);
-  const double al = wli[IV1] - cl * ql;
-  const double ar = wri[IV1] + cr * qr;
+    qr = 1.0 + o.mul(o.div(grc + 1, o.den(o.sqrt(2 * grc))), o.div(pmid, o.den(wri[IPR])) - 1.0);
+  const double al = wli[IV1] - o.mul(cl, ql);
+  const double ar = wri[IV1] + o.mul(cr, qr);
   const double bp = is_pos(ar) ? ar : 0.0;
   const double bm = is_neg(al) ? al : 0.0;
-  const double vxl = wli[IV1] - bm;
-  const double vxr = wri[IV1] - bp;
-  double fl[NHYDRO], fr[NHYDRO];
-  fl[IDN] = wli[IDN] * vxl;
-  fr[IDN] = wri[IDN] * vxr;
-  fl[IV1] = wli[IDN] * wli[IV1] * vxl;
-  fr[IV1] = wri[IDN] * wri[IV1] * vxr;
-  fl[IV2] = wli[IDN] * wli[IV2] * vxl;
-  fr[IV2] = wri[IDN] * wri[IV2] * vxr;
-  fl[IV3] = wli[IDN] * wli[IV3] * vxl;
-  fr[IV3] = wri[IDN] * wri[IV3] * vxr;
-  fl[IV1] += wli[IPR];
-  fr[IV1] += wri[IPR];
-  fl[IEN] = el * vxl + wli[IPR] * wli[IV1];
-  fr[IEN] = er * vxr + wri[IPR] * wri[IV1];
   double tmp = 0.0;
   if (__double_as_longlong(bp) != __double_as_longlong(bm) && (mag(bp) | mag(bm)) != 0ULL)
-    tmp = o.div0(0.5 * (bp + bm), o.den(bp - bm));
+    tmp = o.div0(o.half(bp + bm), o.den(bp - bm));
+  double fl[NHYDRO], fr[NHYDRO];
+  auto fluxes = [&](const double *w, double b, double e, double *f) {
+    const double vx = w[IV1] - b;
+    f[IDN] = o.mul(w[IDN], vx);
+    f[IV1] = o.mul(o.mul(w[IDN], w[IV1]), vx) + w[IPR];
+    f[IV2] = o.mul(o.mul(w[IDN], w[IV2]), vx);
+    f[IV3] = o.mul(o.mul(w[IDN], w[IV3]), vx);
+    f[IEN] = o.mul(e, vx) + o.mul(w[IPR], w[IV1]);
+  };
+  fluxes(wli, bm, el, fl);
+  fluxes(wri, bp, er, fr);
 #pragma unroll
-  for (int n = 0; n < NHYDRO; ++n) flxi[n] = 0.5 * (fl[n] + fr[n]) + (fl[n] - fr[n]) * tmp;
+  for (int n = 0; n < NHYDRO; ++n) flxi[n] = o.half(fl[n] + fr[n]) + o.mul(fl[n] - fr[n], tmp);
 }
 
 #else
@@ -944,10 +1022,36 @@ __device__ __forceinline__ bool pow2_normal(double x) {
   const unsigned long long e = b >> 52;  // the sign bit must be 0
   return (b & 0xfffffffffffffULL) == 0 && e >= 1 && e <= 2045;
 }
+// x times 2^k, k within +-400: an exponent step for x in range or zero, else the product with c = 2^k
+__device__ __forceinline__ double scale_x(double x, double c, int k) {
+  if (far_of(x) <= kFar)
+    return __longlong_as_double(__double_as_longlong(x) + ((long long)k << 52));
+  return is_zero(x) ? x : x * c;
+}
 // y / vol, correctly rounded; ivol = 1 / vol, p2 = pow2_normal(vol) (uniform over a block)
 __device__ __forceinline__ double div_vol(double y, double vol, double ivol, bool p2) {
-  if (p2) return y * ivol;
-  return div_x(y, vol);
+  if (!p2) return div_x(y, vol);
+  const int k = (__double2hiint(ivol) >> 20) - 1023;
+  return k >= -400 && k <= 400 ? scale_x(y, ivol, k) : y * ivol;
+}
+// RN(RN(gam0 u0) + RN(gam1 u1)) of an RK stage, with the products by 0, 1 and powers of two (every
+// stage of RK1, RK2 and VL2) taken off the FP64 pipe.
+struct RkForm {
+  double gam0, gam1;
+  int form;    // 1: gam0 = 0 and gam1 = 1; 2: both powers of two, exponents k0 and k1; 0: any
+  int k0, k1;
+};
+__device__ __forceinline__ RkForm rk_form(double gam0, double gam1) {
+  RkForm r{gam0, gam1, 0, (__double2hiint(gam0) >> 20) - 1023, (__double2hiint(gam1) >> 20) - 1023};
+  if (gam0 == 0.0 && gam1 == 1.0) r.form = 1;
+  else if (pow2_normal(gam0) && pow2_normal(gam1) && abs(r.k0) <= 400 && abs(r.k1) <= 400) r.form = 2;
+  return r;
+}
+__device__ __forceinline__ double rk_sum(const RkForm &r, double u0, double u1) {
+  // 0 u0 + u1 is u1 unless u1 is a zero (whose sign the sum decides) or u0 not finite
+  if (r.form == 1 && !is_zero(u1) && ((__double2hiint(u0) >> 20) & 0x7ff) != 0x7ff) return u1;
+  if (r.form == 2) return scale_x(u0, r.gam0, r.k0) + scale_x(u1, r.gam1, r.k1);
+  return r.gam0 * u0 + r.gam1 * u1;
 }
 
 #if APH_EXACT
@@ -957,15 +1061,10 @@ __device__ __forceinline__ double div_vol(double y, double vol, double ivol, boo
 // adds less than a quarter ulp of X and returns X, so both are skipped.
 template <class OPS>
 __device__ __forceinline__ double csound_exact(double rho, const Den &p, double gamma, double igm1, OPS &o) {
-  const double X = o.div(rho * C_LIGHT2, p);
+  const double X = o.div(o.mul(rho, C_LIGHT2), p);
   const long long ex = (long long)(mag(X) >> 52), ei = (long long)(mag(igm1) >> 52);
   const double d = (ex >= 1023 + 55 && ex >= ei + 55 && ex < 2047) ? X : 1 + (igm1 + X);
-  return C_LIGHT * o.sqrt(o.div(gamma, d));
-}
-
-// exponent field all ones: an infinity or a NaN
-__device__ __forceinline__ bool nonfinite(double x) {
-  return ((__double2hiint(x) >> 20) & 0x7ff) == 0x7ff;
+  return o.mul(C_LIGHT, o.sqrt(o.div(gamma, o.den(d))));
 }
 
 // HLLC in the exact mode with the reference's roundings (hydro_hllc.hpp:45-145, and the
@@ -976,118 +1075,119 @@ __device__ __forceinline__ bool nonfinite(double x) {
 //  * the contact branch picks its operands instead of its code, so both branches are the
 //    same two divisions: ul = sstar / (sstar - bm), ustar = -bm / (sstar - bm) when
 //    sstar >= 0, else ur = -sstar / (bp - sstar), ustar = bp / (bp - sstar);
-//  * TAME (the reconstruction window was tame): the flux is formed from the upwind side only.
-//    The reference's ul*fl + ur*fr has one weight exactly 0, and RN(a + (+-0)) == a for a
-//    nonzero a, so the other side's term (0 * f, a signed zero: no product of values derived
-//    from a tame window overflows) is added, in the reference's order, only where the upwind
-//    term is zero and the sign of the zero sum depends on it, or where the other side is
-//    not finite.  The halvings and doublings run on the integer pipe (half_x, twice_x).
-//    Without TAME both sides' terms are always formed.
-template <bool LOWMACH, bool TAME, class OPS>
+//  * with IntOps (all operands zero or within 2^-400 .. 2^401) the flux is formed from the upwind
+//    side only.  The reference's ul*fl + ur*fr has one weight exactly 0, and RN(a + (+-0)) == a
+//    for every a but -0: there the other side's term 0 * f is +0 or -0 by the sign of f, which
+//    for the mass and transverse fluxes is that of its factors (the normal momentum's and the
+//    energy's -0 give up).  With IeeeOps both sides' terms are formed.
+template <bool LOWMACH, class OPS>
 __device__ __forceinline__ void solve_hllc_exact(const double *wli, const double *wri, double glc,
                                                  double gle, double grc, double gre, double *flxi,
                                                  OPS &o) {
-  auto hlf = [](double x) { return TAME ? half_x(x) : 0.5 * x; };
   const double gammal = glc, gammar = grc;
   const double igm1l = o.rcp(gle - 1), igm1r = o.rcp(gre - 1);
   // the sound speed and the shock factor divide by the pressures
   const Den pl = o.den(wli[IPR]), pr = o.den(wri[IPR]);
   const double cl = csound_exact(wli[IDN], pl, gammal, igm1l, o);
   const double cr = csound_exact(wri[IDN], pr, gammar, igm1r, o);
-  const double rhoa = hlf(wli[IDN] + wri[IDN]);
-  const double ca = hlf(cl + cr);
-  double pstar;
-  if (!LOWMACH) {
-    pstar = hlf(wli[IPR] + wri[IPR]) - hlf(wri[IV1] - wli[IV1]) * rhoa * ca;
-  } else {
+  const double rhoa = o.half(wli[IDN] + wri[IDN]);
+  const double ca = o.half(cl + cr);
+  auto square3 = [&](const double *w) {
+    return o.mul(w[IV1], w[IV1]) + o.mul(w[IV2], w[IV2]) + o.mul(w[IV3], w[IV3]);
+  };
+  double dp = o.mul(o.mul(o.half(wri[IV1] - wli[IV1]), rhoa), ca);
+  if (LOWMACH) {
     auto root = [&](double x) { return is_zero(x) ? x : o.sqrt(is_zero(x) ? 1.0 : x); };
-    const double machl = root(wli[IV1] * wli[IV1] + wli[IV2] * wli[IV2] + wli[IV3] * wli[IV3]);
-    const double machr = root(wri[IV1] * wri[IV1] + wri[IV2] * wri[IV2] + wri[IV3] * wri[IV3]);
-    const double chi = smax(machl, machr);
-    const double phi = chi * (2.0 - chi);
-    pstar = hlf(wli[IPR] + wri[IPR]) - hlf(wri[IV1] - wli[IV1]) * rhoa * ca * phi;
+    const double chi = smax(root(square3(wli)), root(square3(wri)));
+    dp = o.mul(dp, o.mul(chi, 2.0 - chi));
   }
-  double ql = 1.0, qr = 1.0;
+  const double pstar = o.half(wli[IPR] + wri[IPR]) - dp;
+  double cql = cl, cqr = cr;  // the sound speeds times the shock factors
   const bool bl = gt(pstar, wli[IPR]), br = gt(pstar, wri[IPR]);
   if (bl || br) {
-    const double k = o.div(gammal + 1, TAME ? twice_x(gammar) : 2 * gammar);
-    const double q1 = o.sqrt(1.0 + k * (o.div(pstar, bl ? pl : pr) - 1.0));
-    if (bl) ql = q1;
-    else qr = q1;
-    if (bl && br) qr = o.sqrt(1.0 + k * (o.div(pstar, pr) - 1.0));
+    const double k = o.div(gammal + 1, o.den(2 * gammar));
+    const double q1 = o.mul(bl ? cl : cr, o.sqrt(1.0 + o.mul(k, o.div(pstar, bl ? pl : pr) - 1.0)));
+    if (bl) cql = q1;
+    else cqr = q1;
+    if (bl && br) cqr = o.mul(cr, o.sqrt(1.0 + o.mul(k, o.div(pstar, pr) - 1.0)));
   }
-  const double sl = wli[IV1] - cl * ql;
-  const double sr = wri[IV1] + cr * qr;
+  const double sl = wli[IV1] - cql;
+  const double sr = wri[IV1] + cqr;
   const double bp = is_pos(sr) ? sr : TINY_NUMBER;
   const double bm = is_neg(sl) ? sl : -TINY_NUMBER;
-  const double vxl0 = wli[IV1] - sl;
-  const double vxr0 = wri[IV1] - sr;
-  const double tl = wli[IPR] + vxl0 * wli[IDN] * wli[IV1];
-  const double tr = wri[IPR] + vxr0 * wri[IDN] * wri[IV1];
-  const double ml = wli[IDN] * vxl0;
-  const double mr = -(wri[IDN] * vxr0);
+  const double ml = o.mul(wli[IDN], wli[IV1] - sl);
+  const double xr = o.mul(wri[IDN], wri[IV1] - sr), mr = -xr;
+  const double tl = wli[IPR] + o.mul(ml, wli[IV1]);
+  const double tr = wri[IPR] + o.mul(xr, wri[IV1]);
   const Den m = o.den(ml + mr);
   const double sstar = o.div0(tl - tr, m);
-  double cp = o.div0(ml * tr + mr * tl, m);
+  double cp = o.div0(o.mul(ml, tr) + o.mul(mr, tl), m);
   cp = is_pos(cp) ? cp : 0.0;
   const bool L = !is_neg(sstar);  // sstar >= 0.0
   const Den d = o.den(L ? sstar - bm : bp - sstar);
   const double coef = o.div0(L ? sstar : -sstar, d);  // ul (or ur)
   const double ustar = o.div(L ? -bm : bp, d);
-  // the upwind side (U) and the other one (O)
-  const double *wu = L ? wli : wri, *wo = L ? wri : wli;
-  const double igu = L ? igm1l : igm1r;
-  const double bu = L ? bm : bp, bo = L ? bp : bm;
-  const double vx = wu[IV1] - bu;
-  double f[NHYDRO];
-  f[IDN] = wu[IDN] * vx;
-  f[IV1] = wu[IDN] * wu[IV1] * vx + wu[IPR];
-  f[IV2] = wu[IDN] * wu[IV2] * vx;
-  f[IV3] = wu[IDN] * wu[IV3] * vx;
-  const double eu = wu[IPR] * igu + hlf(wu[IDN]) * (wu[IV1] * wu[IV1] + wu[IV2] * wu[IV2] + wu[IV3] * wu[IV3]);
-  f[IEN] = eu * vx + wu[IPR] * wu[IV1];
-  const bool obad = nonfinite(wo[IDN]) || nonfinite(wo[IV1]) || nonfinite(wo[IV2]) ||
-                    nonfinite(wo[IV3]) || nonfinite(wo[IPR]) || nonfinite(bo) ||
-                    nonfinite(L ? igm1r : igm1l);
-  double t[NHYDRO];
+  // the upwind side (u) and the other one (v)
+  double wu[NHYDRO], wv[NHYDRO];
 #pragma unroll
   for (int n = 0; n < NHYDRO; ++n) {
-    t[n] = coef * f[n];
-    if (!TAME || obad || (__double_as_longlong(t[n]) << 1) == 0) {  // add the reference's 0 * fo
-      const double vxo = wo[IV1] - bo;
-      double fo;
-      if (n == IDN) fo = wo[IDN] * vxo;
-      else if (n == IV1) fo = wo[IDN] * wo[IV1] * vxo + wo[IPR];
-      else if (n == IV2) fo = wo[IDN] * wo[IV2] * vxo;
-      else if (n == IV3) fo = wo[IDN] * wo[IV3] * vxo;
-      else {
-        const double eo = wo[IPR] * (L ? igm1r : igm1l) +
-                          hlf(wo[IDN]) * (wo[IV1] * wo[IV1] + wo[IV2] * wo[IV2] + wo[IV3] * wo[IV3]);
-        fo = eo * vxo + wo[IPR] * wo[IV1];
-      }
-      const double zo = 0.0 * fo;
-      t[n] = L ? t[n] + zo : zo + t[n];  // the reference's order: ul*fl + ur*fr
+    wu[n] = L ? wli[n] : wri[n];
+    wv[n] = L ? wri[n] : wli[n];
+  }
+  const double bu = L ? bm : bp, bv = L ? bp : bm;
+  auto side = [&](const double *w, double b, double igm1, double *f) {
+    const double vx = w[IV1] - b;
+    f[IDN] = o.mul(w[IDN], vx);
+    f[IV1] = o.mul(o.mul(w[IDN], w[IV1]), vx) + w[IPR];
+    f[IV2] = o.mul(o.mul(w[IDN], w[IV2]), vx);
+    f[IV3] = o.mul(o.mul(w[IDN], w[IV3]), vx);
+    const double e = o.mul(w[IPR], igm1) + o.mul(o.half(w[IDN]), square3(w));
+    f[IEN] = o.mul(e, vx) + o.mul(w[IPR], w[IV1]);
+  };
+  double t[NHYDRO];
+  side(wu, bu, L ? igm1l : igm1r, t);
+#pragma unroll
+  for (int n = 0; n < NHYDRO; ++n) t[n] = o.mul(coef, t[n]);
+  if (OPS::kInt) {
+    const bool back = lt(wv[IV1], bv);  // the sign of the other side's v - b
+    auto add_zero = [](double x, bool negative) {
+      return __double_as_longlong(x) == (long long)0x8000000000000000ULL && !negative ? 0.0 : x;
+    };
+    t[IDN] = add_zero(t[IDN], back);
+    t[IV2] = add_zero(t[IV2], back != (__double2hiint(wv[IV2]) < 0));
+    t[IV3] = add_zero(t[IV3], back != (__double2hiint(wv[IV3]) < 0));
+    if (__double_as_longlong(t[IV1]) == (long long)0x8000000000000000ULL ||
+        __double_as_longlong(t[IEN]) == (long long)0x8000000000000000ULL)
+      o.give_up();
+  } else {
+    double f[NHYDRO];
+    side(wv, bv, L ? igm1r : igm1l, f);
+#pragma unroll
+    for (int n = 0; n < NHYDRO; ++n) {
+      const double z = o.mul(0.0, f[n]);
+      t[n] = L ? t[n] + z : z + t[n];  // the reference's order: ul*fl + ur*fr
     }
   }
+  const double pu = o.mul(ustar, cp);
   flxi[IDN] = t[IDN];
-  flxi[IV1] = t[IV1] + ustar * cp;
+  flxi[IV1] = t[IV1] + pu;
   flxi[IV2] = t[IV2];
   flxi[IV3] = t[IV3];
-  flxi[IEN] = t[IEN] + ustar * cp * sstar;
+  flxi[IEN] = t[IEN] + o.mul(pu, sstar);
 }
 
 #endif
 
 // Fluxes of one face.  The caller checks o.ok() (IntOps), and takes the face again with IeeeOps
 // where it is false.
-template <int RS, bool CONSTG, bool TAME, class OPS>
+template <int RS, bool CONSTG, class OPS>
 __device__ __forceinline__ void riemann(const double *wl, const double *wr, double glc, double gle,
                                         double grc, double gre, const GasConsts &gc, double *flx,
                                         OPS &o) {
 #if APH_EXACT
   if (RS == RS_HLLE) solve_hlle_exact(wl, wr, glc, gle, grc, gre, flx, o);
   else if (RS == RS_HLLC || RS == RS_LHLLC)
-    solve_hllc_exact<RS == RS_LHLLC, TAME>(wl, wr, glc, gle, grc, gre, flx, o);
+    solve_hllc_exact<RS == RS_LHLLC>(wl, wr, glc, gle, grc, gre, flx, o);
 #else
   if (RS == RS_HLLE) solve_hlle<CONSTG>(wl, wr, glc, gle, grc, gre, gc, flx, o);
   else if (RS == RS_HLLC || RS == RS_LHLLC)
@@ -1101,36 +1201,51 @@ __device__ __forceinline__ void riemann(const double *wl, const double *wr, doub
 
 // EstimateTimestep per-cell candidate (hydro.cpp:384-415): min over active directions
 // of dx_d / (|v_d| + lambda).  dt_cell below is the form the stage kernel uses.
-__device__ __forceinline__ double dt_candidate(const double *w, double e_cons, const double *dx,
-                                               int ndim, double gm1) {
+template <class OPS>
+__device__ __forceinline__ double dt_candidate_ops(const double *w, double e_cons, const double *dx,
+                                                   int ndim, double gm1, OPS &o) {
+#pragma unroll
+  for (int n = 0; n < NHYDRO; ++n) o.see(w[n]);
+  o.see(e_cons);
 #if APH_EXACT
-  const double e_internal = div_x(
-      e_cons - 0.5 * w[IDN] * (w[IV1] * w[IV1] + w[IV2] * w[IV2] + w[IV3] * w[IV3]), w[IDN]);
+  const double v2 = o.mul(w[IV1], w[IV1]) + o.mul(w[IV2], w[IV2]) + o.mul(w[IV3], w[IV3]);
+  const double e_k = o.mul(o.half(w[IDN]), v2);
+  const double e_i = e_cons - e_k;
 #else
-  const double e_internal = div_x(
-      fma(-mul(0.5, w[IDN]), square3(w[IV1], w[IV2], w[IV3]), e_cons), w[IDN]);
+  const double e_i = fma(-o.half(w[IDN]), square3(w[IV1], w[IV2], w[IV3]), e_cons);
 #endif
-  const double bulkmod = eos_bulk_modulus(gm1, w[IDN], e_internal);
-  const Den p = den(w[IPR]);
-  const double gamma_c = div_x(bulkmod, p);
-  const double rat = div_x((e_internal + C_LIGHT2) * w[IDN], p);
-  const double root = sqrt_x(div_x(gamma_c, 1 + rat));  // lambda is C times this
+  const double e_internal = o.div0(e_i, o.den(w[IDN]));
+  const double small = 10.0 * 2.2250738585072014e-308;
+  double bulkmod = o.mul(o.mul(__dmul_rn(gm1, __dadd_rn(gm1, 1.0)), w[IDN]), e_internal);  // eos_bulk_modulus
+  bulkmod = lt(small, bulkmod) ? bulkmod : small;
+  const Den p = o.den(w[IPR]);
+  const double gamma_c = o.div(bulkmod, p);
+  const double rat = o.div(o.mul(__dadd_rn(e_internal, C_LIGHT2), w[IDN]), p);
+  const double root = o.sqrt(o.div(gamma_c, o.den(__dadd_rn(1, rat))));  // lambda is C times this
 #if APH_EXACT
-  const double lam = C_LIGHT * root;
+  const double lam = o.mul(C_LIGHT, root);
   auto rate = [&](int d) { return dabs(w[IV1 + d]) + lam; };
 #else
   auto rate = [&](int d) { return fma(C_LIGHT, root, dabs(w[IV1 + d])); };
 #endif
-  double m = div_x(dx[0], rate(0));
+  double m = o.div(dx[0], o.den(rate(0)));
   if (ndim > 1) {
-    const double c2 = div_x(dx[1], rate(1));
+    const double c2 = o.div(dx[1], o.den(rate(1)));
     m = lt(c2, m) ? c2 : m;
   }
   if (ndim > 2) {
-    const double c3 = div_x(dx[2], rate(2));
+    const double c3 = o.div(dx[2], o.den(rate(2)));
     m = lt(c3, m) ? c3 : m;
   }
   return m;
+}
+__device__ __forceinline__ double dt_candidate(const double *w, double e_cons, const double *dx,
+                                               int ndim, double gm1) {
+  IntOps o;
+  const double m = dt_candidate_ops(w, e_cons, dx, ndim, gm1, o);
+  if (o.ok()) return m;
+  IeeeOps ieee;
+  return dt_candidate_ops(w, e_cons, dx, ndim, gm1, ieee);
 }
 
 // dt candidate of a cell just converted by cons_to_prim_cell (floored: its return value).

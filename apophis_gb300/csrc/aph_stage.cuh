@@ -770,6 +770,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
     constexpr int ivz = IV1 + ((ivx - IV1) + 2) % 3;
     const int w2 = n + 2, w1 = n + 1;
     const size_t vs = (size_t)T * w2;
+    const double area = B.area[DIR - 1];
     bool in_range = true;
     for (int it = tid; it < nl * w1; it += nth) {
       const int t = it / w1, f = it - t * w1;
@@ -795,38 +796,41 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
         grc = SR[nv * vs + oR];
         gre = SR[(nv + 1) * vs + oR];
       }
+      // store in cons order (exact: times the face's area, which both of its cells take), and the
+      // boundary faces' fluxes for the coarse-fine correction
+      auto put = [&](auto &o) {
+        const size_t fs = (size_t)T * w1;
+        const size_t of = (size_t)t * w1 + f;
+        const bool keep = a.cf && (f == 0 || f == n);
+        double *kept = keep ? B.bflux + (size_t)(2 * (DIR - 1) + (f == 0 ? 0 : 1)) * a.bflux_stride + (size_t)(l0 + t) * nv
+                            : nullptr;
+        auto one = [&](int v, double x) {
+          if (keep) kept[v] = x;
+          F[v * fs + of] = APH_EXACT ? o.mul(area, x) : x;
+        };
+        one(IDN, flx[IDN]);
+        one(ivx, flx[IV1]);
+        one(ivy, flx[IV2]);
+        one(ivz, flx[IV3]);
+        one(IEN, flx[IEN]);
+        // passive scalars: upwind by the mass flux (hydro.cpp:607-615)
+        for (int v = NHYDRO; v < nv; ++v)
+          one(v, o.mul(flx[IDN], !is_neg(flx[IDN]) ? SL[v * vs + oL] : SR[v * vs + oR]));
+      };
       if (ARITH == ARITH_IEEE) {
         IeeeOps o;
-        if (!APH_EXACT && constg) riemann<RS, true, false>(wl, wr, 0.0, 0.0, 0.0, 0.0, gc, flx, o);
-        else riemann<RS, false, false>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+        if (!APH_EXACT && constg) riemann<RS, true>(wl, wr, 0.0, 0.0, 0.0, 0.0, gc, flx, o);
+        else riemann<RS, false>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+        put(o);
       } else {
         IntOps o;
-        riemann<RS, !APH_EXACT, kTame>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+        riemann<RS, !APH_EXACT>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+        put(o);
         in_range = in_range && o.ok();
       }
-      // store in cons order
-      const size_t fs = (size_t)T * w1;
-      const size_t of = (size_t)t * w1 + f;
-      F[IDN * fs + of] = flx[IDN];
-      F[ivx * fs + of] = flx[IV1];
-      F[ivy * fs + of] = flx[IV2];
-      F[ivz * fs + of] = flx[IV3];
-      F[IEN * fs + of] = flx[IEN];
-      // passive scalars: upwind by the mass flux (hydro.cpp:607-615)
-      for (int v = NHYDRO; v < nv; ++v)
-        F[v * fs + of] = flx[IDN] * (!is_neg(flx[IDN]) ? SL[v * vs + oL] : SR[v * vs + oR]);
     }
     if (ARITH == ARITH_IEEE) __syncthreads();
     else if (!__syncthreads_and(in_range)) return ITEM_IEEE;
-  }
-  if (a.cf) {  // keep the boundary-face fluxes of every line for the coarse-fine correction
-    const int w1 = n + 1;
-    const size_t fs = (size_t)T * w1;
-    for (int it = tid; it < nl * 2 * nv; it += nth) {
-      const int t = it / (2 * nv), r = it % (2 * nv), side = r / nv, v = r % nv;
-      B.bflux[(size_t)(2 * (DIR - 1) + side) * a.bflux_stride + (size_t)(l0 + t) * nv + v] =
-          F[v * fs + (size_t)t * w1 + (side == 0 ? 0 : n)];
-    }
   }
   if (deferred) {  // first pass: store the floored interior values ConsToPrim left in du
     for (int it = tid; it < nl * n; it += nth) {
@@ -845,7 +849,12 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
   {
     const int w1 = n + 1;
     const size_t fs = (size_t)T * w1;
-    const double area = DIR == 1 ? B.dx[1] * B.dx[2] : DIR == 2 ? B.dx[0] * B.dx[2] : B.dx[0] * B.dx[1];
+#if APH_EXACT
+    auto diff = [&](size_t of) { return F[of + 1] - F[of]; };  // F holds area * flux
+#else
+    const double area = B.area[DIR - 1];
+    auto diff = [&](size_t of) { return (area * F[of + 1] - area * F[of]); };
+#endif
     if (!last_pass) {
       for (int it = tid; it < nl * n; it += nth) {  // per cell: its geometry once, then its nv values
         const int t = it / n, c = it - t * n;
@@ -854,15 +863,16 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
         double *du = B.du + ib + c * is;
         for (int v = 0; v < nv; ++v) {
           const size_t of = v * fs + (size_t)t * w1 + c;
-          const double d = (area * F[of + 1] - area * F[of]);
+          const double d = diff(of);
           du[v * B.nint] = first_pass ? d : du[v * B.nint] + d;
         }
       }
     } else {
-      const double vol = B.dx[0] * B.dx[1] * B.dx[2];
-      const double ivol = 1.0 / vol;
+      const double vol = B.vol;
+      const double ivol = B.ivol;
 #if APH_EXACT
-      const bool vol_p2 = pow2_normal(vol);  // power-of-two volume: exact multiplication
+      const bool vol_p2 = pow2_normal(vol);  // power-of-two volume: an exponent step
+      const RkForm rk = rk_form(a.gam0, a.gam1);
 #endif
       const double beta_dt = a.beta * dt_of(a, B);
       const int fmask = a.cf ? amr_finer_mask(B) : 0;
@@ -878,7 +888,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
           // the correction, and amr_fix updates it
           for (int v = 0; v < nv; ++v) {
             const size_t of = v * fs + (size_t)t * w1 + c;
-            const double d = (area * F[of + 1] - area * F[of]);
+            const double d = diff(of);
             double *du = B.du + v * B.nint + icell;
             *du = first_pass ? d : *du + d;
           }
@@ -888,19 +898,20 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
 #pragma unroll
         for (int v = 0; v < NHYDRO; ++v) {
           const size_t of = v * fs + (size_t)t * w1 + c;
-          double du = (area * F[of + 1] - area * F[of]);
+          double du = diff(of);
           if (!first_pass) du = B.du[v * B.nint + icell] + du;
 #if APH_EXACT
           const double div = div_vol(-du, vol, ivol, vol_p2);
+          u[v] = rk_sum(rk, B.u0[v * nc + cell], B.u1[v * nc + cell]) + mul_x(beta_dt, div);
 #else
           const double div = -du * ivol;
-#endif
           u[v] = a.gam0 * B.u0[v * nc + cell] + a.gam1 * B.u1[v * nc + cell] + beta_dt * div;
+#endif
         }
         bool bad = false;
         for (int v = NHYDRO; v < nv; ++v) {  // passive scalars
           const size_t of = v * fs + (size_t)t * w1 + c;
-          double du = (area * F[of + 1] - area * F[of]);
+          double du = diff(of);
           if (!first_pass) du = B.du[v * B.nint + icell] + du;
 #if APH_EXACT
           const double div = div_vol(-du, vol, ivol, vol_p2);
@@ -1009,7 +1020,7 @@ __device__ __forceinline__ double amr_fixed_du(const StageArgs &a, const StepBlo
     const int d = face / 2, s = face % 2, td = 1 - d;
     if ((d == 0 ? i : j) != (s == 0 ? 0 : B.nx[d] - 1)) continue;
     const int t = d == 0 ? j : i;
-    const double area = d == 0 ? B.dx[1] * B.dx[2] : B.dx[0] * B.dx[2];
+    const double area = B.area[d];
     const int tg2 = 2 * (B.amr.origin[td] + t);
     const StepBlock &F = amr_fine_nbr(a.blocks, B, face, td, tg2);
     const int ft = tg2 - F.amr.origin[td];
@@ -1030,8 +1041,8 @@ static __device__ void amr_fix(const StageArgs &a, const Sched &sched, unsigned 
     const GasConsts gc = gas_of(a, B);
     const double beta_dt = a.beta * dt_of(a, B);
     const long long nc = B.ncell;
-    const double vol = B.dx[0] * B.dx[1] * B.dx[2];
-    const double ivol = 1.0 / vol;
+    const double vol = B.vol;
+    const double ivol = B.ivol;
 #if APH_EXACT
     const bool vol_p2 = pow2_normal(vol);  // power-of-two volume: exact multiplication
 #endif
@@ -1088,8 +1099,10 @@ static __device__ void amr_fix(const StageArgs &a, const Sched &sched, unsigned 
   }
 }
 
-// MINB: resident CTAs per SM the registers are budgeted for (1: as many registers as the code
-// wants; 3: capped near 80 per thread for 256-thread CTAs, trading a few spills for occupancy).
+// MINB: resident 256-thread CTAs per SM the registers are budgeted for: 2 (128 per thread, hardly any
+// spills) or 3 (80, trading spills for warps).  KH 128^3 exact, three lines per item: 7.81 ms per RK2
+// step with 2, 7.02 with 3, 7.02 with 4 (64 registers), 7.62 with 5; left to itself the code takes 150
+// to 180 registers, one CTA per SM, and 13.6 ms.
 template <int RECON, int RS, int MINB>
 __global__ void __launch_bounds__(kStageThreads, MINB) k_stage(const __grid_constant__ StageArgs a) {
   extern __shared__ __align__(128) double sm[];
@@ -1272,7 +1285,7 @@ static const void *kernel_for_rs(int rs) {
 
 template <>
 const void *stage_kernel_of<APH_STAGE_RECON>(int rs, int reg_cap) {
-  return reg_cap ? kernel_for_rs<APH_STAGE_RECON, 3>(rs) : kernel_for_rs<APH_STAGE_RECON, 1>(rs);
+  return reg_cap ? kernel_for_rs<APH_STAGE_RECON, 3>(rs) : kernel_for_rs<APH_STAGE_RECON, 2>(rs);
 }
 
 // What the launches share is compiled with the donor-cell kernels.

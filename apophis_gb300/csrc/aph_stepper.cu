@@ -757,6 +757,11 @@ aph_status aph_stepper_create(const aph_stepper_desc *desc, aph_stepper *out) {
       B.dx[d] = a.dx[d];
       p.max_nx[d] = std::max(p.max_nx[d], a.nx[d]);
     }
+    B.area[0] = B.dx[1] * B.dx[2];
+    B.area[1] = B.dx[0] * B.dx[2];
+    B.area[2] = B.dx[0] * B.dx[1];
+    B.vol = B.dx[0] * B.dx[1] * B.dx[2];
+    B.ivol = 1.0 / B.vol;
     if (!a.cons) {
       delete s;
       return fail(APH_ERR_INVALID, "block %d: cons is NULL", b);
