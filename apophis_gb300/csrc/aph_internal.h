@@ -70,6 +70,7 @@ struct StepBlock {
   double dx[3];
   double area[3];     // of a face across each dimension: dx1 dx2, dx0 dx2, dx0 dx1
   double vol, ivol;   // dx0 dx1 dx2 and its reciprocal
+  unsigned inv[3][7]; // ceil(2^32 / (nx[d] + k)): x / (nx[d] + k) is the high word of x inv (widths above 1)
   AmrFaces amr;
 };
 

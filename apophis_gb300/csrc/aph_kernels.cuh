@@ -171,12 +171,13 @@ __global__ void __launch_bounds__(kThreads) k_fluxes(PackDev p, const BlockDev *
     wr[IV3] = sR[ivz * vs + oR]; wr[IPR] = sR[IPR * vs + oR];
     const double glc = sL[nvar * vs + oL], gle = sL[(nvar + 1) * vs + oL];
     const double grc = sR[nvar * vs + oR], gre = sR[(nvar + 1) * vs + oR];
-    IntOps o;
+    SolveOps o;
+#if APH_EXACT
+    bool in_range = true;
 #pragma unroll
-    for (int k = 0; k < NHYDRO; ++k) {
-      o.see(wl[k]);
-      o.see(wr[k]);
-    }
+    for (int k = 0; k < NHYDRO; ++k) in_range &= snug(wl[k]) & snug(wr[k]);
+    if (!in_range) o.give_up();
+#endif
     riemann<RS, false>(wl, wr, glc, gle, grc, gre, gc, flx, o);
     if (!o.ok()) {  // an operand outside the integer pipe's range
       IeeeOps ieee;

@@ -109,9 +109,12 @@ __device__ __forceinline__ bool tame(double x) {
   const unsigned e = hi >> 20;  // biased exponent
   return (e - (1023u - 200u) <= 400u) | ((hi | (unsigned)__double2loint(x)) == 0u);
 }
-__device__ __forceinline__ bool tame_nz(double x) {  // tame and nonzero
-  const unsigned e = ((unsigned)__double2hiint(x) & 0x7fffffffu) >> 20;
-  return e - (1023u - 200u) <= 400u;
+// Zero or 2^-110 <= |x| < 2^111.  From face states in this range the exact Riemann solvers form no
+// product or quotient outside 2^+-1000 as long as their denominators and the few results they
+// check stay within 2^+-400, so their operations need no checks of their own.
+__device__ __forceinline__ bool snug(double x) {
+  const unsigned hi = abs_hi(x);
+  return (hi - ((1023u - 110u) << 20) < (221u << 20)) | ((hi | (unsigned)__double2loint(x)) == 0u);
 }
 // (word by word: from a test of all 64 bits the compiler makes a DSETP, an FP64 instruction)
 __device__ __forceinline__ bool is_zero(double x) {
@@ -280,9 +283,9 @@ __device__ __forceinline__ double quot_bits(unsigned long long ua, unsigned long
   const unsigned long long r2 = (r1 << 23) - (unsigned long long)q2 * B;
   q2 += r2 >= B ? 1u : 0u;
   const unsigned long long m = (((unsigned long long)q1 << 23) + q2 + 1) >> 1;  // 53 bits, rounded
-  const unsigned e = ((unsigned)(ua >> 52) & 0x7ffu) - ((unsigned)(ub >> 52) & 0x7ffu) + 1022u - less;
-  return __longlong_as_double(
-      (long long)((m + ((unsigned long long)(e << 20) << 32)) | ((ua ^ ub) & 0x8000000000000000ULL)));
+  const unsigned ah = (unsigned)(ua >> 32), bh = (unsigned)(ub >> 32);
+  const unsigned e = (ah & 0x7ff00000u) - (bh & 0x7ff00000u) + ((1022u - less) << 20);
+  return __hiloint2double((int)(((unsigned)(m >> 32) + e) | ((ah ^ bh) & 0x80000000u)), (int)(unsigned)m);
 }
 
 // RN(sqrt(x)) for x normal and positive.  With x = X 4^k, 1 <= X < 4, M = X 2^52 and y = 1/sqrt(X):
@@ -314,15 +317,13 @@ __device__ __forceinline__ double sqrt_bits(unsigned long long u) {
   return __longlong_as_double((long long)(m + ((unsigned long long)((e + 1022u - odd) >> 1) << 52)));
 }
 
-// How far x's exponent field lies above 2^-400's; more than kFar above: x is outside
+// How far the high word of |x| lies above that of 2^-400; kFar or more above: x is outside
 // 2^-400 .. 2^401 (zero, infinite and NaN included; signed: also where x is negative).  Quotients,
 // products of two and roots of values inside are normal.
-constexpr unsigned kFar = 800u;
-__device__ __forceinline__ unsigned far_of(double x) {
-  return (((unsigned)__double2hiint(x) & 0x7fffffffu) >> 20) - 623u;
-}
+constexpr unsigned kFar = 801u << 20;
+__device__ __forceinline__ unsigned far_of(double x) { return abs_hi(x) - (623u << 20); }
 __device__ __forceinline__ unsigned far_of_signed(double x) {
-  return ((unsigned)__double2hiint(x) >> 20) - 623u;
+  return (unsigned)__double2hiint(x) - (623u << 20);
 }
 
 // A denominator and its reciprocal word, which several quotients may share.
@@ -331,9 +332,10 @@ struct Den {
   unsigned R;
 };
 
-// The operations of a Riemann solve on the integer pipe, unchecked and free of branches: far
-// collects the largest distance over all operands, and the caller takes the whole solve again
-// with IeeeOps where it exceeds kFar.  div0 allows a numerator of zero.
+// Operations of a Riemann solve on the integer pipe, free of branches: far collects the largest
+// distance over the denominators and what else the caller has it see; where that is out of range
+// the solve is taken again with IeeeOps.  Other operands are not checked (snug states).  div0
+// allows a numerator of zero, mul any zeros.
 struct IntOps {
   static constexpr bool kInt = true;
   unsigned far = 0;
@@ -342,61 +344,84 @@ struct IntOps {
     return Den{b, rcp_word(significand((unsigned long long)__double_as_longlong(b)))};
   }
   __device__ __forceinline__ double div(double a, const Den &d) {
-    far = max(far, far_of(a));
     return quot_bits((unsigned long long)__double_as_longlong(a),
                      (unsigned long long)__double_as_longlong(d.b), d.R);
   }
   __device__ __forceinline__ double div0(double a, const Den &d) {
-    const bool z = is_zero(a);
-    far = max(far, z ? 0u : far_of(a));
-    const unsigned long long ua = (unsigned long long)__double_as_longlong(a);
-    const unsigned long long ub = (unsigned long long)__double_as_longlong(d.b);
-    const double q = quot_bits(ua, ub, d.R);
-    return z ? __longlong_as_double((long long)((ua ^ ub) & 0x8000000000000000ULL)) : q;
+    const double q = div(a, d);
+    const int sg = (__double2hiint(a) ^ __double2hiint(d.b)) & (int)0x80000000;
+    return is_zero(a) ? __hiloint2double(sg, 0) : q;
   }
-  __device__ __forceinline__ double div(double a, double b) { return div(a, den(b)); }
   __device__ __forceinline__ double rcp(double b) { return div(1.0, den(b)); }
   __device__ __forceinline__ double sqrt(double x) {
-    far = max(far, far_of_signed(x));
     return sqrt_bits((unsigned long long)__double_as_longlong(x));
   }
   // RN(a b), a and b zero or normal: the 106-bit product of the significands, rounded by a carry
   // chain.  13 SM-cycles per warp on pipes of its own, where a DMUL holds the FP64 pipe for 17.
   __device__ __forceinline__ double mul(double a, double b) {
-    const unsigned long long ua = (unsigned long long)__double_as_longlong(a);
-    const unsigned long long ub = (unsigned long long)__double_as_longlong(b);
-    const unsigned ea = (unsigned)(ua >> 52) & 0x7ffu, eb = (unsigned)(ub >> 52) & 0x7ffu;
-    unsigned __int128 P = (unsigned __int128)significand(ua) * (significand(ub) << 11);
-    const unsigned low = (unsigned)((unsigned long long)(P >> 64) >> 52) ^ 1u;  // 1: below 2^116
+    const unsigned ah = (unsigned)__double2hiint(a), bh = (unsigned)__double2hiint(b);
+    const unsigned ea = ah & 0x7ff00000u, eb = bh & 0x7ff00000u;
+    unsigned __int128 P = (unsigned __int128)significand((unsigned long long)__double_as_longlong(a)) *
+                          (significand((unsigned long long)__double_as_longlong(b)) << 11);
+    const unsigned low = ((unsigned)((unsigned long long)(P >> 64) >> 32) >> 20) ^ 1u;  // 1: below 2^116
     P <<= low;
     P += 0x7fffffffffffffffULL + ((unsigned)(unsigned long long)(P >> 64) & 1u);  // to even
-    const unsigned e = ea + eb - 1023u - low;  // the leading bit of the significand adds one
-    const unsigned long long sg = (ua ^ ub) & 0x8000000000000000ULL;
+    const unsigned long long m = (unsigned long long)(P >> 64);
+    // (the leading bit of the significand adds one to the exponent)
+    const unsigned e = ea + eb - ((1023u + low) << 20);
+    const unsigned sg = (ah ^ bh) & 0x80000000u;
     const bool z = min(ea, eb) == 0u;
-    far = max(far, z ? 0u : e - 622u);
-    return __longlong_as_double(
-        (long long)(z ? sg : (((unsigned long long)(P >> 64) + ((unsigned long long)(e << 20) << 32)) | sg)));
+    return __hiloint2double((int)(z ? sg : (((unsigned)(m >> 32) + e) | sg)), (int)(z ? 0u : (unsigned)m));
   }
   __device__ __forceinline__ double half(double x) { return half_x(x); }
-  // an input: zero or inside the range
+  __device__ __forceinline__ double twice(double x) { return twice_x(x); }
+  // a value that has to be zero or inside the range
   __device__ __forceinline__ void see(double x) { far = max(far, is_zero(x) ? 0u : far_of(x)); }
   __device__ __forceinline__ void give_up() { far = ~0u; }
-  __device__ __forceinline__ bool ok() const { return far <= kFar; }
+  __device__ __forceinline__ bool ok() const { return far < kFar; }
+};
+// The same with every operand and product checked, for arithmetic on any values.
+struct CheckedOps : IntOps {
+  __device__ __forceinline__ double div(double a, const Den &d) {
+    far = max(far, far_of(a));
+    return IntOps::div(a, d);
+  }
+  __device__ __forceinline__ double div0(double a, const Den &d) {
+    see(a);
+    return IntOps::div0(a, d);
+  }
+  __device__ __forceinline__ double rcp(double b) { return IntOps::div(1.0, den(b)); }
+  __device__ __forceinline__ double sqrt(double x) {
+    far = max(far, far_of_signed(x));
+    return IntOps::sqrt(x);
+  }
+  __device__ __forceinline__ double mul(double a, double b) {
+    const double r = IntOps::mul(a, b);
+    see(r);
+    return r;
+  }
 };
 struct IeeeOps {
   static constexpr bool kInt = false;
   __device__ __forceinline__ Den den(double b) { return Den{b, 0u}; }
   __device__ __forceinline__ double div(double a, const Den &d) { return __ddiv_rn(a, d.b); }
   __device__ __forceinline__ double div0(double a, const Den &d) { return __ddiv_rn(a, d.b); }
-  __device__ __forceinline__ double div(double a, double b) { return __ddiv_rn(a, b); }
   __device__ __forceinline__ double rcp(double b) { return __drcp_rn(b); }
   __device__ __forceinline__ double sqrt(double x) { return __dsqrt_rn(x); }
   __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
   __device__ __forceinline__ double half(double x) { return __dmul_rn(0.5, x); }
+  __device__ __forceinline__ double twice(double x) { return __dadd_rn(x, x); }
   __device__ __forceinline__ void see(double) {}
   __device__ __forceinline__ void give_up() {}
   __device__ __forceinline__ bool ok() const { return true; }
 };
+
+// A face's solve: the exact one takes snug states, the fast one any.
+#if APH_EXACT
+using SolveOps = IntOps;
+#else
+using SolveOps = CheckedOps;
+#endif
 
 // Single operations for any operands: the digits, or the IEEE instruction where an operand is far
 // (a branch: predicating the instruction instead leaves its whole FP64 sequence in the path, which
@@ -405,27 +430,27 @@ __device__ __forceinline__ Den den(double b) {
   return Den{b, rcp_word(significand((unsigned long long)__double_as_longlong(b)))};
 }
 __device__ __forceinline__ double div_x(double a, const Den &d) {
-  IntOps o;
+  CheckedOps o;
   const double q = o.div0(a, d);
-  if (max(o.far, far_of(d.b)) > kFar) return __ddiv_rn(a, d.b);
+  if (max(o.far, far_of(d.b)) >= kFar) return __ddiv_rn(a, d.b);
   return q;
 }
 __device__ __forceinline__ double div_x(double a, double b) { return div_x(a, den(b)); }
 __device__ __forceinline__ double rcp_x(double b) {
-  if (far_of(b) > kFar) return __drcp_rn(b);
+  if (far_of(b) >= kFar) return __drcp_rn(b);
   return quot_bits(0x3ff0000000000000ULL, (unsigned long long)__double_as_longlong(b), den(b).R);
 }
 __device__ __forceinline__ double mul_x(double a, double b) {
-  IntOps o;
+  CheckedOps o;
   o.see(a);
   o.see(b);
-  const double r = o.mul(a, b);
+  const double r = o.IntOps::mul(a, b);
   if (!o.ok()) return __dmul_rn(a, b);
   return r;
 }
 __device__ __forceinline__ double sqrt_x(double x) {
   if (is_zero(x)) return x;
-  if (far_of_signed(x) > kFar) return __dsqrt_rn(x);
+  if (far_of_signed(x) >= kFar) return __dsqrt_rn(x);
   return sqrt_bits((unsigned long long)__double_as_longlong(x));
 }
 
@@ -492,7 +517,7 @@ __device__ __forceinline__ bool cons_to_prim_tail(double *u, double *w, double &
 // The same for any state: on the integer pipe, or again with the IEEE instructions.
 __device__ __forceinline__ bool cons_to_prim_any(double *u, double *w, double &g_c, double &g_e,
                                                  double u_d, double gm1, double pfloor) {
-  IntOps o;
+  CheckedOps o;
   const double e = u[IEN];
   cons_to_prim_tail(u, w, g_c, g_e, u_d, gm1, pfloor, o);
   if (o.ok()) return false;
@@ -667,10 +692,14 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
       mx = a2 > mx ? a2 : mx;
       mx = a3 > mx ? a3 : mx;
       mx = a4 > mx ? a4 : mx;
-      // the roundoff guard |d2qf| > 1e-12 * max|q| (ppm_simple.hpp:132): RN(1e-12 * mx), mx tame,
-      // from the product of the significands; 0 > anything is false, a nonzero value over 0 true
+      // the roundoff guard |d2qf| > 1e-12 * max|q| (ppm_simple.hpp:132); RN(1e-12 * mx) lies in
+      // [2^-40, 2^-38) times mx's binade, so the exponents decide it except within two binades
+      // (0 > anything is false, a nonzero value over 0 true)
       IntOps o;  // (tame operands: all in range)
-      const bool guard = md > mag(o.mul(1.0e-12, from_bits(mx)));
+      const int ed = (int)(md >> 52), em = (int)(mx >> 52);
+      bool guard = ed >= em - 38;
+      if ((ed < em - 38) & (ed > em - 41)) guard = md > mag(o.mul(1.0e-12, from_bits(mx)));
+      guard = guard & (md != 0ULL);
       // rho = qe / d2qf with the guard, else +0.  Where it is a zero (of qe's and d2qf's signs with
       // the guard) the steps are signed zeros; where qe is d2qf it is 1 > 1 - 1e-12: the face
       // values stay
@@ -842,7 +871,7 @@ __device__ __forceinline__ void reconstruct(const double *q, double &ql_ip1, dou
 #if APH_EXACT
 template <class OPS>
 __device__ __forceinline__ double sound_speed(double rho, double p, double gamma, double igm1, OPS &o) {
-  return o.mul(C_LIGHT, o.sqrt(o.div(gamma, 1 + (igm1 + o.div(o.mul(rho, C_LIGHT2), o.den(p))))));
+  return o.mul(C_LIGHT, o.sqrt(o.div(gamma, o.den(1 + (igm1 + o.div(o.mul(rho, C_LIGHT2), o.den(p)))))));
 }
 
 template <class OPS>
@@ -862,9 +891,9 @@ __device__ __forceinline__ void solve_hlle_exact(const double *wli, const double
   const double pmid = o.half(wli[IPR] + wri[IPR] + o.mul(o.mul(wli[IV1] - wri[IV1], rhoa), ca));
   double ql = 1.0, qr = 1.0;
   if (gt(pmid, wli[IPR]))
-    ql = 1.0 + o.mul(o.div(glc + 1, o.den(o.sqrt(2 * glc))), o.div(pmid, o.den(wli[IPR])) - 1.0);
+    ql = 1.0 + o.mul(o.div(glc + 1, o.den(o.sqrt(o.twice(glc)))), o.div(pmid, o.den(wli[IPR])) - 1.0);
   if (gt(pmid, wri[IPR]))
-    qr = 1.0 + o.mul(o.div(grc + 1, o.den(o.sqrt(2 * grc))), o.div(pmid, o.den(wri[IPR])) - 1.0);
+    qr = 1.0 + o.mul(o.div(grc + 1, o.den(o.sqrt(o.twice(grc)))), o.div(pmid, o.den(wri[IPR])) - 1.0);
   const double al = wli[IV1] - o.mul(cl, ql);
   const double ar = wri[IV1] + o.mul(cr, qr);
   const double bp = is_pos(ar) ? ar : 0.0;
@@ -978,7 +1007,7 @@ __device__ __forceinline__ void solve_hllc(const double *wl, const double *wr, d
   const bool bl = gt(pstar, wl[IPR]), br = gt(pstar, wr[IPR]);
   if (bl || br) {
     const double ipp = o.rcp(mul(wl[IPR], wr[IPR]));
-    const double k = CONSTG ? gc.hllc_k : o.div(add(gl, 1), mul(2, gr));
+    const double k = CONSTG ? gc.hllc_k : o.div(add(gl, 1), o.den(mul(2, gr)));
     if (bl) ql = o.sqrt(fma(k, fma(mul(pstar, wr[IPR]), ipp, -1.0), 1.0));
     if (br) qr = o.sqrt(fma(k, fma(mul(pstar, wl[IPR]), ipp, -1.0), 1.0));
   }
@@ -1024,7 +1053,7 @@ __device__ __forceinline__ bool pow2_normal(double x) {
 }
 // x times 2^k, k within +-400: an exponent step for x in range or zero, else the product with c = 2^k
 __device__ __forceinline__ double scale_x(double x, double c, int k) {
-  if (far_of(x) <= kFar)
+  if (far_of(x) < kFar)
     return __longlong_as_double(__double_as_longlong(x) + ((long long)k << 52));
   return is_zero(x) ? x : x * c;
 }
@@ -1075,7 +1104,7 @@ __device__ __forceinline__ double csound_exact(double rho, const Den &p, double 
 //  * the contact branch picks its operands instead of its code, so both branches are the
 //    same two divisions: ul = sstar / (sstar - bm), ustar = -bm / (sstar - bm) when
 //    sstar >= 0, else ur = -sstar / (bp - sstar), ustar = bp / (bp - sstar);
-//  * with IntOps (all operands zero or within 2^-400 .. 2^401) the flux is formed from the upwind
+//  * with IntOps (snug states) the flux is formed from the upwind
 //    side only.  The reference's ul*fl + ur*fr has one weight exactly 0, and RN(a + (+-0)) == a
 //    for every a but -0: there the other side's term 0 * f is +0 or -0 by the sign of f, which
 //    for the mass and transverse fluxes is that of its factors (the normal momentum's and the
@@ -1105,7 +1134,7 @@ __device__ __forceinline__ void solve_hllc_exact(const double *wli, const double
   double cql = cl, cqr = cr;  // the sound speeds times the shock factors
   const bool bl = gt(pstar, wli[IPR]), br = gt(pstar, wri[IPR]);
   if (bl || br) {
-    const double k = o.div(gammal + 1, o.den(2 * gammar));
+    const double k = o.div(gammal + 1, o.den(o.twice(gammar)));
     const double q1 = o.mul(bl ? cl : cr, o.sqrt(1.0 + o.mul(k, o.div(pstar, bl ? pl : pr) - 1.0)));
     if (bl) cql = q1;
     else cqr = q1;
@@ -1168,6 +1197,9 @@ __device__ __forceinline__ void solve_hllc_exact(const double *wli, const double
       t[n] = L ? t[n] + z : z + t[n];  // the reference's order: ul*fl + ur*fr
     }
   }
+  o.see(sstar);
+  o.see(cp);
+  o.see(coef);
   const double pu = o.mul(ustar, cp);
   flxi[IDN] = t[IDN];
   flxi[IV1] = t[IV1] + pu;
@@ -1241,7 +1273,7 @@ __device__ __forceinline__ double dt_candidate_ops(const double *w, double e_con
 }
 __device__ __forceinline__ double dt_candidate(const double *w, double e_cons, const double *dx,
                                                int ndim, double gm1) {
-  IntOps o;
+  CheckedOps o;
   const double m = dt_candidate_ops(w, e_cons, dx, ndim, gm1, o);
   if (o.ok()) return m;
   IeeeOps ieee;

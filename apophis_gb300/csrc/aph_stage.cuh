@@ -130,6 +130,11 @@ __device__ __forceinline__ void tma_load_5d(unsigned dst, const void *tmap, unsi
       : "memory");
 }
 
+// x / w for 0 <= x, x w < 2^32, with inv = ceil(2^32 / w).
+__device__ __forceinline__ int quick_div(int x, int w, unsigned inv) {
+  return w == 1 ? x : (int)__umulhi((unsigned)x, inv);
+}
+
 // Work distribution of a phase with n items.
 struct Sched {
   int mode;
@@ -291,7 +296,7 @@ __device__ __forceinline__ bool ghost_copy_src(const StageArgs &a, const StepBlo
   if (!p.amr) {  // the uniform block grid's map (ghost_cell)
     bool flip = false;
     const int g = map_index(B.loc[d] * n + c, p.mesh_nx[d], p.bc[d][0], p.bc[d][1], flip);
-    const int sl = g / n;
+    const int sl = quick_div(g, n, B.inv[d][0]);
     int loc[3] = {B.loc[0], B.loc[1], B.loc[2]};
     loc[d] = sl;
     S = &a.blocks[(loc[2] * p.nb[1] + loc[1]) * p.nb[0] + loc[0]];
@@ -412,22 +417,23 @@ __device__ __forceinline__ void line_of(const StepBlock &B, int ndim, int ng, in
   const int sj = ndim >= 2 ? ng : 0, sk = ndim >= 3 ? ng : 0;
   const int n0 = B.nx[0], n1 = B.nx[1];
   if (DIR == 1) {
-    const int j = l % n1, k = l / n1;
+    const int k = quick_div(l, n1, B.inv[1][0]), j = l - k * n1;
     base = ((long long)(k + sk) * B.nj + (j + sj)) * B.ni + ng;
     stride = 1;
     ibase = (long long)l * n0;
     istride = 1;
-  } else if (DIR == 2) {
-    const int i = l % n0, k = l / n0;
-    base = ((long long)(k + sk) * B.nj + sj) * B.ni + (i + ng);
+    return;
+  }
+  const int q = quick_div(l, n0, B.inv[0][0]), i = l - q * n0;
+  if (DIR == 2) {
+    base = ((long long)(q + sk) * B.nj + sj) * B.ni + (i + ng);
     stride = B.ni;
-    ibase = (long long)k * n1 * n0 + i;
+    ibase = (long long)q * n1 * n0 + i;
     istride = n0;
   } else {
-    const int i = l % n0, j = l / n0;
-    base = ((long long)sk * B.nj + (j + sj)) * B.ni + (i + ng);
+    base = ((long long)sk * B.nj + (q + sj)) * B.ni + (i + ng);
     stride = (long long)B.ni * B.nj;
-    ibase = (long long)j * n0 + i;
+    ibase = (long long)q * n0 + i;
     istride = (long long)n0 * n1;
   }
 }
@@ -491,61 +497,55 @@ __host__ __device__ constexpr size_t tma_stage_offset(int recon, int n, int T, i
 // the limited value DPH once (faces -1..n+1), then per cell the parabola limiter writes the
 // left state of face c+1 to SL[c+1] and the right state of face c to SR[c+1] (cells -1..n).
 // also(0) and also(1) run beside the face and the cell phase (the adiabatic-index offsets).
+// inv: the block's quick_div factors for the widths n + k.
 template <bool TAME, class ALSO>
 __device__ __forceinline__ void ppm_window(const double *W, double *D2, double *DD, double *DPH,
                                            double *SL, double *SR, int V, int nl, int T, int n,
-                                           int G, ALSO also) {
+                                           const unsigned *inv, ALSO also) {
+  constexpr int G = 3;
   const int NW = n + 2 * G;
   const int tid = threadIdx.x, nth = blockDim.x;
-  // row v * T + t of the slabs and position i in it, for element it of rows of width w (one
-  // division where the item fills its T lines, as plain-load items do)
+  // row v * T + t of the slabs, position i in it and index o = row * w + i, for element it of rows
+  // of width w (o is it where the item fills its T lines, as plain-load items do)
   const bool full = nl == T;
-  auto decode = [&](int it, int w, int &row, int &i) {
-    if (full) {
-      row = it / w;
-      i = it - row * w;
-    } else {
-      const int v = it / (nl * w);
-      const int r = it - v * nl * w;
-      const int t = r / w;
-      i = r - t * w;
-      row = v * T + t;
+  auto decode = [&](int it, int w, unsigned iw, int &row, int &i, int &o) {
+    row = quick_div(it, w, iw);
+    i = it - row * w;
+    o = it;
+    if (!full) {
+      const int v = row / nl;
+      row += v * (T - nl);
+      o = row * w + i;
     }
   };
-  auto w_at = [&](int row, int c) -> double { return W[(size_t)row * NW + c + G]; };
-  const int w4 = n + 4, w3 = n + 3;
+  const int w4 = n + 4, w3 = n + 3, w2 = n + 2;
   for (int it = tid; it < V * nl * w4; it += nth) {  // cells -2..n+1
-    int row, i;
-    decode(it, w4, row, i);
-    const int c = i - 2;
-    const double qm = w_at(row, c - 1), q0 = w_at(row, c), qp = w_at(row, c + 1);
-    D2[(size_t)row * w4 + c + 2] = ppm_d2<TAME>(qm, q0, qp);
-    DD[(size_t)row * w4 + c + 2] = ppm_dd<TAME>(qm, q0, qp);
+    int row, i, o;
+    decode(it, w4, inv[4], row, i, o);
+    const double *q = W + row * NW + i + 1;
+    const double qm = q[-1], q0 = q[0], qp = q[1];
+    D2[o] = ppm_d2<TAME>(qm, q0, qp);
+    DD[o] = ppm_dd<TAME>(qm, q0, qp);
   }
   __syncthreads();
   for (int it = tid; it < V * nl * w3; it += nth) {  // faces -1..n+1
-    int row, i;
-    decode(it, w3, row, i);
-    const int f = i - 1;
-    const size_t o = (size_t)row * w4;
-    DPH[(size_t)row * w3 + f + 1] =
-        ppm_face<TAME>(w_at(row, f - 1), w_at(row, f), DD[o + f + 1], DD[o + f + 2],
-                       D2[o + f + 1], D2[o + f + 2]);
+    int row, i, o;
+    decode(it, w3, inv[3], row, i, o);
+    const double *q = W + row * NW + i + 2;
+    const double *d = DD + row * w4 + i, *e = D2 + row * w4 + i;
+    DPH[o] = ppm_face<TAME>(q[-1], q[0], d[0], d[1], e[0], e[1]);
   }
   also(0);
   __syncthreads();
-  const int w2 = n + 2;
   for (int it = tid; it < V * nl * w2; it += nth) {  // cells -1..n
-    int row, i;
-    decode(it, w2, row, i);
-    const int c = i - 1;
-    const size_t o4 = (size_t)row * w4, o3 = (size_t)row * w3;
+    int row, i, o;
+    decode(it, w2, inv[2], row, i, o);
+    const double *q = W + row * NW + i + 2;
+    const double *e = D2 + row * w4 + i, *f = DPH + row * w3 + i;
     double ql, qr;
-    ppm_cell<TAME>(w_at(row, c - 2), w_at(row, c - 1), w_at(row, c), w_at(row, c + 1),
-                   w_at(row, c + 2), D2[o4 + c + 1], D2[o4 + c + 2], D2[o4 + c + 3],
-                   DPH[o3 + c + 1], DPH[o3 + c + 2], ql, qr);
-    SL[(size_t)row * w2 + c + 1] = ql;
-    SR[(size_t)row * w2 + c + 1] = qr;
+    ppm_cell<TAME>(q[-2], q[-1], q[0], q[1], q[2], e[0], e[1], e[2], f[0], f[1], ql, qr);
+    SL[o] = ql;
+    SR[o] = qr;
   }
   also(1);
 }
@@ -579,7 +579,6 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
   double *SR = DPH + (RECON == RECON_PPM ? (size_t)V * T * (n + 3) : 0);  // right states
   double *SL = (RECON == RECON_PPM) ? DD : SR + (size_t)V * T * (n + 2);  // left states
   double *F = W;                                   // fluxes, after the window is dead
-  auto w_at = [&](int v, int t, int c) -> double & { return W[((size_t)v * T + t) * NW + c + G]; };
 #if APH_EXACT
   // offsets of gamma_c (low half) and gamma_e: window, PPM face values, states
   int *GW = (int *)(sm + pass_smem_doubles(RECON, n, T, nv));
@@ -644,7 +643,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
     // per window cell: its line geometry and source once, then its V values
     for (int it = tid; it < per; it += nth) {
       int t, w;
-      if (DIR == 1) { t = it / NW; w = it - t * NW; } else { w = it / nl; t = it - w * nl; }
+      if (DIR == 1) { t = quick_div(it, NW, B.inv[0][2 * G]); w = it - t * NW; } else { w = it / nl; t = it - w * nl; }
       long long base, stride, ib, is;
       line_of<DIR>(B, a.p.ndim, a.p.ng, l0 + t, base, stride, ib, is);
       const int c = w - G;
@@ -653,17 +652,34 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
       int flipv = -1;
       if (src_ghosts && (c < 0 || c >= n)) ghost_copy_src<DIR>(a, B, l0 + t, c, base, stride, S, cell, flipv);
       const long long snc = S->ncell;
-      for (int v = 0; v < nv; ++v) {
-        const double x = flip_if(S->prim[v * snc + cell], v == flipv);
-        W[((size_t)v * T + t) * NW + w] = x;
-        if (kTame) tame_ok = tame_ok && tame(x);
+      // every load before the first store (a store to shared memory might alias them for all the
+      // compiler knows, and would make them wait for one another)
+      const double *P = S->prim + cell;
+      double x[NHYDRO];
+#pragma unroll
+      for (int v = 0; v < NHYDRO; ++v) x[v] = P[v * snc];
+#if APH_EXACT
+      long long kc = 0, ke = 0;
+      if (kOffsets) {
+        kc = __double_as_longlong(S->gamma[cell]) - gbase;
+        ke = __double_as_longlong(S->gamma[snc + cell]) - gbase;
+      }
+#endif
+#pragma unroll
+      for (int v = 0; v < NHYDRO; ++v) {
+        const double y = flip_if(x[v], v == flipv);
+        W[(v * T + t) * NW + w] = y;
+        if (kTame) tame_ok = tame_ok & snug(y);
+      }
+      for (int v = NHYDRO; v < nv; ++v) {
+        const double y = P[v * snc];
+        W[(v * T + t) * NW + w] = y;
+        if (kTame) tame_ok = tame_ok & tame(y);
       }
 #if APH_EXACT
       if (kOffsets) {
-        const long long kc = __double_as_longlong(S->gamma[cell]) - gbase;
-        const long long ke = __double_as_longlong(S->gamma[snc + cell]) - gbase;
-        offset_ok = offset_ok && (unsigned long long)(kc + kGamMax) <= 2u * kGamMax &&
-                    (unsigned long long)(ke + kGamMax) <= 2u * kGamMax;
+        offset_ok = offset_ok & ((unsigned long long)(kc + kGamMax) <= 2u * kGamMax) &
+                    ((unsigned long long)(ke + kGamMax) <= 2u * kGamMax);
         GW[t * NW + w] = pack2((int)kc, (int)ke);
       }
 #endif
@@ -672,7 +688,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
 #if APH_EXACT
         g_c = S->gamma[cell];
         g_e = S->gamma[snc + cell];
-        if (kTame) tame_ok = tame_ok && tame(g_c) && tame(g_e);
+        if (kTame) tame_ok = tame_ok & snug(g_c) & snug(g_e);
 #else
         // the fast ConsToPrim leaves the constants where no floor fired; the reference's
         // values (which the limiters see) are recomputed from the cell's state there (a
@@ -688,8 +704,8 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
           gamma_ref(uc, gc.gm1, g_c, g_e);
         }
 #endif
-        W[((size_t)nv * T + t) * NW + w] = g_c;
-        W[((size_t)(nv + 1) * T + t) * NW + w] = g_e;
+        W[(nv * T + t) * NW + w] = g_c;
+        W[((nv + 1) * T + t) * NW + w] = g_e;
       }
     }
   }
@@ -708,19 +724,19 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
 #endif
   // B-D: reconstruction; left state of face c+1 -> SL[c+1], right state of face c -> SR[c+1]
   if (RECON == RECON_PPM) {
-    ppm_window<kTame>(W, D2, DD, DPH, SL, SR, V, nl, T, n, G, [&](int phase) {
+    ppm_window<kTame>(W, D2, DD, DPH, SL, SR, V, nl, T, n, B.inv[DIR - 1], [&](int phase) {
 #if APH_EXACT
       if (!kOffsets) return;
       if (phase == 0) {
         for (int it = tid; it < nl * (n + 3); it += nth) {  // faces -1..n+1
-          const int t = it / (n + 3), f = it - t * (n + 3) - 1;
+          const int t = quick_div(it, n + 3, B.inv[DIR - 1][3]), f = it - t * (n + 3) - 1;
           const int *g = GW + t * NW + f + G;
           GD[it] = pack2(gam_face(low(g[-2]), low(g[-1]), low(g[0]), low(g[1]), godd),
                          gam_face(high(g[-2]), high(g[-1]), high(g[0]), high(g[1]), godd));
         }
       } else {
         for (int it = tid; it < nl * (n + 2); it += nth) {  // cells -1..n
-          const int t = it / (n + 2), c = it - t * (n + 2) - 1;
+          const int t = quick_div(it, n + 2, B.inv[DIR - 1][2]), c = it - t * (n + 2) - 1;
           const int *g = GW + t * NW + c + G, *f = GD + t * (n + 3) + c + 1;
           int lc, rc, le, re;
           gam_cell(low(g[-1]), low(g[0]), low(g[1]), low(f[0]), low(f[1]), lc, rc);
@@ -734,22 +750,24 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
   } else {
     const int w2 = n + 2;
     for (int it = tid; it < V * nl * w2; it += nth) {
-      const int v = it / (nl * w2);
-      const int r = it - v * nl * w2;
-      const int t = r / w2, c = r - t * w2 - 1;
-      double ql, qr;
-      if (RECON == RECON_PLM) {
-        plm(w_at(v, t, c - 1), w_at(v, t, c), w_at(v, t, c + 1), ql, qr);
-      } else {
-        ql = qr = w_at(v, t, c);
+      int row = quick_div(it, w2, B.inv[DIR - 1][2]);
+      const int i = it - row * w2;  // cell i - 1
+      int o = it;
+      if (nl != T) {
+        row += row / nl * (T - nl);
+        o = row * w2 + i;
       }
-      SL[((size_t)v * T + t) * w2 + c + 1] = ql;
-      SR[((size_t)v * T + t) * w2 + c + 1] = qr;
+      const double *q = W + row * NW + i + G - 1;
+      double ql, qr;
+      if (RECON == RECON_PLM) plm(q[-1], q[0], q[1], ql, qr);
+      else ql = qr = q[0];
+      SL[o] = ql;
+      SR[o] = qr;
     }
 #if APH_EXACT
     if (kOffsets) {
       for (int it = tid; it < nl * w2; it += nth) {
-        const int t = it / w2, c = it - t * w2 - 1;
+        const int t = quick_div(it, w2, B.inv[DIR - 1][2]), c = it - t * w2 - 1;
         const int *g = GW + t * NW + c + G;
         int lc = low(g[0]), le = high(g[0]), rc = lc, re = le;
         if (RECON == RECON_PLM) {
@@ -769,12 +787,12 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
     constexpr int ivy = IV1 + ((ivx - IV1) + 1) % 3;
     constexpr int ivz = IV1 + ((ivx - IV1) + 2) % 3;
     const int w2 = n + 2, w1 = n + 1;
-    const size_t vs = (size_t)T * w2;
+    const int vs = T * w2;
     const double area = B.area[DIR - 1];
     bool in_range = true;
     for (int it = tid; it < nl * w1; it += nth) {
-      const int t = it / w1, f = it - t * w1;
-      const size_t oL = (size_t)t * w2 + f, oR = oL + 1;
+      const int t = quick_div(it, w1, B.inv[DIR - 1][1]), f = it - t * w1;
+      const int oL = t * w2 + f, oR = oL + 1;
       double wl[NHYDRO], wr[NHYDRO], flx[NHYDRO];
       wl[IDN] = SL[IDN * vs + oL]; wl[IV1] = SL[ivx * vs + oL]; wl[IV2] = SL[ivy * vs + oL];
       wl[IV3] = SL[ivz * vs + oL]; wl[IPR] = SL[IPR * vs + oL];
@@ -798,15 +816,23 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
       }
       // store in cons order (exact: times the face's area, which both of its cells take), and the
       // boundary faces' fluxes for the coarse-fine correction
+      auto times = [](auto &o, double x, double y) {
+#if APH_EXACT
+        const double r = o.mul(x, y);
+        o.see(r);
+        return r;
+#else
+        return x * y;
+#endif
+      };
       auto put = [&](auto &o) {
-        const size_t fs = (size_t)T * w1;
-        const size_t of = (size_t)t * w1 + f;
+        const int fs = T * w1, of = t * w1 + f;
         const bool keep = a.cf && (f == 0 || f == n);
         double *kept = keep ? B.bflux + (size_t)(2 * (DIR - 1) + (f == 0 ? 0 : 1)) * a.bflux_stride + (size_t)(l0 + t) * nv
                             : nullptr;
         auto one = [&](int v, double x) {
           if (keep) kept[v] = x;
-          F[v * fs + of] = APH_EXACT ? o.mul(area, x) : x;
+          F[v * fs + of] = APH_EXACT ? times(o, area, x) : x;
         };
         one(IDN, flx[IDN]);
         one(ivx, flx[IV1]);
@@ -815,7 +841,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
         one(IEN, flx[IEN]);
         // passive scalars: upwind by the mass flux (hydro.cpp:607-615)
         for (int v = NHYDRO; v < nv; ++v)
-          one(v, o.mul(flx[IDN], !is_neg(flx[IDN]) ? SL[v * vs + oL] : SR[v * vs + oR]));
+          one(v, times(o, flx[IDN], !is_neg(flx[IDN]) ? SL[v * vs + oL] : SR[v * vs + oR]));
       };
       if (ARITH == ARITH_IEEE) {
         IeeeOps o;
@@ -823,7 +849,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
         else riemann<RS, false>(wl, wr, glc, gle, grc, gre, gc, flx, o);
         put(o);
       } else {
-        IntOps o;
+        SolveOps o;
         riemann<RS, !APH_EXACT>(wl, wr, glc, gle, grc, gre, gc, flx, o);
         put(o);
         in_range = in_range && o.ok();
@@ -834,7 +860,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
   }
   if (deferred) {  // first pass: store the floored interior values ConsToPrim left in du
     for (int it = tid; it < nl * n; it += nth) {
-      const int t = it / n, c = it - t * n;
+      const int t = quick_div(it, n, B.inv[DIR - 1][0]), c = it - t * n;
       long long base, stride, ib, is;
       line_of<DIR>(B, a.p.ndim, a.p.ng, l0 + t, base, stride, ib, is);
       const long long icell = ib + c * is;
@@ -848,37 +874,52 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
   // F: flux difference of each interior cell; du accumulates x, y, z in order
   {
     const int w1 = n + 1;
-    const size_t fs = (size_t)T * w1;
+    const int fs = T * w1;
 #if APH_EXACT
-    auto diff = [&](size_t of) { return F[of + 1] - F[of]; };  // F holds area * flux
+    auto diff = [&](int of) { return F[of + 1] - F[of]; };  // F holds area * flux
 #else
     const double area = B.area[DIR - 1];
-    auto diff = [&](size_t of) { return (area * F[of + 1] - area * F[of]); };
+    auto diff = [&](int of) { return (area * F[of + 1] - area * F[of]); };
 #endif
     if (!last_pass) {
       for (int it = tid; it < nl * n; it += nth) {  // per cell: its geometry once, then its nv values
-        const int t = it / n, c = it - t * n;
+        const int t = quick_div(it, n, B.inv[DIR - 1][0]), c = it - t * n;
         long long base, stride, ib, is;
         line_of<DIR>(B, a.p.ndim, a.p.ng, l0 + t, base, stride, ib, is);
         double *du = B.du + ib + c * is;
-        for (int v = 0; v < nv; ++v) {
-          const size_t of = v * fs + (size_t)t * w1 + c;
-          const double d = diff(of);
-          du[v * B.nint] = first_pass ? d : du[v * B.nint] + d;
+        const long long ni = B.nint;
+        double x[NHYDRO];
+        if (!first_pass) {  // all loads before the first store
+#pragma unroll
+          for (int v = 0; v < NHYDRO; ++v) x[v] = du[v * ni];
+        }
+#pragma unroll
+        for (int v = 0; v < NHYDRO; ++v) {
+          const double d = diff(v * fs + t * w1 + c);
+          du[v * ni] = first_pass ? d : x[v] + d;
+        }
+        for (int v = NHYDRO; v < nv; ++v) {
+          const double d = diff(v * fs + t * w1 + c);
+          du[v * ni] = first_pass ? d : du[v * ni] + d;
         }
       }
     } else {
       const double vol = B.vol;
       const double ivol = B.ivol;
 #if APH_EXACT
-      const bool vol_p2 = pow2_normal(vol);  // power-of-two volume: an exponent step
       const RkForm rk = rk_form(a.gam0, a.gam1);
 #endif
       const double beta_dt = a.beta * dt_of(a, B);
+#if APH_EXACT
+      // a power-of-two volume scales beta_dt instead of the flux difference, exactly: it takes
+      // neither beta_dt nor du (checked below) near an underflow
+      const double bdt_ivol = beta_dt * ivol;
+      const bool vol_p2 = pow2_normal(vol) && far_of(vol) < kFar && far_of(beta_dt) < kFar;
+#endif
       const int fmask = a.cf ? amr_finer_mask(B) : 0;
       unsigned long long mymin = ~0ULL;
       for (int it = tid; it < nl * n; it += nth) {
-        const int t = it / n, c = it - t * n;
+        const int t = quick_div(it, n, B.inv[DIR - 1][0]), c = it - t * n;
         long long base, stride, ib, is;
         line_of<DIR>(B, a.p.ndim, a.p.ng, l0 + t, base, stride, ib, is);
         const long long cell = base + c * stride;
@@ -887,7 +928,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
           // a coarse cell at a face with a finer neighbour: its flux difference waits for
           // the correction, and amr_fix updates it
           for (int v = 0; v < nv; ++v) {
-            const size_t of = v * fs + (size_t)t * w1 + c;
+            const int of = v * fs + t * w1 + c;
             const double d = diff(of);
             double *du = B.du + v * B.nint + icell;
             *du = first_pass ? d : *du + d;
@@ -897,12 +938,13 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
         double u[NHYDRO];
 #pragma unroll
         for (int v = 0; v < NHYDRO; ++v) {
-          const size_t of = v * fs + (size_t)t * w1 + c;
+          const int of = v * fs + t * w1 + c;
           double du = diff(of);
           if (!first_pass) du = B.du[v * B.nint + icell] + du;
 #if APH_EXACT
-          const double div = div_vol(-du, vol, ivol, vol_p2);
-          u[v] = rk_sum(rk, B.u0[v * nc + cell], B.u1[v * nc + cell]) + mul_x(beta_dt, div);
+          double rate = vol_p2 ? bdt_ivol * -du : 0.0;
+          if (!vol_p2 || (far_of(du) >= kFar && !is_zero(du))) rate = beta_dt * div_vol(-du, vol, ivol, pow2_normal(vol));
+          u[v] = rk_sum(rk, B.u0[v * nc + cell], B.u1[v * nc + cell]) + rate;
 #else
           const double div = -du * ivol;
           u[v] = a.gam0 * B.u0[v * nc + cell] + a.gam1 * B.u1[v * nc + cell] + beta_dt * div;
@@ -910,11 +952,11 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
         }
         bool bad = false;
         for (int v = NHYDRO; v < nv; ++v) {  // passive scalars
-          const size_t of = v * fs + (size_t)t * w1 + c;
+          const int of = v * fs + t * w1 + c;
           double du = diff(of);
           if (!first_pass) du = B.du[v * B.nint + icell] + du;
 #if APH_EXACT
-          const double div = div_vol(-du, vol, ivol, vol_p2);
+          const double div = div_vol(-du, vol, ivol, pow2_normal(vol));
 #else
           const double div = -du * ivol;
 #endif

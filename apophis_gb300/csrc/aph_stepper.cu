@@ -762,6 +762,8 @@ aph_status aph_stepper_create(const aph_stepper_desc *desc, aph_stepper *out) {
     B.area[2] = B.dx[0] * B.dx[1];
     B.vol = B.dx[0] * B.dx[1] * B.dx[2];
     B.ivol = 1.0 / B.vol;
+    for (int d = 0; d < 3; ++d)
+      for (int k = 0; k < 7; ++k) B.inv[d][k] = 0xffffffffu / (unsigned)(B.nx[d] + k) + 1u;
     if (!a.cons) {
       delete s;
       return fail(APH_ERR_INVALID, "block %d: cons is NULL", b);
