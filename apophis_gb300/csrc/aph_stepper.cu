@@ -194,13 +194,45 @@ aph_status upload_items(aph_stepper s, int2 **dst, const std::vector<int2> &v) {
   return e == cudaSuccess ? APH_OK : cuda_fail(e, "stepper items");
 }
 
-int auto_lines(int n) { return (n + 2 >= 256) ? 1 : std::max(1, 256 / (n + 2)); }
+// Lines of n cells per item: the faces of one round of 256 threads, and two lines where one would
+// leave most of a second line's room empty (2D blocks of 128, exact PPM: 1.46 ms per RK2 step of a
+// 768^2 mesh with two lines, 1.87 with one; at 16 to 96 cells the count for one round is within 2 %
+// of the best).
+int auto_lines(int n) { return n + 2 >= 224 ? 1 : n + 2 >= 128 ? 2 : 256 / (n + 2); }
 
 void destroy_graph(aph_stepper s) {
   if (s->exec) cudaGraphExecDestroy(s->exec);
   if (s->graph) cudaGraphDestroy(s->graph);
   s->exec = nullptr;
   s->graph = nullptr;
+}
+
+// The launch configuration of a new stepper.  A pack whose passes hold several items per SM takes the
+// build for three CTAs per SM in exact mode (KH 192^3: 21.5 against 22.9 ms per RK2 step, refined RT 1.45
+// against 1.69; fast mode is the other way round, KH 512^2 PLM 0.57 against 0.53) and, where a CTA
+// gets more than a few, the dynamic schedule (KH 192^3: 21.2 against 22.4 ms strided).  A smaller pack
+// never fills an SM twice: registers as needed, no work counter.
+void default_launch(aph_stepper s) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  aph_stepper_config &c = s->cfg;
+  c.threads = 256;
+  c.ctas_per_sm = 0;
+  long long most = 0;  // items of the longest pass
+  for (int d = 0; d < 3; ++d) {
+    c.lines[d] = 0;
+    c.order[d] = d + 1;
+    if (d >= s->dev.ndim) continue;
+    const int T = auto_lines(s->dev.max_nx[d]);
+    long long items = 0;
+    for (const StepBlock &B : s->hblocks) items += (B.nint / B.nx[d] + T - 1) / T;
+    most = std::max(most, items);
+  }
+  c.use_graph = 1;
+  c.tma = 0;
+  c.reg_cap = s->params.exact && most > 2LL * sms ? 1 : 0;
+  c.schedule = most > 6LL * sms ? 2 : 0;
 }
 
 // TMA staging of pass windows (cfg.tma): every block of the same size, laid out back to back
@@ -792,16 +824,7 @@ aph_status aph_stepper_create(const aph_stepper_desc *desc, aph_stepper *out) {
   s->total_interior = inter;
   s->gravity = desc->use_gravity != 0;
   for (int d = 0; d < 3; ++d) s->grav[d] = desc->gravity[d];
-  s->cfg.threads = 256;
-  s->cfg.ctas_per_sm = 0;
-  for (int d = 0; d < 3; ++d) {
-    s->cfg.lines[d] = 0;
-    s->cfg.order[d] = d + 1;
-  }
-  s->cfg.schedule = 0;
-  s->cfg.use_graph = 1;
-  s->cfg.reg_cap = 0;
-  s->cfg.tma = 0;
+  default_launch(s);
   cudaError_t e = cudaSuccess;
   auto ck = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
   ck(cudaMalloc(&s->d_u1, sizeof(double) * nvar * cells));

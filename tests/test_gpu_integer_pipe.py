@@ -78,3 +78,20 @@ def test_exact_stepper_outside_the_main_path(recon, rsolver, gamma, scale):
     _same(np.ascontiguousarray(st.state()[:, :, sk, sj, si]), np.ascontiguousarray(ref.get()[:, :, sk, sj, si]))
     assert st.status()["dt"] == ref.state()["dt"]
     st.close()
+
+
+@pytest.mark.parametrize("n", [125, 126, 127, 221, 222, 250])
+@pytest.mark.parametrize("recon", ["ppm", "plm"])
+def test_default_lines_around_the_rule(n, recon):
+    """The default lines per item at the widths where their count changes: one step of a single
+    block (fewer items than SMs) equals the oracle."""
+    from oracle import oracle as O
+    cfg, cons = problems.kh2d(n=n, block=n, ng=3, recon=recon, rsolver="hllc")
+    ref = O.Mesh(cfg)
+    ref.set_cons(cons)
+    ref.run(nsteps=1)
+    st = Stepper(cfg, cons, exact=True)
+    st.step(1)
+    sk, sj, si = cfg.interior
+    _same(np.ascontiguousarray(st.state()[:, :, sk, sj, si]), np.ascontiguousarray(ref.get()[:, :, sk, sj, si]))
+    st.close()
