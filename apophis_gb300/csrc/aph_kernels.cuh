@@ -7,6 +7,7 @@
 #include "aph_amr.cuh"
 #include "aph_internal.h"
 #include "aph_math.cuh"
+#include "aph_window.cuh"
 
 #ifndef APH_NS
 #error "APH_NS must name the namespace of this translation unit"
@@ -57,141 +58,184 @@ __global__ void __launch_bounds__(kThreads) k_cons_to_prim(PackDev p, const Bloc
 // ---------------------------------------------------------------------------------------
 // CalculateFluxes for one direction (hydro.cpp:580-740): reconstruction of every
 // primitive and both adiabatic indices on the cells s-1..e+1 of each line, then the
-// Riemann solve on the faces s..e+1.  A CTA takes T whole lines; the face states go
-// through shared memory and never reach HBM.  Only lines through the interior are
-// computed (the reference also fills the unused fluxes on ghost rows).
+// Riemann solve on the faces s..e+1.  A CTA takes a segment of M cells of T lines as a window in
+// shared memory (aph_window.cuh), so each face value is formed once and no state reaches HBM;
+// long lines are cut so that any length fits and a pack of few lines still spreads over the SMs.
+// Only lines through the interior are computed (the reference also fills the unused fluxes on
+// ghost rows).  The FP64 pipe and integer issue bound it, as the stage kernel.
 // ---------------------------------------------------------------------------------------
-template <int RECON>
-__device__ __forceinline__ void recon_strided(const double *q, long long s, double &ql, double &qr) {
-  if (RECON == RECON_DC) {
-    ql = qr = q[0];
-  } else if (RECON == RECON_PLM) {
-    plm(q[-s], q[0], q[s], ql, qr);
-  } else {
-    ppm(q[-2 * s], q[-s], q[0], q[s], q[2 * s], ql, qr);
-  }
-}
-
 template <int DIR>
 __device__ __forceinline__ void line_geometry(const BlockDev &B, int ndim, int ng, int line,
-                                              int &i0, int &j0, int &k0, long long &s,
-                                              int &n) {
+                                              int &i0, int &j0, int &k0) {
   const int si = ng, sj = dim_start(1, ndim, ng), sk = dim_start(2, ndim, ng);
+  const int w = DIR == 1 ? B.nx[1] : B.nx[0], q = line / w, r = line - q * w;
   if (DIR == 1) {
-    n = B.nx[0];
-    s = 1;
-    j0 = sj + line % B.nx[1];
-    k0 = sk + line / B.nx[1];
+    j0 = sj + r;
+    k0 = sk + q;
     i0 = si;
   } else if (DIR == 2) {
-    n = B.nx[1];
-    s = B.ni;
-    i0 = si + line % B.nx[0];
-    k0 = sk + line / B.nx[0];
+    i0 = si + r;
+    k0 = sk + q;
     j0 = sj;
   } else {
-    n = B.nx[2];
-    s = (long long)B.ni * B.nj;
-    i0 = si + line % B.nx[0];
-    j0 = sj + line / B.nx[0];
+    i0 = si + r;
+    j0 = sj + q;
     k0 = sk;
   }
 }
 
-template <int DIR, int RECON, int RS>
-__global__ void __launch_bounds__(kThreads) k_fluxes(PackDev p, const BlockDev *blocks, int T) {
-  extern __shared__ double sm[];
-  const BlockDev &B = blocks[p.block0 + blockIdx.y];
-  const int ntrans = (DIR == 1) ? B.nx[1] * B.nx[2] : (DIR == 2) ? B.nx[0] * B.nx[2] : B.nx[0] * B.nx[1];
-  const int line0 = blockIdx.x * T;
-  if (line0 >= ntrans) return;
-  const int nl = min(T, ntrans - line0);
-  const int n = B.nx[DIR - 1];
-  const int P = n + 2;  // slots: cell c in [-1, n] stores at slot c+1
-  const int V = p.nvar + 2;
-  const int maxP = p.max_nx[DIR - 1] + 2;
-  double *sL = sm;                      // [V][T][maxP]: left state of face slot
-  double *sR = sm + (size_t)V * T * maxP;  // [V][T][maxP]: right state of face slot-1
-  const long long nc = B.ncell;
-  const int nvar = p.nvar;
+// Where a CTA's lines lie: cells c0..c0+n-1 of lines l0..l0+nl-1.
+struct Segment {
+  int l0, nl, c0, n;
+  bool last;  // up to the lines' ends: the high face of the last cell is the segment's too
+};
 
-  // phase 1: reconstruction, one item per (line, cell)
-  const int n1 = nl * P;
-  for (int it = threadIdx.x; it < n1; it += blockDim.x) {
-    int t, slot;
-    if (DIR == 1) { t = it / P; slot = it - t * P; }
-    else { slot = it / nl; t = it - slot * nl; }
-    int i0, j0, k0, ln;
-    long long s;
-    line_geometry<DIR>(B, p.ndim, p.ng, line0 + t, i0, j0, k0, s, ln);
-    const long long cell = ((long long)k0 * B.nj + j0) * B.ni + i0 + (long long)(slot - 1) * s;
-    const size_t o = ((size_t)t) * maxP + slot;
-    for (int v = 0; v < nvar; ++v) {
-      double ql, qr;
-      recon_strided<RECON>(B.prim + v * nc + cell, s, ql, qr);
-      sL[(size_t)v * T * maxP + o] = ql;  // left state of face c+1 (slot c+1)
-      sR[(size_t)v * T * maxP + o] = qr;  // right state of face c   (slot c+1)
+// How a segment is solved: exact build, gamma offsets (kFluxMain), then double slabs on tame windows
+// (kFluxSlabs); fast build, kFluxSlabs; last, any window with the IEEE instructions.  Returns false
+// where the window or an operand is out of range (nothing but fluxes to be rewritten was stored).
+constexpr int kFluxMain = 0, kFluxSlabs = 1, kFluxIeee = 2;
+
+template <int DIR, int RECON, int RS, int HOW>
+__device__ __forceinline__ bool flux_segment(const PackDev &p, const BlockDev &B, const Segment &g, int T,
+                                             const unsigned *inv, double *sm) {
+  constexpr int G = Halo<RECON>::G;
+  constexpr bool kTame = APH_EXACT && HOW != kFluxIeee, kOffsets = HOW == kFluxMain;
+  const int nvar = p.nvar, V = kOffsets ? nvar : nvar + 2, n = g.n, nl = g.nl, NW = n + 2 * G;
+  const int tid = threadIdx.x, nth = blockDim.x;
+  const long long nc = B.ncell;
+  const long long stride = DIR == 1 ? 1 : DIR == 2 ? B.ni : (long long)B.ni * B.nj;
+  const Window w = window_regions<RECON>(sm, n, T, V, nvar);
+  bool tame_ok = true;
+#if APH_EXACT
+  const long long gbase = __double_as_longlong(p.gamma);
+  const int odd = (int)gbase & 1;
+#else
+  const int odd = 0;
+#endif
+  for (int it = tid; it < nl * NW; it += nth) {
+    int t, x0;
+    if (DIR == 1) { t = it / NW; x0 = it - t * NW; }
+    else { x0 = it / nl; t = it - x0 * nl; }
+    int i0, j0, k0;
+    line_geometry<DIR>(B, p.ndim, p.ng, g.l0 + t, i0, j0, k0);
+    const long long cell = ((long long)k0 * B.nj + j0) * B.ni + i0 + (long long)(g.c0 + x0 - G) * stride;
+    double x[NHYDRO];  // (loads before stores: they would wait for one another)
+#pragma unroll
+    for (int v = 0; v < NHYDRO; ++v) x[v] = B.prim[v * nc + cell];
+    const double gc = B.gamma[cell], ge = B.gamma[nc + cell];
+#pragma unroll
+    for (int v = 0; v < NHYDRO; ++v) {
+      w.W[(v * T + t) * NW + x0] = x[v];
+      if (kTame) tame_ok = tame_ok & snug(x[v]);
     }
-    for (int v = 0; v < 2; ++v) {
-      double ql, qr;
-      recon_strided<RECON>(B.gamma + v * nc + cell, s, ql, qr);
-      sL[(size_t)(nvar + v) * T * maxP + o] = ql;
-      sR[(size_t)(nvar + v) * T * maxP + o] = qr;
+    for (int v = NHYDRO; v < nvar; ++v) {
+      const double y = B.prim[v * nc + cell];
+      w.W[(v * T + t) * NW + x0] = y;
+      if (kTame) tame_ok = tame_ok & tame(y);
+    }
+#if APH_EXACT
+    if (kOffsets) {
+      const long long kc = __double_as_longlong(gc) - gbase, ke = __double_as_longlong(ge) - gbase;
+      tame_ok = tame_ok & gam_near(kc) & gam_near(ke);
+      w.GW[t * NW + x0] = gam_pack((int)kc, (int)ke);
+    }
+#endif
+    if (!kOffsets) {
+      w.W[(nvar * T + t) * NW + x0] = gc;
+      w.W[((nvar + 1) * T + t) * NW + x0] = ge;
+      if (kTame) tame_ok = tame_ok & snug(gc) & snug(ge);
     }
   }
+#if APH_EXACT
+  if (kOffsets) tame_ok = tame_ok && gamma_inside(p.gamma);
+#endif
+  if (kTame) {
+    if (!__syncthreads_and(tame_ok)) return false;
+  } else {
+    __syncthreads();
+  }
+  window_states<RECON, kTame, kOffsets>(w, V, nl, T, n, inv, odd);
   __syncthreads();
 
-  // phase 2: Riemann solve, one item per (line, face); face f in [0, n]
+  // Riemann solve, one item per (line, face); face f in [0, n]
   constexpr int ivx = DIR;
   constexpr int ivy = IV1 + ((ivx - IV1) + 1) % 3;
   constexpr int ivz = IV1 + ((ivx - IV1) + 2) % 3;
-  const GasConsts gc{};
+  const GasConsts none{};
   double *flux = B.flux[DIR - 1];
-  const int nf = n + 1;
-  const int n2 = nl * nf;
-  for (int it = threadIdx.x; it < n2; it += blockDim.x) {
+  const int nf = g.last ? n + 1 : n, w2 = n + 2, vs = T * w2;
+  bool in_range = true;
+  for (int it = tid; it < nl * nf; it += nth) {
     int t, f;
     if (DIR == 1) { t = it / nf; f = it - t * nf; }
     else { f = it / nl; t = it - f * nl; }
-    int i0, j0, k0, ln;
-    long long s;
-    line_geometry<DIR>(B, p.ndim, p.ng, line0 + t, i0, j0, k0, s, ln);
-    // face f of the line: cell (k0, j0, i0) moved f cells along DIR, in flux[DIR-1]'s layout
-    const long long* fs = B.fs[DIR - 1];
-    const long long fcell = (long long)(k0 + (DIR == 3 ? f : 0)) * fs[1] +
-                            (long long)(j0 + (DIR == 2 ? f : 0)) * fs[2] + (i0 + (DIR == 1 ? f : 0));
-    const long long fn = fs[0];
-    const size_t oL = ((size_t)t) * maxP + f;      // ql_f  (from cell f-1)
-    const size_t oR = ((size_t)t) * maxP + f + 1;  // qr_f  (from cell f)
-    const size_t vs = (size_t)T * maxP;
-    double wl[NHYDRO], wr[NHYDRO], flx[NHYDRO];
-    wl[IDN] = sL[IDN * vs + oL]; wl[IV1] = sL[ivx * vs + oL]; wl[IV2] = sL[ivy * vs + oL];
-    wl[IV3] = sL[ivz * vs + oL]; wl[IPR] = sL[IPR * vs + oL];
-    wr[IDN] = sR[IDN * vs + oR]; wr[IV1] = sR[ivx * vs + oR]; wr[IV2] = sR[ivy * vs + oR];
-    wr[IV3] = sR[ivz * vs + oR]; wr[IPR] = sR[IPR * vs + oR];
-    const double glc = sL[nvar * vs + oL], gle = sL[(nvar + 1) * vs + oL];
-    const double grc = sR[nvar * vs + oR], gre = sR[(nvar + 1) * vs + oR];
-    SolveOps o;
-#if APH_EXACT
-    bool in_range = true;
-#pragma unroll
-    for (int k = 0; k < NHYDRO; ++k) in_range &= snug(wl[k]) & snug(wr[k]);
-    if (!in_range) o.give_up();
-#endif
-    riemann<RS, false>(wl, wr, glc, gle, grc, gre, gc, flx, o);
-    if (!o.ok()) {  // an operand outside the integer pipe's range
-      IeeeOps ieee;
-      riemann<RS, false>(wl, wr, glc, gle, grc, gre, gc, flx, ieee);
+    double wl[NHYDRO], wr[NHYDRO], gm[4], flx[NHYDRO];
+    const int oL = t * w2 + f;
+    face_states<DIR, kOffsets>(w, oL, vs, V, nvar, p.gamma, wl, wr, gm);
+    if (HOW == kFluxIeee) {
+      IeeeOps o;
+      riemann<RS, false>(wl, wr, gm[0], gm[1], gm[2], gm[3], none, flx, o);
+    } else {
+      SolveOps o;
+      riemann<RS, false>(wl, wr, gm[0], gm[1], gm[2], gm[3], none, flx, o);
+      in_range = in_range & o.ok();
     }
-    flux[IDN * fn + fcell] = flx[IDN];
-    flux[ivx * fn + fcell] = flx[IV1];
-    flux[ivy * fn + fcell] = flx[IV2];
-    flux[ivz * fn + fcell] = flx[IV3];
-    flux[IEN * fn + fcell] = flx[IEN];
+    int i0, j0, k0;
+    line_geometry<DIR>(B, p.ndim, p.ng, g.l0 + t, i0, j0, k0);
+    // face f of the segment: cell (k0, j0, i0) moved c0 + f cells along DIR, in flux's layout
+    const long long *fs = B.fs[DIR - 1];
+    const int m = g.c0 + f;
+    double *out = flux + (long long)(k0 + (DIR == 3 ? m : 0)) * fs[1] + (long long)(j0 + (DIR == 2 ? m : 0)) * fs[2] +
+                  (i0 + (DIR == 1 ? m : 0));
+    const long long fn = fs[0];
+    out[IDN * fn] = flx[IDN];
+    out[ivx * fn] = flx[IV1];
+    out[ivy * fn] = flx[IV2];
+    out[ivz * fn] = flx[IV3];
+    out[IEN * fn] = flx[IEN];
     // passive scalars: upwind by the mass flux (hydro.cpp:607-615)
     for (int v = NHYDRO; v < nvar; ++v)
-      flux[v * fn + fcell] = flx[IDN] * (!is_neg(flx[IDN]) ? sL[v * vs + oL] : sR[v * vs + oR]);
+      out[v * fn] = flx[IDN] * (!is_neg(flx[IDN]) ? w.SL[v * vs + oL] : w.SR[v * vs + oL + 1]);
   }
+  return HOW == kFluxIeee || __syncthreads_and(in_range);
+}
+
+// A segment whose window left the first arithmetic's range, in chunks of lines that fit the slabs of
+// the adiabatic indices (out of line: it is rare).
+template <int DIR, int RECON, int RS>
+static __device__ __noinline__ void flux_general(const PackDev &p, const BlockDev &B, Segment g, int T,
+                                                 const unsigned *inv, double *sm) {
+  const int l0 = g.l0, nl = g.nl;
+  const int Tc = APH_EXACT ? max(1, p.nvar * T / (p.nvar + 2)) : T;
+  for (int o = 0; o < nl; o += Tc) {
+    g.l0 = l0 + o;
+    g.nl = min(Tc, nl - o);
+    __syncthreads();
+    if (APH_EXACT && flux_segment<DIR, RECON, RS, kFluxSlabs>(p, B, g, Tc, inv, sm)) continue;
+    __syncthreads();
+    flux_segment<DIR, RECON, RS, kFluxIeee>(p, B, g, Tc, inv, sm);
+  }
+}
+
+template <int DIR, int RECON, int RS>
+__global__ void __launch_bounds__(kThreads, 2) k_fluxes(const __grid_constant__ PackDev p, const BlockDev *blocks,
+                                                        int T, int M, int nseg) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ unsigned inv[7];
+  const BlockDev &B = blocks[p.block0 + blockIdx.y];
+  const int ntrans = (DIR == 1) ? B.nx[1] * B.nx[2] : (DIR == 2) ? B.nx[0] * B.nx[2] : B.nx[0] * B.nx[1];
+  const int N = B.nx[DIR - 1];
+  Segment g;
+  g.l0 = (int)(blockIdx.x / nseg) * T;
+  g.c0 = (int)(blockIdx.x % nseg) * M;
+  if (g.l0 >= ntrans || g.c0 >= N) return;
+  g.nl = min(T, ntrans - g.l0);
+  g.n = min(M, N - g.c0);
+  g.last = g.c0 + g.n == N;
+  if (threadIdx.x < 7) inv[threadIdx.x] = 0xffffffffu / (unsigned)(g.n + threadIdx.x) + 1u;
+  __syncthreads();
+  if (!flux_segment<DIR, RECON, RS, APH_EXACT ? kFluxMain : kFluxSlabs>(p, B, g, T, inv, sm))
+    flux_general<DIR, RECON, RS>(p, B, g, T, inv, sm);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -225,20 +269,39 @@ __global__ void __launch_bounds__(kThreads) k_update(PackDev p, const BlockDev *
   const double a1 = B.dx[1] * B.dx[2], a2 = B.dx[0] * B.dx[2], a3 = B.dx[0] * B.dx[1];
   const Den vol = den(B.dx[0] * B.dx[1] * B.dx[2]);
   const long long nc = B.ncell;
-  for (int n = 0; n < p.nvar; ++n) {
-    const long long q = n * nc + c;
-    const long long f1 = flux_index(B, 0, n, ck, cj, ci);
-    double du = (a1 * B.flux[0][f1 + 1] - a1 * B.flux[0][f1]);
-    if (p.ndim >= 2) {
-      const long long f2 = flux_index(B, 1, n, ck, cj, ci);
-      du += (a2 * B.flux[1][f2 + B.fs[1][2]] - a2 * B.flux[1][f2]);
+  // five variables at a time, every load before the first store (they would wait for one another)
+  const long long f0 = flux_index(B, 0, 0, ck, cj, ci), s0 = B.fs[0][0];
+  const long long f1 = p.ndim >= 2 ? flux_index(B, 1, 0, ck, cj, ci) : 0, s1 = B.fs[1][0];
+  const long long f2 = p.ndim == 3 ? flux_index(B, 2, 0, ck, cj, ci) : 0, s2 = B.fs[2][0];
+  constexpr int K = 5;
+  for (int m = 0; m < p.nvar; m += K) {
+    double x[K][8];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int n = m + k;
+      if (n >= p.nvar) break;
+      x[k][0] = B.flux[0][f0 + n * s0 + 1];
+      x[k][1] = B.flux[0][f0 + n * s0];
+      if (p.ndim >= 2) {
+        x[k][2] = B.flux[1][f1 + n * s1 + B.fs[1][2]];
+        x[k][3] = B.flux[1][f1 + n * s1];
+      }
+      if (p.ndim == 3) {
+        x[k][4] = B.flux[2][f2 + n * s2 + B.fs[2][1]];
+        x[k][5] = B.flux[2][f2 + n * s2];
+      }
+      x[k][6] = B.cons[n * nc + c];
+      x[k][7] = B.u1[n * nc + c];
     }
-    if (p.ndim == 3) {
-      const long long f3 = flux_index(B, 2, n, ck, cj, ci);
-      du += (a3 * B.flux[2][f3 + B.fs[2][1]] - a3 * B.flux[2][f3]);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (m + k >= p.nvar) break;
+      double du = (a1 * x[k][0] - a1 * x[k][1]);
+      if (p.ndim >= 2) du += (a2 * x[k][2] - a2 * x[k][3]);
+      if (p.ndim == 3) du += (a3 * x[k][4] - a3 * x[k][5]);
+      const double div = div_x(-du, vol);
+      B.cons[(m + k) * nc + c] = gam0 * x[k][6] + gam1 * x[k][7] + beta_dt * div;
     }
-    const double div = div_x(-du, vol);
-    B.cons[q] = gam0 * B.cons[q] + gam1 * B.u1[q] + beta_dt * div;
   }
 }
 
@@ -403,26 +466,40 @@ cudaError_t launch_cons_to_prim(const PackDev &p, const BlockDev *blocks, int ma
 
 template <int DIR, int RECON, int RS>
 static cudaError_t launch_fluxes_t(const PackDev &p, const BlockDev *blocks, cudaStream_t s) {
-  const int n = p.max_nx[DIR - 1];
+  // segments of at most kSegment cells (fewer where many scalars would not fit), evenly cut: their
+  // halo costs 2 G cells of window each
+  constexpr int kSegment = 160;
+  constexpr size_t kMost = 200 * 1024;
+  const int N = p.max_nx[DIR - 1];
+  int nseg = (N + kSegment - 1) / kSegment, n = (N + nseg - 1) / nseg;
+  auto bytes = [&](int T) {
+    const size_t general = pass_smem_doubles(RECON, n, APH_EXACT ? 1 : T, p.nvar + 2);
+    const size_t main = APH_EXACT ? main_smem_doubles(RECON, n, T, p.nvar) : 0;
+    return sizeof(double) * (general > main ? general : main);
+  };
+  while (bytes(1) > kMost && n > 1) {
+    ++nseg;
+    n = (N + nseg - 1) / nseg;
+  }
+  if (bytes(1) > kMost) return cudaErrorInvalidValue;
   long long ntrans;
   if (DIR == 1) ntrans = (long long)p.max_nx[1] * p.max_nx[2];
   else if (DIR == 2) ntrans = (long long)p.max_nx[0] * p.max_nx[2];
   else ntrans = (long long)p.max_nx[0] * p.max_nx[1];
-  int T = (n + 2 >= kThreads) ? 1 : kThreads / (n + 2);
-  while (T > 1 && (long long)cdiv(ntrans, T) * p.nblocks < 2LL * sm_count()) T = (T + 1) / 2;
-  const int nt = (int)std::min<long long>(kThreads, 32LL * cdiv((long long)T * (n + 2), 32));
-  const int V = p.nvar + 2;
-  const size_t smem = (size_t)2 * V * T * (n + 2) * sizeof(double);
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  int T = std::max(1, kThreads / (n + 2));
+  while (T > 1 && (bytes(T) > kMost / 2 || (long long)cdiv(ntrans, T) * nseg * p.nblocks < 2LL * sm_count()))
+    T = (T + 1) / 2;
+  const int nt = (int)std::min<long long>(kThreads, 32LL * cdiv((long long)p.nvar * T * (n + 2), 32));
+  const size_t smem = bytes(T);
   static bool attr_set = false;
-  if (!attr_set || smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_fluxes<DIR, RECON, RS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(k_fluxes<DIR, RECON, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kMost);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  dim3 grid(cdiv(ntrans, T), p.nblocks);
-  k_fluxes<DIR, RECON, RS><<<grid, nt, smem, s>>>(p, blocks, T);
+  dim3 grid(cdiv(ntrans, T) * nseg, p.nblocks);
+  k_fluxes<DIR, RECON, RS><<<grid, nt, smem, s>>>(p, blocks, T, n, nseg);
   return cudaGetLastError();
 }
 

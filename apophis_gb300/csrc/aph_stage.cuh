@@ -20,6 +20,7 @@
 #include "aph_amr.cuh"
 #include "aph_internal.h"
 #include "aph_math.cuh"
+#include "aph_window.cuh"
 
 #ifndef APH_NS
 #error "APH_NS must name the namespace of this translation unit"
@@ -128,11 +129,6 @@ __device__ __forceinline__ void tma_load_5d(unsigned dst, const void *tmap, unsi
       " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
       "l"((unsigned long long)tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
       : "memory");
-}
-
-// x / w for 0 <= x, x w < 2^32, with inv = ceil(2^32 / w).
-__device__ __forceinline__ int quick_div(int x, int w, unsigned inv) {
-  return w == 1 ? x : (int)__umulhi((unsigned)x, inv);
 }
 
 // Work distribution of a phase with n items.
@@ -438,19 +434,6 @@ __device__ __forceinline__ void line_of(const StepBlock &B, int ndim, int ng, in
   }
 }
 
-template <int RECON>
-struct Halo {
-  static constexpr int G = RECON == RECON_PPM ? 3 : RECON == RECON_PLM ? 2 : 1;
-};
-
-// Shared-memory doubles needed by one pass item of T lines of n cells with V
-// reconstructed variables.
-__host__ __device__ constexpr size_t pass_smem_doubles(int recon, int n, int T, int V) {
-  return recon == RECON_PPM
-             ? (size_t)V * T * ((n + 6) + 2 * (n + 4) + (n + 3) + (n + 2))
-             : (size_t)V * T * ((n + 2 * (recon == RECON_PLM ? 2 : 1)) + 2 * (n + 2));
-}
-
 // The arithmetic of a pass item.
 //   ARITH_MAIN   quotients and roots on the integer pipe; exact build: tame windows whose
 //                adiabatic indices are gamma to within kGamMax units of the last place, which
@@ -464,23 +447,6 @@ __host__ __device__ constexpr size_t pass_smem_doubles(int recon, int n, int T, 
 constexpr int ARITH_MAIN = 0, ARITH_SLABS = 1, ARITH_IEEE = 2;
 constexpr int ITEM_DONE = 0, ITEM_TIMEOUT = 1, ITEM_SLABS = 2, ITEM_IEEE = 3;
 
-// The adiabatic-index offsets of an item (exact build), two 16-bit values a cell: the window,
-// the PPM face values, and the left and right states.
-__host__ __device__ constexpr size_t gamma_smem_doubles(int recon, int n, int T) {
-#if APH_EXACT
-  return ((size_t)T * ((n + 2 * (recon == RECON_PPM ? 3 : recon == RECON_PLM ? 2 : 1)) + 2 * (n + 2) +
-                       (recon == RECON_PPM ? n + 3 : 0)) +
-          1) / 2;
-#else
-  return 0;
-#endif
-}
-
-// What ARITH_MAIN needs for T lines.
-__host__ __device__ constexpr size_t main_smem_doubles(int recon, int n, int T, int nvar) {
-  return pass_smem_doubles(recon, n, T, nvar) + gamma_smem_doubles(recon, n, T);
-}
-
 // Lines of a chunk that fits the two gamma slabs into the shared memory of T lines.
 __host__ __device__ constexpr int split_lines(int T, int nvar) {
   return nvar * T / (nvar + 2) > 1 ? nvar * T / (nvar + 2) : 1;
@@ -490,64 +456,6 @@ __host__ __device__ constexpr int split_lines(int T, int nvar) {
 // padded to a multiple of 16 doubles so that the staging area starts 128-byte aligned.
 __host__ __device__ constexpr size_t tma_stage_offset(int recon, int n, int T, int nvar) {
   return ((size_t)nvar * T * (n + 2 * (recon == RECON_PPM ? 3 : recon == RECON_PLM ? 2 : 1)) + 15) / 16 * 16;
-}
-
-// PPM of a pass item's window: W holds V x T lines of cells -G..n+G-1 (row width n + 2G);
-// per cell the second differences D2 and centred differences DD (cells -2..n+1), per face
-// the limited value DPH once (faces -1..n+1), then per cell the parabola limiter writes the
-// left state of face c+1 to SL[c+1] and the right state of face c to SR[c+1] (cells -1..n).
-// also(0) and also(1) run beside the face and the cell phase (the adiabatic-index offsets).
-// inv: the block's quick_div factors for the widths n + k.
-template <bool TAME, class ALSO>
-__device__ __forceinline__ void ppm_window(const double *W, double *D2, double *DD, double *DPH,
-                                           double *SL, double *SR, int V, int nl, int T, int n,
-                                           const unsigned *inv, ALSO also) {
-  constexpr int G = 3;
-  const int NW = n + 2 * G;
-  const int tid = threadIdx.x, nth = blockDim.x;
-  // row v * T + t of the slabs, position i in it and index o = row * w + i, for element it of rows
-  // of width w (o is it where the item fills its T lines, as plain-load items do)
-  const bool full = nl == T;
-  auto decode = [&](int it, int w, unsigned iw, int &row, int &i, int &o) {
-    row = quick_div(it, w, iw);
-    i = it - row * w;
-    o = it;
-    if (!full) {
-      const int v = row / nl;
-      row += v * (T - nl);
-      o = row * w + i;
-    }
-  };
-  const int w4 = n + 4, w3 = n + 3, w2 = n + 2;
-  for (int it = tid; it < V * nl * w4; it += nth) {  // cells -2..n+1
-    int row, i, o;
-    decode(it, w4, inv[4], row, i, o);
-    const double *q = W + row * NW + i + 1;
-    const double qm = q[-1], q0 = q[0], qp = q[1];
-    D2[o] = ppm_d2<TAME>(qm, q0, qp);
-    DD[o] = ppm_dd<TAME>(qm, q0, qp);
-  }
-  __syncthreads();
-  for (int it = tid; it < V * nl * w3; it += nth) {  // faces -1..n+1
-    int row, i, o;
-    decode(it, w3, inv[3], row, i, o);
-    const double *q = W + row * NW + i + 2;
-    const double *d = DD + row * w4 + i, *e = D2 + row * w4 + i;
-    DPH[o] = ppm_face<TAME>(q[-1], q[0], d[0], d[1], e[0], e[1]);
-  }
-  also(0);
-  __syncthreads();
-  for (int it = tid; it < V * nl * w2; it += nth) {  // cells -1..n
-    int row, i, o;
-    decode(it, w2, inv[2], row, i, o);
-    const double *q = W + row * NW + i + 2;
-    const double *e = D2 + row * w4 + i, *f = DPH + row * w3 + i;
-    double ql, qr;
-    ppm_cell<TAME>(q[-2], q[-1], q[0], q[1], q[2], e[0], e[1], e[2], f[0], f[1], ql, qr);
-    SL[o] = ql;
-    SR[o] = qr;
-  }
-  also(1);
 }
 
 // One pass item: lines l0..l0+nl-1 of block B along DIR, T lines of shared memory.  b: the block's
@@ -571,23 +479,15 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
   const int NW = n + 2 * G;
   const long long nc = B.ncell;
   const int tid = threadIdx.x, nth = blockDim.x;
-  // shared-memory regions (V x T x width each)
-  double *W = sm;                                  // prim window, cells -G..n+G-1
-  double *D2 = W + (size_t)V * T * NW;             // PPM: d2, cells -2..n+1
-  double *DD = D2 + (RECON == RECON_PPM ? (size_t)V * T * (n + 4) : 0);  // PPM: dd
-  double *DPH = DD + (RECON == RECON_PPM ? (size_t)V * T * (n + 4) : 0);  // PPM: face values
-  double *SR = DPH + (RECON == RECON_PPM ? (size_t)V * T * (n + 3) : 0);  // right states
-  double *SL = (RECON == RECON_PPM) ? DD : SR + (size_t)V * T * (n + 2);  // left states
-  double *F = W;                                   // fluxes, after the window is dead
+  const Window w = window_regions<RECON>(sm, n, T, V, nv);
+  double *W = w.W, *F = w.W;  // the fluxes take the window's place once it is dead
+  const double *SL = w.SL, *SR = w.SR;
 #if APH_EXACT
-  // offsets of gamma_c (low half) and gamma_e: window, PPM face values, states
-  int *GW = (int *)(sm + pass_smem_doubles(RECON, n, T, nv));
-  int *GL = GW + T * NW, *GR = GL + T * (n + 2), *GD = GR + T * (n + 2);
+  int *GW = w.GW;
   const long long gbase = __double_as_longlong(gc.gamma);
   const int godd = (int)gbase & 1;
-  auto pack2 = [](int c, int e) { return (int)((unsigned)(c & 0xffff) | ((unsigned)e << 16)); };
-  auto low = [](int x) { return (int)(short)(x & 0xffff); };
-  auto high = [](int x) { return x >> 16; };
+#else
+  const int godd = 0;
 #endif
 
   // A: load the window of prim (and gamma) along each line
@@ -630,11 +530,11 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
     for (int it = tid; it < nv * nl * NW; it += nth) {
       const int v = it / (nl * NW);
       const int r = it - v * nl * NW;
-      const int t = r / NW, w = r - t * NW;
-      const int cell = w - G + ng;  // position along the line's whole extent
+      const int t = r / NW, x0 = r - t * NW;
+      const int cell = x0 - G + ng;  // position along the line's whole extent
       const double *src = t < T1 ? stg : stg + box;
       const int tt = t < T1 ? t : t - T1;
-      W[((size_t)v * T + t) * NW + w] = DIR == 1 ? src[((size_t)v * T + tt) * L + cell]
+      W[((size_t)v * T + t) * NW + x0] = DIR == 1 ? src[((size_t)v * T + tt) * L + cell]
                                                  : src[((size_t)v * L + cell) * T + tt];
     }
   } else {
@@ -642,11 +542,11 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
     const bool src_ghosts = ghosts_from_sources(a);
     // per window cell: its line geometry and source once, then its V values
     for (int it = tid; it < per; it += nth) {
-      int t, w;
-      if (DIR == 1) { t = quick_div(it, NW, B.inv[0][2 * G]); w = it - t * NW; } else { w = it / nl; t = it - w * nl; }
+      int t, x0;
+      if (DIR == 1) { t = quick_div(it, NW, B.inv[0][2 * G]); x0 = it - t * NW; } else { x0 = it / nl; t = it - x0 * nl; }
       long long base, stride, ib, is;
       line_of<DIR>(B, a.p.ndim, a.p.ng, l0 + t, base, stride, ib, is);
-      const int c = w - G;
+      const int c = x0 - G;
       long long cell = base + (long long)c * stride;
       const StepBlock *S = &B;  // the block holding the cell's primitives
       int flipv = -1;
@@ -668,19 +568,18 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
 #pragma unroll
       for (int v = 0; v < NHYDRO; ++v) {
         const double y = flip_if(x[v], v == flipv);
-        W[(v * T + t) * NW + w] = y;
+        W[(v * T + t) * NW + x0] = y;
         if (kTame) tame_ok = tame_ok & snug(y);
       }
       for (int v = NHYDRO; v < nv; ++v) {
         const double y = P[v * snc];
-        W[(v * T + t) * NW + w] = y;
+        W[(v * T + t) * NW + x0] = y;
         if (kTame) tame_ok = tame_ok & tame(y);
       }
 #if APH_EXACT
       if (kOffsets) {
-        offset_ok = offset_ok & ((unsigned long long)(kc + kGamMax) <= 2u * kGamMax) &
-                    ((unsigned long long)(ke + kGamMax) <= 2u * kGamMax);
-        GW[t * NW + w] = pack2((int)kc, (int)ke);
+        offset_ok = offset_ok & gam_near(kc) & gam_near(ke);
+        GW[t * NW + x0] = gam_pack((int)kc, (int)ke);
       }
 #endif
       if (V > nv) {
@@ -704,16 +603,14 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
           gamma_ref(uc, gc.gm1, g_c, g_e);
         }
 #endif
-        W[(nv * T + t) * NW + w] = g_c;
-        W[((nv + 1) * T + t) * NW + w] = g_e;
+        W[(nv * T + t) * NW + x0] = g_c;
+        W[((nv + 1) * T + t) * NW + x0] = g_e;
       }
     }
   }
 #if APH_EXACT
   if (kOffsets) {
-    // gamma far enough from the ends of its binade for the offsets of all face values
-    const unsigned long long gm = (unsigned long long)gbase & 0xfffffffffffffULL;
-    if (!__syncthreads_and(tame_ok && offset_ok && gm >= 4096 && gm <= 0xfffffffffffffULL - 4096)) return ITEM_SLABS;
+    if (!__syncthreads_and(tame_ok && offset_ok && gamma_inside(gc.gamma))) return ITEM_SLABS;
   } else if (kTame) {
     if (!__syncthreads_and(tame_ok)) return ITEM_IEEE;
   } else {
@@ -723,63 +620,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
   __syncthreads();
 #endif
   // B-D: reconstruction; left state of face c+1 -> SL[c+1], right state of face c -> SR[c+1]
-  if (RECON == RECON_PPM) {
-    ppm_window<kTame>(W, D2, DD, DPH, SL, SR, V, nl, T, n, B.inv[DIR - 1], [&](int phase) {
-#if APH_EXACT
-      if (!kOffsets) return;
-      if (phase == 0) {
-        for (int it = tid; it < nl * (n + 3); it += nth) {  // faces -1..n+1
-          const int t = quick_div(it, n + 3, B.inv[DIR - 1][3]), f = it - t * (n + 3) - 1;
-          const int *g = GW + t * NW + f + G;
-          GD[it] = pack2(gam_face(low(g[-2]), low(g[-1]), low(g[0]), low(g[1]), godd),
-                         gam_face(high(g[-2]), high(g[-1]), high(g[0]), high(g[1]), godd));
-        }
-      } else {
-        for (int it = tid; it < nl * (n + 2); it += nth) {  // cells -1..n
-          const int t = quick_div(it, n + 2, B.inv[DIR - 1][2]), c = it - t * (n + 2) - 1;
-          const int *g = GW + t * NW + c + G, *f = GD + t * (n + 3) + c + 1;
-          int lc, rc, le, re;
-          gam_cell(low(g[-1]), low(g[0]), low(g[1]), low(f[0]), low(f[1]), lc, rc);
-          gam_cell(high(g[-1]), high(g[0]), high(g[1]), high(f[0]), high(f[1]), le, re);
-          GL[it] = pack2(lc, le);
-          GR[it] = pack2(rc, re);
-        }
-      }
-#endif
-    });
-  } else {
-    const int w2 = n + 2;
-    for (int it = tid; it < V * nl * w2; it += nth) {
-      int row = quick_div(it, w2, B.inv[DIR - 1][2]);
-      const int i = it - row * w2;  // cell i - 1
-      int o = it;
-      if (nl != T) {
-        row += row / nl * (T - nl);
-        o = row * w2 + i;
-      }
-      const double *q = W + row * NW + i + G - 1;
-      double ql, qr;
-      if (RECON == RECON_PLM) plm(q[-1], q[0], q[1], ql, qr);
-      else ql = qr = q[0];
-      SL[o] = ql;
-      SR[o] = qr;
-    }
-#if APH_EXACT
-    if (kOffsets) {
-      for (int it = tid; it < nl * w2; it += nth) {
-        const int t = quick_div(it, w2, B.inv[DIR - 1][2]), c = it - t * w2 - 1;
-        const int *g = GW + t * NW + c + G;
-        int lc = low(g[0]), le = high(g[0]), rc = lc, re = le;
-        if (RECON == RECON_PLM) {
-          gam_plm(low(g[-1]), low(g[0]), low(g[1]), godd, lc, rc);
-          gam_plm(high(g[-1]), high(g[0]), high(g[1]), godd, le, re);
-        }
-        GL[it] = pack2(lc, le);
-        GR[it] = pack2(rc, re);
-      }
-    }
-#endif
-  }
+  window_states<RECON, kTame, kOffsets>(w, V, nl, T, n, B.inv[DIR - 1], godd);
   __syncthreads();
   // E: Riemann solve on faces 0..n
   {
@@ -793,27 +634,8 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
     for (int it = tid; it < nl * w1; it += nth) {
       const int t = quick_div(it, w1, B.inv[DIR - 1][1]), f = it - t * w1;
       const int oL = t * w2 + f, oR = oL + 1;
-      double wl[NHYDRO], wr[NHYDRO], flx[NHYDRO];
-      wl[IDN] = SL[IDN * vs + oL]; wl[IV1] = SL[ivx * vs + oL]; wl[IV2] = SL[ivy * vs + oL];
-      wl[IV3] = SL[ivz * vs + oL]; wl[IPR] = SL[IPR * vs + oL];
-      wr[IDN] = SR[IDN * vs + oR]; wr[IV1] = SR[ivx * vs + oR]; wr[IV2] = SR[ivy * vs + oR];
-      wr[IV3] = SR[ivz * vs + oR]; wr[IPR] = SR[IPR * vs + oR];
-      double glc = 0.0, gle = 0.0, grc = 0.0, gre = 0.0;
-#if APH_EXACT
-      if (kOffsets) {
-        const int gl = GL[oL], gr = GR[oR];
-        glc = __longlong_as_double(gbase + low(gl));
-        gle = __longlong_as_double(gbase + high(gl));
-        grc = __longlong_as_double(gbase + low(gr));
-        gre = __longlong_as_double(gbase + high(gr));
-      }
-#endif
-      if (V > nv) {
-        glc = SL[nv * vs + oL];
-        gle = SL[(nv + 1) * vs + oL];
-        grc = SR[nv * vs + oR];
-        gre = SR[(nv + 1) * vs + oR];
-      }
+      double wl[NHYDRO], wr[NHYDRO], g[4], flx[NHYDRO];
+      face_states<DIR, kOffsets>(w, oL, vs, V, nv, gc.gamma, wl, wr, g);
       // store in cons order (exact: times the face's area, which both of its cells take), and the
       // boundary faces' fluxes for the coarse-fine correction
       auto times = [](auto &o, double x, double y) {
@@ -845,12 +667,12 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
       };
       if (ARITH == ARITH_IEEE) {
         IeeeOps o;
-        if (!APH_EXACT && constg) riemann<RS, true>(wl, wr, 0.0, 0.0, 0.0, 0.0, gc, flx, o);
-        else riemann<RS, false>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+        if (!APH_EXACT && constg) riemann<RS, true>(wl, wr, g[0], g[1], g[2], g[3], gc, flx, o);
+        else riemann<RS, false>(wl, wr, g[0], g[1], g[2], g[3], gc, flx, o);
         put(o);
       } else {
         SolveOps o;
-        riemann<RS, !APH_EXACT>(wl, wr, glc, gle, grc, gre, gc, flx, o);
+        riemann<RS, !APH_EXACT>(wl, wr, g[0], g[1], g[2], g[3], gc, flx, o);
         put(o);
         in_range = in_range && o.ok();
       }

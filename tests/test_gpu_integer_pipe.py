@@ -95,3 +95,25 @@ def test_default_lines_around_the_rule(n, recon):
     sk, sj, si = cfg.interior
     _same(np.ascontiguousarray(st.state()[:, :, sk, sj, si]), np.ascontiguousarray(ref.get()[:, :, sk, sj, si]))
     st.close()
+
+
+@pytest.mark.parametrize("nx,nscalars", [(159, 0), (160, 0), (161, 0), (321, 0), (1500, 0), (100, 24), (161, 40)])
+@pytest.mark.parametrize("recon", ["ppm", "plm"])
+def test_flux_segments(nx, nscalars, recon):
+    """The per-kernel path's flux kernel cuts long lines (and lines of many scalars) into segments:
+    two steps of one long block equal the oracle, exact arithmetic, and the fast ones run."""
+    from oracle import oracle as O
+    cfg, cons = problems.sod(nx=nx, recon=recon, rsolver="hllc", ng=3)
+    if nscalars:
+        cfg, cons = problems.with_tracers(cfg, cons, nscalars)
+    ref = O.Mesh(cfg)
+    ref.set_cons(cons)
+    ref.run(nsteps=2)
+    sk, sj, si = cfg.interior
+    want = ref.get()[:, :, sk, sj, si]
+    drv = hydro.Driver(cfg, cons, exact=True)
+    drv.run(nsteps=2)
+    _same(np.ascontiguousarray(drv.cons()[:, :, sk, sj, si]), np.ascontiguousarray(want))
+    fast = hydro.Driver(cfg, cons, exact=False)
+    fast.run(nsteps=2)
+    assert np.allclose(fast.cons()[:, :, sk, sj, si], want, rtol=1e-10, atol=1e-10)
