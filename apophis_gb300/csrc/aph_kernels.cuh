@@ -267,8 +267,20 @@ __global__ void __launch_bounds__(kThreads) k_update(PackDev p, const BlockDev *
   if (!interior_cell(B, p.ndim, p.ng, blockIdx.x * blockDim.x + threadIdx.x, c, ci, cj, ck)) return;
   const double beta_dt = dt_dev ? beta * dt_dev[0] : beta_dt_host;
   const double a1 = B.dx[1] * B.dx[2], a2 = B.dx[0] * B.dx[2], a3 = B.dx[0] * B.dx[1];
-  const Den vol = den(B.dx[0] * B.dx[1] * B.dx[2]);
   const long long nc = B.ncell;
+#if APH_EXACT
+  // areas, the volume and RK factors that are powers of two (every mesh of such widths) are
+  // exponent steps: the FP64 pipe is what this kernel waits for (KH 128^3: 517 us with products
+  // and a division per variable)
+  const double vol = B.dx[0] * B.dx[1] * B.dx[2];
+  const double ivol = rcp_x(vol);
+  const bool p2 = pow2_normal(vol);
+  const int k1 = pow2_step(a1), k2 = pow2_step(a2), k3 = pow2_step(a3);
+  const RkForm rk = rk_form(gam0, gam1);
+  auto times = [](double f, double area, int k) { return k != kNoStep ? scale_x(f, area, k) : f * area; };
+#else
+  const Den vol_den = den(B.dx[0] * B.dx[1] * B.dx[2]);
+#endif
   // five variables at a time, every load before the first store (they would wait for one another)
   const long long f0 = flux_index(B, 0, 0, ck, cj, ci), s0 = B.fs[0][0];
   const long long f1 = p.ndim >= 2 ? flux_index(B, 1, 0, ck, cj, ci) : 0, s1 = B.fs[1][0];
@@ -296,11 +308,21 @@ __global__ void __launch_bounds__(kThreads) k_update(PackDev p, const BlockDev *
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       if (m + k >= p.nvar) break;
+#if APH_EXACT
+      double du = times(x[k][0], a1, k1) - times(x[k][1], a1, k1);
+      if (p.ndim >= 2) du += times(x[k][2], a2, k2) - times(x[k][3], a2, k2);
+      if (p.ndim == 3) du += times(x[k][4], a3, k3) - times(x[k][5], a3, k3);
+#else
       double du = (a1 * x[k][0] - a1 * x[k][1]);
       if (p.ndim >= 2) du += (a2 * x[k][2] - a2 * x[k][3]);
       if (p.ndim == 3) du += (a3 * x[k][4] - a3 * x[k][5]);
-      const double div = div_x(-du, vol);
+#endif
+#if APH_EXACT
+      B.cons[(m + k) * nc + c] = rk_sum(rk, x[k][6], x[k][7]) + beta_dt * div_vol(-du, vol, ivol, p2);
+#else
+      const double div = div_x(-du, vol_den);
       B.cons[(m + k) * nc + c] = gam0 * x[k][6] + gam1 * x[k][7] + beta_dt * div;
+#endif
     }
   }
 }

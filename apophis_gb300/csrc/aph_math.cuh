@@ -1057,6 +1057,12 @@ __device__ __forceinline__ double scale_x(double x, double c, int k) {
     return __longlong_as_double(__double_as_longlong(x) + ((long long)k << 52));
   return is_zero(x) ? x : x * c;
 }
+// k where x = 2^k within +-400, else kNoStep
+constexpr int kNoStep = 1 << 20;
+__device__ __forceinline__ int pow2_step(double x) {
+  const int k = (__double2hiint(x) >> 20) - 1023;
+  return pow2_normal(x) && k >= -400 && k <= 400 ? k : kNoStep;
+}
 // y / vol, correctly rounded; ivol = 1 / vol, p2 = pow2_normal(vol) (uniform over a block)
 __device__ __forceinline__ double div_vol(double y, double vol, double ivol, bool p2) {
   if (!p2) return div_x(y, vol);
