@@ -37,7 +37,12 @@ __global__ void k_exact_ops2(int op, const double *x, const double *y, double *o
     else if (op == 7) r = sqrt(a);
     else if (op == 8) r = div_x(a, b);
     else if (op == 9) r = rcp_x(b);
-    else r = sqrt_x(a);
+    else if (op == 10) r = sqrt_x(a);
+    else {
+      FaceOps o;
+      r = o.mul(a, b);
+      if (!o.ok()) r = __dmul_rn(a, b);
+    }
     out[i] = r;
   }
 }

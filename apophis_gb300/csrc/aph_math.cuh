@@ -359,6 +359,11 @@ struct IntOps {
   // RN(a b), a and b zero or normal: the 106-bit product of the significands, rounded by a carry
   // chain.  13 SM-cycles per warp on pipes of its own, where a DMUL holds the FP64 pipe for 17.
   __device__ __forceinline__ double mul(double a, double b) {
+    unsigned unused;
+    return product(a, b, unused);
+  }
+  // far_e: far_of the product, before its exponent can wrap
+  __device__ __forceinline__ double product(double a, double b, unsigned &far_e) {
     const unsigned ah = (unsigned)__double2hiint(a), bh = (unsigned)__double2hiint(b);
     const unsigned ea = ah & 0x7ff00000u, eb = bh & 0x7ff00000u;
     unsigned __int128 P = (unsigned __int128)significand((unsigned long long)__double_as_longlong(a)) *
@@ -371,6 +376,7 @@ struct IntOps {
     const unsigned e = ea + eb - ((1023u + low) << 20);
     const unsigned sg = (ah ^ bh) & 0x80000000u;
     const bool z = min(ea, eb) == 0u;
+    far_e = z ? 0u : (unsigned)(m >> 32) + e - (623u << 20);
     return __hiloint2double((int)(z ? sg : (((unsigned)(m >> 32) + e) | sg)), (int)(z ? 0u : (unsigned)m));
   }
   __device__ __forceinline__ double half(double x) { return half_x(x); }
@@ -401,6 +407,17 @@ struct CheckedOps : IntOps {
     return r;
   }
 };
+// The fast solvers': an operand of a product is a state value the solver has seen, a product, a
+// quotient or a sum of those, so it is finite and zero or normal, and the exponent of the product
+// tells whether the result is.
+struct FaceOps : CheckedOps {
+  __device__ __forceinline__ double mul(double a, double b) {
+    unsigned e;
+    const double r = product(a, b, e);
+    far = max(far, e);
+    return r;
+  }
+};
 struct IeeeOps {
   static constexpr bool kInt = false;
   __device__ __forceinline__ Den den(double b) { return Den{b, 0u}; }
@@ -420,7 +437,7 @@ struct IeeeOps {
 #if APH_EXACT
 using SolveOps = IntOps;
 #else
-using SolveOps = CheckedOps;
+using SolveOps = FaceOps;
 #endif
 
 // Single operations for any operands: the digits, or the IEEE instruction where an operand is far
@@ -921,69 +938,90 @@ __device__ __forceinline__ void solve_hlle_exact(const double *wli, const double
 // are fused depends on how it splits the code into blocks, and PPM's discontinuous limiters turn
 // a difference of one rounding into a different flux, so that builds and launches would no
 // longer agree with one another.
-__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+// Their plain products take the integer pipe (FaceOps), the same bits: with PLM + HLLE the stage
+// kernel held the FP64 pipe for 67 % of its cycles (PPM + HLLC: 77 %) and the ALU for 6 (12) %.  A
+// step of the 512^2 Kelvin-Helmholtz pack (PPM + HLLC) went from 547 to 479 us with it, of the 512^2
+// rollout's forward and backward from 8.41 to 7.94 ms.
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double square3(double a, double b, double c) {  // a^2 + b^2 + c^2
-  return fma(c, c, fma(a, a, mul(b, b)));
+template <class OPS>
+__device__ __forceinline__ double square3(double a, double b, double c, OPS &o) {  // a^2 + b^2 + c^2
+  return fma(c, c, fma(a, a, o.mul(b, b)));
 }
 
 // the square of the sound speed as num / den
-template <bool CONSTG>
+template <bool CONSTG, class OPS>
 __device__ __forceinline__ void sound_parts(double rho, double p, double gamma, double igm1,
-                                            const GasConsts &gc, double &num, double &root) {
-  num = CONSTG ? mul(gc.c2g, p) : mul(mul(C_LIGHT2, gamma), p);
-  const double den = fma(p, CONSTG ? gc.one_igm1 : add(1.0, igm1), mul(rho, C_LIGHT2));
-  root = rsqrt(mul(num, den));  // the speed is num * root
+                                            const GasConsts &gc, double &num, double &root, OPS &o) {
+  num = CONSTG ? o.mul(gc.c2g, p) : o.mul(o.mul(C_LIGHT2, gamma), p);
+  const double den = fma(p, CONSTG ? gc.one_igm1 : add(1.0, igm1), o.mul(rho, C_LIGHT2));
+  root = rsqrt(o.mul(num, den));  // the speed is num * root
 }
-template <bool CONSTG>
+template <bool CONSTG, class OPS>
 __device__ __forceinline__ double sound_speed(double rho, double p, double gamma, double igm1,
-                                              const GasConsts &gc) {
+                                              const GasConsts &gc, OPS &o) {
   double num, root;
-  sound_parts<CONSTG>(rho, p, gamma, igm1, gc, num, root);
-  return mul(num, root);
+  sound_parts<CONSTG>(rho, p, gamma, igm1, gc, num, root, o);
+  return o.mul(num, root);
+}
+// the values a face's products start from
+template <bool CONSTG, class OPS>
+__device__ __forceinline__ void see_face(const double *wl, const double *wr, double glc, double gle,
+                                         double grc, double gre, OPS &o) {
+#pragma unroll
+  for (int n = 0; n < NHYDRO; ++n) {
+    o.see(wl[n]);
+    o.see(wr[n]);
+  }
+  if (!CONSTG) {
+    o.see(glc);
+    o.see(gle);
+    o.see(grc);
+    o.see(gre);
+  }
 }
 
 template <bool CONSTG, class OPS>
 __device__ __forceinline__ void solve_hlle(const double *wl, const double *wr, double glc, double gle,
                                            double grc, double gre, const GasConsts &gc, double *flx,
                                            OPS &o) {
+  see_face<CONSTG>(wl, wr, glc, gle, grc, gre, o);
   const double gl = CONSTG ? gc.gamma : glc, gr = CONSTG ? gc.gamma : grc;
   const double il = CONSTG ? gc.igm1 : o.rcp(sub(gle, 1)), ir = CONSTG ? gc.igm1 : o.rcp(sub(gre, 1));
-  const double cl = sound_speed<CONSTG>(wl[IDN], wl[IPR], gl, il, gc);
-  const double cr = sound_speed<CONSTG>(wr[IDN], wr[IPR], gr, ir, gc);
-  const double el = fma(wl[IPR], il, mul(mul(0.5, wl[IDN]), square3(wl[IV1], wl[IV2], wl[IV3])));
-  const double er = fma(wr[IPR], ir, mul(mul(0.5, wr[IDN]), square3(wr[IV1], wr[IV2], wr[IV3])));
-  const double rhoa = mul(.5, add(wl[IDN], wr[IDN])), ca = mul(.5, add(cl, cr));
-  const double pmid = mul(.5, fma(mul(sub(wl[IV1], wr[IV1]), rhoa), ca, add(wl[IPR], wr[IPR])));
+  const double cl = sound_speed<CONSTG>(wl[IDN], wl[IPR], gl, il, gc, o);
+  const double cr = sound_speed<CONSTG>(wr[IDN], wr[IPR], gr, ir, gc, o);
+  const double el = fma(wl[IPR], il, o.mul(o.half(wl[IDN]), square3(wl[IV1], wl[IV2], wl[IV3], o)));
+  const double er = fma(wr[IPR], ir, o.mul(o.half(wr[IDN]), square3(wr[IV1], wr[IV2], wr[IV3], o)));
+  const double rhoa = o.half(add(wl[IDN], wr[IDN])), ca = o.half(add(cl, cr));
+  const double pmid = o.half(fma(o.mul(sub(wl[IV1], wr[IV1]), rhoa), ca, add(wl[IPR], wr[IPR])));
   double ql = 1.0, qr = 1.0;
   const bool bl = gt(pmid, wl[IPR]), br = gt(pmid, wr[IPR]);
   if (bl || br) {
-    const double ipp = o.rcp(mul(wl[IPR], wr[IPR]));  // shared reciprocal
-    const double kl = CONSTG ? gc.hlle_k : mul(add(gl, 1), rsqrt(mul(2, gl)));
-    const double kr = CONSTG ? gc.hlle_k : mul(add(gr, 1), rsqrt(mul(2, gr)));
-    if (bl) ql = fma(kl, fma(mul(pmid, wr[IPR]), ipp, -1.0), 1.0);
-    if (br) qr = fma(kr, fma(mul(pmid, wl[IPR]), ipp, -1.0), 1.0);
+    const double ipp = o.rcp(o.mul(wl[IPR], wr[IPR]));  // shared reciprocal
+    const double kl = CONSTG ? gc.hlle_k : o.mul(add(gl, 1), rsqrt(o.twice(gl)));
+    const double kr = CONSTG ? gc.hlle_k : o.mul(add(gr, 1), rsqrt(o.twice(gr)));
+    if (bl) ql = fma(kl, fma(o.mul(pmid, wr[IPR]), ipp, -1.0), 1.0);
+    if (br) qr = fma(kr, fma(o.mul(pmid, wl[IPR]), ipp, -1.0), 1.0);
   }
   const double al = fma(-cl, ql, wl[IV1]), ar = fma(cr, qr, wr[IV1]);
   const double bp = is_pos(ar) ? ar : 0.0, bm = is_neg(al) ? al : 0.0;
   const double vl = sub(wl[IV1], bm), vr = sub(wr[IV1], bp);
   double fl[NHYDRO], fr[NHYDRO];
-  fl[IDN] = mul(wl[IDN], vl);
-  fr[IDN] = mul(wr[IDN], vr);
-  fl[IV1] = fma(mul(wl[IDN], wl[IV1]), vl, wl[IPR]);
-  fr[IV1] = fma(mul(wr[IDN], wr[IV1]), vr, wr[IPR]);
-  fl[IV2] = mul(mul(wl[IDN], wl[IV2]), vl);
-  fr[IV2] = mul(mul(wr[IDN], wr[IV2]), vr);
-  fl[IV3] = mul(mul(wl[IDN], wl[IV3]), vl);
-  fr[IV3] = mul(mul(wr[IDN], wr[IV3]), vr);
-  fl[IEN] = fma(el, vl, mul(wl[IPR], wl[IV1]));
-  fr[IEN] = fma(er, vr, mul(wr[IPR], wr[IV1]));
+  fl[IDN] = o.mul(wl[IDN], vl);
+  fr[IDN] = o.mul(wr[IDN], vr);
+  fl[IV1] = fma(o.mul(wl[IDN], wl[IV1]), vl, wl[IPR]);
+  fr[IV1] = fma(o.mul(wr[IDN], wr[IV1]), vr, wr[IPR]);
+  fl[IV2] = o.mul(o.mul(wl[IDN], wl[IV2]), vl);
+  fr[IV2] = o.mul(o.mul(wr[IDN], wr[IV2]), vr);
+  fl[IV3] = o.mul(o.mul(wl[IDN], wl[IV3]), vl);
+  fr[IV3] = o.mul(o.mul(wr[IDN], wr[IV3]), vr);
+  fl[IEN] = fma(el, vl, o.mul(wl[IPR], wl[IV1]));
+  fr[IEN] = fma(er, vr, o.mul(wr[IPR], wr[IV1]));
   double t = 0.0;
   if (__double_as_longlong(bp) != __double_as_longlong(bm) && (mag(bp) | mag(bm)) != 0ULL)
-    t = o.div0(mul(0.5, add(bp, bm)), o.den(sub(bp, bm)));
+    t = o.div0(o.half(add(bp, bm)), o.den(sub(bp, bm)));
 #pragma unroll
-  for (int n = 0; n < NHYDRO; ++n) flx[n] = fma(0.5, add(fl[n], fr[n]), mul(sub(fl[n], fr[n]), t));
+  for (int n = 0; n < NHYDRO; ++n) flx[n] = fma(0.5, add(fl[n], fr[n]), o.mul(sub(fl[n], fr[n]), t));
 }
 
 // HLLC; LOWMACH: the pstar of hydro_lhllc.hpp:71-79, whose "Mach" is the speed |v| itself
@@ -991,36 +1029,37 @@ template <bool CONSTG, bool LOWMACH, class OPS>
 __device__ __forceinline__ void solve_hllc(const double *wl, const double *wr, double glc, double gle,
                                            double grc, double gre, const GasConsts &gc, double *flx,
                                            OPS &o) {
+  see_face<CONSTG>(wl, wr, glc, gle, grc, gre, o);
   const double gl = CONSTG ? gc.gamma : glc, gr = CONSTG ? gc.gamma : grc;
   const double il = CONSTG ? gc.igm1 : o.rcp(sub(gle, 1)), ir = CONSTG ? gc.igm1 : o.rcp(sub(gre, 1));
-  const double cl = sound_speed<CONSTG>(wl[IDN], wl[IPR], gl, il, gc);
-  const double cr = sound_speed<CONSTG>(wr[IDN], wr[IPR], gr, ir, gc);
-  const double rhoa = mul(.5, add(wl[IDN], wr[IDN])), ca = mul(.5, add(cl, cr));
-  double x = mul(mul(mul(.5, sub(wr[IV1], wl[IV1])), rhoa), ca);
+  const double cl = sound_speed<CONSTG>(wl[IDN], wl[IPR], gl, il, gc, o);
+  const double cr = sound_speed<CONSTG>(wr[IDN], wr[IPR], gr, ir, gc, o);
+  const double rhoa = o.half(add(wl[IDN], wr[IDN])), ca = o.half(add(cl, cr));
+  double x = o.mul(o.mul(o.half(sub(wr[IV1], wl[IV1])), rhoa), ca);
   if (LOWMACH) {
     auto root = [&](double q) { return is_zero(q) ? q : o.sqrt(is_zero(q) ? 1.0 : q); };
-    const double chi = smax(root(square3(wl[IV1], wl[IV2], wl[IV3])), root(square3(wr[IV1], wr[IV2], wr[IV3])));
-    x = mul(x, mul(chi, sub(2.0, chi)));
+    const double chi = smax(root(square3(wl[IV1], wl[IV2], wl[IV3], o)), root(square3(wr[IV1], wr[IV2], wr[IV3], o)));
+    x = o.mul(x, o.mul(chi, sub(2.0, chi)));
   }
   const double pstar = fma(.5, add(wl[IPR], wr[IPR]), -x);
   double ql = 1.0, qr = 1.0;
   const bool bl = gt(pstar, wl[IPR]), br = gt(pstar, wr[IPR]);
   if (bl || br) {
-    const double ipp = o.rcp(mul(wl[IPR], wr[IPR]));
-    const double k = CONSTG ? gc.hllc_k : o.div(add(gl, 1), o.den(mul(2, gr)));
-    if (bl) ql = o.sqrt(fma(k, fma(mul(pstar, wr[IPR]), ipp, -1.0), 1.0));
-    if (br) qr = o.sqrt(fma(k, fma(mul(pstar, wl[IPR]), ipp, -1.0), 1.0));
+    const double ipp = o.rcp(o.mul(wl[IPR], wr[IPR]));
+    const double k = CONSTG ? gc.hllc_k : o.div(add(gl, 1), o.den(o.twice(gr)));
+    if (bl) ql = o.sqrt(fma(k, fma(o.mul(pstar, wr[IPR]), ipp, -1.0), 1.0));
+    if (br) qr = o.sqrt(fma(k, fma(o.mul(pstar, wl[IPR]), ipp, -1.0), 1.0));
   }
   const double sl = fma(-cl, ql, wl[IV1]), sr = fma(cr, qr, wr[IV1]);
   const double bp = is_pos(sr) ? sr : TINY_NUMBER;
   const double bm = is_neg(sl) ? sl : -TINY_NUMBER;
   const double vl = sub(wl[IV1], sl), vr = sub(wr[IV1], sr);
-  const double tl = fma(mul(vl, wl[IDN]), wl[IV1], wl[IPR]);
-  const double tr = fma(mul(vr, wr[IDN]), wr[IV1], wr[IPR]);
-  const double ml = mul(wl[IDN], vl), mr = -mul(wr[IDN], vr);
+  const double tl = fma(o.mul(vl, wl[IDN]), wl[IV1], wl[IPR]);
+  const double tr = fma(o.mul(vr, wr[IDN]), wr[IV1], wr[IPR]);
+  const double ml = o.mul(wl[IDN], vl), mr = -o.mul(wr[IDN], vr);
   const double imm = o.rcp(add(ml, mr));
-  const double sstar = mul(sub(tl, tr), imm);
-  double cp = mul(fma(ml, tr, mul(mr, tl)), imm);
+  const double sstar = o.mul(sub(tl, tr), imm);
+  double cp = o.mul(fma(ml, tr, o.mul(mr, tl)), imm);
   cp = is_pos(cp) ? cp : 0.0;
   // one-sided: the flux is sstar/(sstar - b) times the physical flux of the upwind side of
   // the contact (left with b = bm when sstar >= 0, else right with b = bp) plus the pressure
@@ -1031,16 +1070,16 @@ __device__ __forceinline__ void solve_hllc(const double *wl, const double *wr, d
   const double v = L ? wl[IV2] : wr[IV2], z = L ? wl[IV3] : wr[IV3];
   const double p = L ? wl[IPR] : wr[IPR];
   const double b = L ? bm : bp;
-  const double e = fma(p, L ? il : ir, mul(mul(0.5, rho), square3(u, v, z)));
+  const double e = fma(p, L ? il : ir, o.mul(o.half(rho), square3(u, v, z, o)));
   const double id = o.rcp(sub(sstar, b));
-  const double coef = mul(sstar, id);
-  const double ustar = mul(-b, id);
+  const double coef = o.mul(sstar, id);
+  const double ustar = o.mul(-b, id);
   const double vx = sub(u, b);
-  flx[IDN] = mul(coef, mul(rho, vx));
-  flx[IV1] = fma(coef, fma(mul(rho, u), vx, p), mul(ustar, cp));
-  flx[IV2] = mul(coef, mul(mul(rho, v), vx));
-  flx[IV3] = mul(coef, mul(mul(rho, z), vx));
-  flx[IEN] = fma(mul(ustar, cp), sstar, mul(coef, fma(p, u, mul(e, vx))));
+  flx[IDN] = o.mul(coef, o.mul(rho, vx));
+  flx[IV1] = fma(coef, fma(o.mul(rho, u), vx, p), o.mul(ustar, cp));
+  flx[IV2] = o.mul(coef, o.mul(o.mul(rho, v), vx));
+  flx[IV3] = o.mul(coef, o.mul(o.mul(rho, z), vx));
+  flx[IEN] = fma(o.mul(ustar, cp), sstar, o.mul(coef, fma(p, u, o.mul(e, vx))));
 }
 #endif
 
@@ -1250,7 +1289,7 @@ __device__ __forceinline__ double dt_candidate_ops(const double *w, double e_con
   const double e_k = o.mul(o.half(w[IDN]), v2);
   const double e_i = e_cons - e_k;
 #else
-  const double e_i = fma(-o.half(w[IDN]), square3(w[IV1], w[IV2], w[IV3]), e_cons);
+  const double e_i = fma(-o.half(w[IDN]), square3(w[IV1], w[IV2], w[IV3], o), e_cons);
 #endif
   const double e_internal = o.div0(e_i, o.den(w[IDN]));
   const double small = 10.0 * 2.2250738585072014e-308;
@@ -1297,7 +1336,8 @@ __device__ __forceinline__ double dt_cell(const double *w, double e_cons, const 
 #else
   if (floored) return dt_candidate(w, e_cons, dx, ndim, gc.gm1);
   double num, root;
-  sound_parts<true>(w[IDN], w[IPR], 0.0, 0.0, gc, num, root);
+  IeeeOps o;
+  sound_parts<true>(w[IDN], w[IPR], 0.0, 0.0, gc, num, root, o);
   double r = div_x(fma(num, root, dabs(w[IV1])), dx[0]);
   if (ndim > 1) {
     const double r2 = div_x(fma(num, root, dabs(w[IV2])), dx[1]);

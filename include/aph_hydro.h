@@ -322,7 +322,7 @@ aph_status aph_diag_exact_ops(int op, const double *x, double *out, long long n,
  * 1: x - y, 2: 3 * x, 3: 6 * x, 4: 1.25 * x (y unused by ops 2-4), for operands zero or normal
  * with 2^-900 < |x| < 2^900; for the FP64 pipe's operations they are weighed against,
  * 5: x / y, 6: the reciprocal 1 / y, 7: sqrt(x); and for any operands the integer-pipe
- * 8: x / y, 9: 1 / y, 10: sqrt(x). */
+ * 8: x / y, 9: 1 / y, 10: sqrt(x); and for finite operands, zero or normal, 11: x * y. */
 aph_status aph_diag_exact_ops2(int op, const double *x, const double *y, double *out, long long n,
                                void *stream);
 

@@ -13,7 +13,7 @@ from apophis_gb300.stepper import Stepper
 
 pytestmark = pytest.mark.gpu
 SIG = [0, 1, 2, 3, (1 << 52) - 1, (1 << 52) - 2, (1 << 51), (1 << 51) - 1, (1 << 51) + 1, (1 << 29) - 1, 1 << 29]
-DIV, RCP, SQRT = 8, 9, 10
+DIV, RCP, SQRT, MUL = 8, 9, 10, 11
 
 
 def _values(rng, n, lo, hi):
@@ -56,6 +56,20 @@ def test_quotients_and_roots_are_ieee(lo, hi):
         _same(_run(SQRT, a, b), np.sqrt(a))
         r = _values(rng, 100_000, 0, 1)  # roots next to representable numbers
         _same(_run(SQRT, r * r, r), np.sqrt(r * r))
+
+
+@pytest.mark.parametrize("lo,hi", [(-1, 1), (-205, -195), (195, 205), (-1022, 1023)])
+def test_face_products_are_ieee(lo, hi):
+    """Products of the fast solvers: rounded as IEEE in their range (zeros included, exponents up to
+    the largest and smallest of the operands), refused outside it."""
+    rng = np.random.default_rng(20_000 + lo * 7 + hi)
+    zero = np.array([0.0, -0.0, 1.0, -3.0, 2.0 ** 900, 2.0 ** -900])
+    a, b = (np.concatenate([_values(rng, 400_000, lo, hi), v]) for v in
+            (np.repeat(zero, zero.size), np.tile(zero, zero.size)))
+    a[:100_000] = 1.0 + rng.integers(0, 1 << 26, 100_000) * 2.0 ** -26  # products half-way between numbers
+    b[:100_000] = 1.0 + (2 * rng.integers(0, 1 << 26, 100_000) + 1) * 2.0 ** -27
+    with np.errstate(all="ignore"):
+        _same(_run(MUL, a, b), a * b)
 
 
 @pytest.mark.parametrize("recon,rsolver", [("ppm", "hllc"), ("plm", "hlle"), ("ppm", "lhllc"), ("dc", "hllc")])
