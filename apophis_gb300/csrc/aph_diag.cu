@@ -52,7 +52,7 @@ __global__ void k_exact_ops2(int op, const double *x, const double *y, double *o
 extern "C" aph_status aph_diag_exact_ops2(int op, const double *x, const double *y, double *out,
                                           long long n, void *stream) {
   clear_error();
-  if (op < 0 || op > 10) return fail(APH_ERR_INVALID, "op %d not in 0..10", op);
+  if (op < 0 || op > 11) return fail(APH_ERR_INVALID, "op %d not in 0..11", op);
   if (n < 0 || (n > 0 && (!x || !y || !out))) return fail(APH_ERR_INVALID, "NULL argument");
   if (n == 0) return APH_OK;
   const long long blocks = (n + 255) / 256;
