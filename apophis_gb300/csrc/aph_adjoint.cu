@@ -94,17 +94,38 @@ __device__ __forceinline__ void riemann_pass_vjp(const AdjMember &M, int T, int 
   const int perm[5] = {IDN, ivx, ivy, ivz, IEN};
   for (int it = threadIdx.x; it < nl * (n + 1); it += blockDim.x) {  // faces 0..n
     const int t = it / (n + 1), f = it % (n + 1);
+    auto load = [&](double *wl, double *wr, double *gf) {
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        const int v = perm[k];
+        wl[k] = SL[(v * T + t) * W2 + f];
+        wr[k] = SR[(v * T + t) * W2 + f + 1];
+        const double mhi = f < n ? MU[(v * T + t) * n + f] : 0.0;
+        const double mlo = f > 0 ? MU[(v * T + t) * n + f - 1] : 0.0;
+        gf[k] = scale * (mhi - mlo);
+      }
+    };
     double wl[5], wr[5], gf[5], gwl[5], gwr[5];
+    load(wl, wr, gf);
+    FaceOps o;
+#pragma unroll
     for (int k = 0; k < 5; ++k) {
-      const int v = perm[k];
-      wl[k] = SL[(v * T + t) * W2 + f];
-      wr[k] = SR[(v * T + t) * W2 + f + 1];
-      const double mhi = f < n ? MU[(v * T + t) * n + f] : 0.0;
-      const double mlo = f > 0 ? MU[(v * T + t) * n + f - 1] : 0.0;
-      gf[k] = scale * (mhi - mlo);
+      o.see(wl[k]);
+      o.see(wr[k]);
+      o.see(gf[k]);
     }
-    if (RS == RS_HLLE) hlle_vjp(wl, wr, M.gc, M.ic2g, gf, gwl, gwr);
-    else hllc_vjp(wl, wr, M.gc, M.ic2g, gf, gwl, gwr);
+    if (RS == RS_HLLE) hlle_vjp(wl, wr, M.gc, M.ic2g, gf, gwl, gwr, o);
+    else hllc_vjp(wl, wr, M.gc, M.ic2g, gf, gwl, gwr, o);
+    if (!o.ok()) {  // (loaded again: kept for this branch, they would cost spills in the other)
+      double x[15];
+      load(x, x + 5, x + 10);
+      riemann_vjp_ieee<RS>(x, M.gc, M.ic2g);
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        gwl[k] = x[k];
+        gwr[k] = x[5 + k];
+      }
+    }
     for (int k = 0; k < 5; ++k) {
       GL[(perm[k] * T + t) * W2 + f] = gwl[k];
       GR[(perm[k] * T + t) * W2 + f] = gwr[k];

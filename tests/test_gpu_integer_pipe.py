@@ -131,3 +131,22 @@ def test_flux_segments(nx, nscalars, recon):
     fast = hydro.Driver(cfg, cons, exact=False)
     fast.run(nsteps=2)
     assert np.allclose(fast.cons()[:, :, sk, sj, si], want, rtol=1e-10, atol=1e-10)
+
+
+@pytest.mark.parametrize("recon,rsolver", [("plm", "hlle"), ("plm", "hllc"), ("ppm", "hllc"), ("ppm", "hlle")])
+@pytest.mark.parametrize("scale", [-500, 500])
+def test_adjoint_outside_the_main_path(recon, rsolver, scale):
+    """The adjoint is linear and a power of two changes no rounding: a seed 2^scale as large (products
+    beyond the integer pipe's range) gives 2^scale times the gradient, bit for bit."""
+    from apophis_gb300.adjoint import Adjoint
+    cfg, cons = problems.kh2d_smooth(n=32, block=16, ng=4 if recon == "ppm" else 2, recon=recon,
+                                     rsolver=rsolver, integrator="rk2")
+    u = torch.from_numpy(cons).cuda()
+    lam = torch.zeros_like(u)
+    sk, sj, si = cfg.interior
+    lam[:, :, sk, sj, si] = torch.randn(lam[:, :, sk, sj, si].shape, dtype=torch.float64, device="cuda",
+                                        generator=torch.Generator(device="cuda").manual_seed(11))
+    adj = Adjoint(cfg)
+    want = adj.step_vjp(u, 2e-3, lam).clone()
+    got = adj.step_vjp(u, 2e-3, lam * 2.0 ** scale)
+    _same((got * 2.0 ** -scale).cpu().numpy(), want.cpu().numpy())
