@@ -217,8 +217,8 @@ static __device__ __noinline__ void flux_general(const PackDev &p, const BlockDe
   }
 }
 
-template <int DIR, int RECON, int RS>
-__global__ void __launch_bounds__(kThreads, 2) k_fluxes(const __grid_constant__ PackDev p, const BlockDev *blocks,
+template <int DIR, int RECON, int RS, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB) k_fluxes(const __grid_constant__ PackDev p, const BlockDev *blocks,
                                                         int T, int M, int nseg) {
   extern __shared__ __align__(16) double sm[];
   __shared__ unsigned inv[7];
@@ -486,12 +486,27 @@ cudaError_t launch_cons_to_prim(const PackDev &p, const BlockDev *blocks, int ma
   return cudaGetLastError();
 }
 
+constexpr size_t kSegmentBytes = 200 * 1024;  // the most shared memory of a segment
+
+template <int DIR, int RECON, int RS, int MINB>
+static cudaError_t launch_segments(const PackDev &p, const BlockDev *blocks, dim3 grid, int nt, size_t smem,
+                                   int T, int n, int nseg, cudaStream_t s) {
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(k_fluxes<DIR, RECON, RS, MINB>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSegmentBytes);
+    if (e != cudaSuccess) return e;
+    attr_set = true;
+  }
+  k_fluxes<DIR, RECON, RS, MINB><<<grid, nt, smem, s>>>(p, blocks, T, n, nseg);
+  return cudaGetLastError();
+}
+
 template <int DIR, int RECON, int RS>
 static cudaError_t launch_fluxes_t(const PackDev &p, const BlockDev *blocks, cudaStream_t s) {
   // segments of at most kSegment cells (fewer where many scalars would not fit), evenly cut: their
   // halo costs 2 G cells of window each
   constexpr int kSegment = 160;
-  constexpr size_t kMost = 200 * 1024;
   const int N = p.max_nx[DIR - 1];
   int nseg = (N + kSegment - 1) / kSegment, n = (N + nseg - 1) / nseg;
   auto bytes = [&](int T) {
@@ -499,30 +514,28 @@ static cudaError_t launch_fluxes_t(const PackDev &p, const BlockDev *blocks, cud
     const size_t main = APH_EXACT ? main_smem_doubles(RECON, n, T, p.nvar) : 0;
     return sizeof(double) * (general > main ? general : main);
   };
-  while (bytes(1) > kMost && n > 1) {
+  while (bytes(1) > kSegmentBytes && n > 1) {
     ++nseg;
     n = (N + nseg - 1) / nseg;
   }
-  if (bytes(1) > kMost) return cudaErrorInvalidValue;
+  if (bytes(1) > kSegmentBytes) return cudaErrorInvalidValue;
   long long ntrans;
   if (DIR == 1) ntrans = (long long)p.max_nx[1] * p.max_nx[2];
   else if (DIR == 2) ntrans = (long long)p.max_nx[0] * p.max_nx[2];
   else ntrans = (long long)p.max_nx[0] * p.max_nx[1];
   int T = std::max(1, kThreads / (n + 2));
-  while (T > 1 && (bytes(T) > kMost / 2 || (long long)cdiv(ntrans, T) * nseg * p.nblocks < 2LL * sm_count()))
+  while (T > 1 && (bytes(T) > kSegmentBytes / 2 || (long long)cdiv(ntrans, T) * nseg * p.nblocks < 2LL * sm_count()))
     T = (T + 1) / 2;
   const int nt = (int)std::min<long long>(kThreads, 32LL * cdiv((long long)p.nvar * T * (n + 2), 32));
   const size_t smem = bytes(T);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_fluxes<DIR, RECON, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kMost);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
   dim3 grid(cdiv(ntrans, T) * nseg, p.nblocks);
-  k_fluxes<DIR, RECON, RS><<<grid, nt, smem, s>>>(p, blocks, T, n, nseg);
-  return cudaGetLastError();
+  // Exact mode, more segments than two CTAs an SM: three (80 registers and some spills; 128^3 in blocks of 64^3
+  // take 5.57 ms a step where two take 5.94), or else two, whose segments end sooner (meshblocks one
+  // by one, 32^2 cells each: 1.425 ms a step against 1.46)
+  constexpr int kMost3 = APH_EXACT ? 3 : 2;
+  if ((long long)grid.x * grid.y > 2LL * sm_count())
+    return launch_segments<DIR, RECON, RS, kMost3>(p, blocks, grid, nt, smem, T, n, nseg, s);
+  return launch_segments<DIR, RECON, RS, 2>(p, blocks, grid, nt, smem, T, n, nseg, s);
 }
 
 template <int DIR>
