@@ -543,6 +543,18 @@ __device__ __forceinline__ bool cons_to_prim_any(double *u, double *w, double &g
   return cons_to_prim_tail(u, w, g_c, g_e, u_d, gm1, pfloor, ieee);
 }
 
+#if !APH_EXACT
+// Velocities into w and the returned pressure of the fast ConsToPrim.
+template <class OPS>
+__device__ __forceinline__ double fast_prim(const double *u, double u_d, double gm1, double *w, OPS &o) {
+  const double di = o.rcp(u_d);
+  w[IV1] = o.mul(u[IM1], di);
+  w[IV2] = o.mul(u[IM2], di);
+  w[IV3] = o.mul(u[IM3], di);
+  return o.mul(gm1, fma(-o.half(di), fma(u[IM3], u[IM3], fma(u[IM1], u[IM1], o.mul(u[IM2], u[IM2]))), u[IEN]));
+}
+#endif
+
 // ConsToPrim for one cell (hydro.cpp:459-531, ideal gas).  u[] is updated in place
 // by the floors (density, energy); w[] gets rho, v1, v2, v3, p; g_c, g_e the two
 // adiabatic indices.  Returns true when the pressure floor was applied.
@@ -557,14 +569,17 @@ __device__ __forceinline__ bool cons_to_prim_cell(double *u, double *w, double &
   // adiabatic indices are gamma (B / p = gm1 + 1 = p / (rho e) + 1), so one division per cell
   // (a floored density takes the reference's arithmetic below, whose indices are kept)
   if (dens_ok) {
-    const double di = rcp_x(u_d);
     w[IDN] = u_d;
-    w[IV1] = __dmul_rn(u[IM1], di);
-    w[IV2] = __dmul_rn(u[IM2], di);
-    w[IV3] = __dmul_rn(u[IM3], di);
-    const double pe =
-        __dmul_rn(gm1, fma(-__dmul_rn(0.5, di),
-                           fma(u[IM3], u[IM3], fma(u[IM1], u[IM1], __dmul_rn(u[IM2], u[IM2]))), u[IEN]));
+    FaceOps o;
+    o.see(u[IM1]);
+    o.see(u[IM2]);
+    o.see(u[IM3]);
+    o.see(u[IEN]);
+    double pe = fast_prim(u, u_d, gm1, w, o);
+    if (!o.ok()) {
+      IeeeOps ieee;
+      pe = fast_prim(u, u_d, gm1, w, ieee);
+    }
     const double wp = is_neg(pe) ? 0.0 : pe;
     if (gt(wp, pfloor)) {
       w[IPR] = wp;
@@ -589,9 +604,21 @@ __device__ __forceinline__ void plm(double q_im1, double q_i, double q_ip1, doub
                                     double &qr_i) {
   const double dql = q_i - q_im1;
   const double dqr = q_ip1 - q_i;
-  const double dq2 = dql * dqr;
   double dqm = 0.0;
+#if APH_EXACT
+  const double dq2 = dql * dqr;
   if (is_pos(dq2)) dqm = div_x(dq2, dql + dqr);
+#else
+  FaceOps o;  // (the fast kernel's FP64 pipe is the busier one)
+  o.see(dql);
+  o.see(dqr);
+  double dq2 = o.mul(dql, dqr);
+  if (is_pos(dq2)) dqm = o.div(dq2, o.den(dql + dqr));
+  if (!o.ok()) {
+    dq2 = dql * dqr;
+    dqm = is_pos(dq2) ? __ddiv_rn(dq2, dql + dqr) : 0.0;
+  }
+#endif
   ql_ip1 = q_i + dqm;
   qr_i = q_i - dqm;
 }
