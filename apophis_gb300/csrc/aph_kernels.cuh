@@ -99,7 +99,7 @@ template <int DIR, int RECON, int RS, int HOW>
 __device__ __forceinline__ bool flux_segment(const PackDev &p, const BlockDev &B, const Segment &g, int T,
                                              const unsigned *inv, double *sm) {
   constexpr int G = Halo<RECON>::G;
-  constexpr bool kTame = APH_EXACT && HOW != kFluxIeee, kOffsets = HOW == kFluxMain;
+  constexpr bool kTame = (APH_EXACT || RECON == RECON_PPM) && HOW != kFluxIeee, kOffsets = HOW == kFluxMain;
   const int nvar = p.nvar, V = kOffsets ? nvar : nvar + 2, n = g.n, nl = g.nl, NW = n + 2 * G;
   const int tid = threadIdx.x, nth = blockDim.x;
   const long long nc = B.ncell;

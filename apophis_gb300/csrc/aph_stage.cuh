@@ -469,7 +469,8 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
                                          double *sm, unsigned long long &dtmin, unsigned mbar,
                                          unsigned &tma_phase) {
   constexpr int G = Halo<RECON>::G;
-  constexpr bool kTame = APH_EXACT && ARITH != ARITH_IEEE;   // the window is tame
+  // the window is tame (fast mode: only PPM profits)
+  constexpr bool kTame = (APH_EXACT || RECON == RECON_PPM) && ARITH != ARITH_IEEE;
   constexpr bool kOffsets = APH_EXACT && ARITH == ARITH_MAIN;  // gamma as small integers
   const int n = B.nx[DIR - 1];
   const int nv = a.p.nvar;  // 5 hydro variables, then the passive scalars
@@ -491,7 +492,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
 #endif
 
   // A: load the window of prim (and gamma) along each line
-  bool tame_ok = true;    // exact: whether every window value is tame (aph_math.cuh)
+  bool tame_ok = true;    // whether every window value is tame (aph_math.cuh)
   bool offset_ok = true;  // and every adiabatic index near gamma, inside its binade
   (void)tame_ok;
   (void)offset_ok;
@@ -534,8 +535,9 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
       const int cell = x0 - G + ng;  // position along the line's whole extent
       const double *src = t < T1 ? stg : stg + box;
       const int tt = t < T1 ? t : t - T1;
-      W[((size_t)v * T + t) * NW + x0] = DIR == 1 ? src[((size_t)v * T + tt) * L + cell]
-                                                 : src[((size_t)v * L + cell) * T + tt];
+      const double y = DIR == 1 ? src[((size_t)v * T + tt) * L + cell] : src[((size_t)v * L + cell) * T + tt];
+      W[((size_t)v * T + t) * NW + x0] = y;
+      if (kTame) tame_ok = tame_ok & tame(y);
     }
   } else {
     const int per = nl * NW;
@@ -569,7 +571,7 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
       for (int v = 0; v < NHYDRO; ++v) {
         const double y = flip_if(x[v], v == flipv);
         W[(v * T + t) * NW + x0] = y;
-        if (kTame) tame_ok = tame_ok & snug(y);
+        if (kTame) tame_ok = tame_ok & (APH_EXACT ? snug(y) : tame(y));  // (snug: the solver's need)
       }
       for (int v = NHYDRO; v < nv; ++v) {
         const double y = P[v * snc];
@@ -617,7 +619,11 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
     __syncthreads();
   }
 #else
-  __syncthreads();
+  if (kTame) {
+    if (!__syncthreads_and(tame_ok)) return ITEM_IEEE;
+  } else {
+    __syncthreads();
+  }
 #endif
   // B-D: reconstruction; left state of face c+1 -> SL[c+1], right state of face c -> SR[c+1]
   window_states<RECON, kTame, kOffsets>(w, V, nl, T, n, B.inv[DIR - 1], godd);

@@ -94,6 +94,31 @@ def test_exact_stepper_outside_the_main_path(recon, rsolver, gamma, scale):
     st.close()
 
 
+@pytest.mark.parametrize("recon,rsolver", [("ppm", "hllc"), ("ppm", "hlle"), ("ppm", "lhllc"), ("plm", "hlle")])
+@pytest.mark.parametrize("scale", [-190, 195, -260, 300])
+@pytest.mark.parametrize("path", ["stepper", "driver"])
+def test_fast_mode_outside_the_main_path(recon, rsolver, scale, path):
+    """Fast mode, densities and energies 2^scale as large (at the edges of tame windows and beyond,
+    and products out of range): every operation rounds as before (rsqrt to an ulp), so two steps give
+    2^scale times the unscaled ones."""
+    cfg, cons = problems.kh2d(n=32, block=16, ng=3, recon=recon, rsolver=rsolver)
+    cfg = dataclasses.replace(cfg, dfloor=0.0, pfloor=0.0)
+    out = []
+    for k in (0, scale):
+        if path == "driver":
+            dr = hydro.Driver(cfg, cons * 2.0 ** k, exact=False)
+            dr.run(nsteps=2)
+            got = dr.cons()
+        else:
+            st = Stepper(cfg, cons * 2.0 ** k, exact=False)
+            st.step(2)
+            got = st.state()
+            st.close()
+        sk, sj, si = cfg.interior
+        out.append(got[:, :, sk, sj, si] * 2.0 ** -k)
+    assert np.allclose(out[1], out[0], rtol=1e-12, atol=1e-13)
+
+
 @pytest.mark.parametrize("n", [125, 126, 127, 221, 222, 250])
 @pytest.mark.parametrize("recon", ["ppm", "plm"])
 def test_default_lines_around_the_rule(n, recon):
