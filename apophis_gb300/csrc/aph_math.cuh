@@ -1,8 +1,8 @@
 // aph_math.cuh -- device arithmetic of the hydro flux path (sm_103a).
 //
-// On GB300 every FP64 instruction -- add, mul, fma, but also compare (DSETP) and
-// min/max -- goes through a pipe that retires about two warp-lanes per clock per SM,
-// while the integer and FP32 pipes run about sixty times faster.  The predicates and
+// On GB300 every FP64 instruction -- add, mul, fma, but also compare (DSETP), negation,
+// absolute value and min/max -- holds a pipe that takes 17 cycles of an SM for a warp, where
+// an integer or FP32 one takes half a cycle.  Quotients, roots, most products, predicates and
 // min/max below therefore work on the IEEE bit patterns with integer instructions.
 // They give the same answer as the IEEE comparison for every non-NaN input, -0.0 and
 // +0.0 included, so using them changes no result bit.
@@ -83,12 +83,12 @@ __device__ __forceinline__ double from_bits(unsigned long long b) { return __lon
 // b strictly between a and c: the reference's sign test (b - a) * (c - b) > 0 without the FP64
 // subtractions and product (a difference of finite doubles is zero only when they are
 // equal; the two differ only where the product underflows to zero, for differences of
-// order 1e-162).  Fast mode.
+// order 1e-162).  Fast mode, and tame windows.
 __device__ __forceinline__ bool strictly_between(double a, double b, double c) {
   const long long ka = okey(a), kb = okey(b), kc = okey(c);
   return ((ka < kb) & (kb < kc)) | ((ka > kb) & (kb > kc));
 }
-// x beyond both a and b on the same side: the sign test (x - a) * (b - x) < 0.  Fast mode.
+// x beyond both a and b on the same side: the sign test (x - a) * (b - x) < 0.  As above.
 __device__ __forceinline__ bool strictly_outside(double x, double a, double b) {
   const long long kx = okey(x), ka = okey(a), kb = okey(b);
   return ((kx > ka) & (kx > kb)) | ((kx < ka) & (kx < kb));
@@ -149,75 +149,7 @@ __device__ __forceinline__ double div6_x(double x) {
   return is_zero(x) ? x : __longlong_as_double((long long)r);  // +-0 / 6 = +-0
 }
 
-// ---- IEEE double additions and small multiplications on the integer pipe ---------------
-// Round-to-nearest-even sums and products by 3, 5/4 and 6 computed with 64-bit integer
-// arithmetic (the textbook alignment with a sticky bit, guard bits, renormalisation and
-// rounding), for operands that are zero or normal with 2^-900 < |x| < 2^900 and results that
-// stay so -- every value the reconstruction forms from a tame window.  They return exactly the
-// bits of the FP64 instruction they replace, on a pipe that retires ~60 times more lanes per
-// clock than GB300's FP64 pipe.
-
-// Pack a positive significand S (leading 1 at bit 62, sticky bits below bit 10) with biased
-// exponent e and sign bit sg, rounding to nearest even.
-__device__ __forceinline__ double round_pack_x(unsigned long long sg, long long e, unsigned long long S) {
-  const unsigned long long r = S & 0x3ffULL;
-  unsigned long long m = S >> 10;  // 53 bits, leading 1 at bit 52
-  if (r > 0x200ULL || (r == 0x200ULL && (m & 1ULL))) ++m;
-  if (m >> 53) {  // rounding carried into bit 53
-    m >>= 1;
-    ++e;
-  }
-  return __longlong_as_double((long long)(sg | ((unsigned long long)e << 52) | (m & 0xfffffffffffffULL)));
-}
-
-// RN(a + b)
-__device__ __forceinline__ double add_x(double a, double b) {
-  unsigned long long ua = (unsigned long long)__double_as_longlong(a);
-  unsigned long long ub = (unsigned long long)__double_as_longlong(b);
-  unsigned long long ma = ua & 0x7fffffffffffffffULL, mb = ub & 0x7fffffffffffffffULL;
-  if (mb > ma) {  // |a| >= |b| from here on
-    const unsigned long long t = ua;
-    ua = ub;
-    ub = t;
-    const unsigned long long tm = ma;
-    ma = mb;
-    mb = tm;
-  }
-  const unsigned long long sg = ua & 0x8000000000000000ULL;
-  if (mb == 0) {  // b is a zero: a, or the sum of two zeros (-0 only for -0 + -0)
-    if (ma != 0) return __longlong_as_double((long long)ua);
-    return __longlong_as_double((long long)(ua & ub));
-  }
-  const long long ea = (long long)(ma >> 52), eb = (long long)(mb >> 52);
-  const long long d = ea - eb;
-  if (d > 55) return __longlong_as_double((long long)ua);  // |b| below a quarter ulp of a
-  // significands with 9 guard bits (leading 1 at bit 61); b's shifted out bits as a sticky bit
-  const unsigned long long A = ((ma & 0xfffffffffffffULL) | 0x10000000000000ULL) << 9;
-  const unsigned long long Bf = ((mb & 0xfffffffffffffULL) | 0x10000000000000ULL) << 9;
-  const unsigned long long Bt = Bf >> d;
-  const unsigned long long st = ((Bf << (63 - d)) << 1) != 0 ? 1ULL : 0ULL;  // only for d >= 10
-  long long e = ea;
-  unsigned long long S;
-  if (((ua ^ ub) >> 63) == 0) {  // same signs: the sum's floor, sticky; leading 1 at bit 61 or 62
-    S = (A + Bt) | st;
-    if (S >> 62) {
-      S = (S >> 1) | (S & 1ULL);
-      ++e;
-    }
-    S <<= 1;  // leading 1 at bit 62
-  } else {  // the difference's floor (sticky: b was truncated, subtract one more), then sticky
-    S = A - Bt - st;
-    if (S == 0) return 0.0;  // x - x = +0 (st is 0 then)
-    const int sh = __clzll((long long)S) - 1;  // bring the leading 1 to bit 62 (sh <= 2 if st)
-    S = (S << sh) | st;
-    e -= sh - 1;
-  }
-  return round_pack_x(sg, e, S);
-}
-__device__ __forceinline__ double sub_x(double a, double b) {
-  return add_x(a, __longlong_as_double(__double_as_longlong(b) ^ (long long)0x8000000000000000ULL));
-}
-
+// ---- IEEE double multiplications by constants on the integer pipe -------------------------
 // RN(k * x) for k = C * 2^S2 with C = 3 (k = 3 or 6) or C = 5 (k = 1.25): the product of the
 // significand and C is one or two (C = 5: two or three) bits longer than a significand.
 template <int C, int S2>
@@ -456,14 +388,6 @@ __device__ __forceinline__ double div_x(double a, double b) { return div_x(a, de
 __device__ __forceinline__ double rcp_x(double b) {
   if (far_of(b) >= kFar) return __drcp_rn(b);
   return quot_bits(0x3ff0000000000000ULL, (unsigned long long)__double_as_longlong(b), den(b).R);
-}
-__device__ __forceinline__ double mul_x(double a, double b) {
-  CheckedOps o;
-  o.see(a);
-  o.see(b);
-  const double r = o.IntOps::mul(a, b);
-  if (!o.ok()) return __dmul_rn(a, b);
-  return r;
 }
 __device__ __forceinline__ double sqrt_x(double x) {
   if (is_zero(x)) return x;
@@ -861,20 +785,6 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
   qr_i = qr;
 }
 
-// Whole-cell PPM from the five-point stencil (used where the face values are not shared).
-__device__ __forceinline__ void ppm(double q_im2, double q_im1, double q_i, double q_ip1,
-                                    double q_ip2, double &ql_ip1, double &qr_i) {
-  const double dd_m1 = ppm_dd(q_im2, q_im1, q_i);
-  const double dd_0 = ppm_dd(q_im1, q_i, q_ip1);
-  const double dd_p1 = ppm_dd(q_i, q_ip1, q_ip2);
-  const double d2_m1 = ppm_d2(q_im2, q_im1, q_i);
-  const double d2_0 = ppm_d2(q_im1, q_i, q_ip1);
-  const double d2_p1 = ppm_d2(q_i, q_ip1, q_ip2);
-  const double lo = ppm_face(q_im1, q_i, dd_m1, dd_0, d2_m1, d2_0);
-  const double hi = ppm_face(q_i, q_ip1, dd_0, dd_p1, d2_0, d2_p1);
-  ppm_cell(q_im2, q_im1, q_i, q_ip1, q_ip2, d2_m1, d2_0, d2_p1, lo, hi, ql_ip1, qr_i);
-}
-
 #if APH_EXACT
 // ---- reconstruction of the adiabatic indices as small integers --------------------------
 // Where no floor fired, gamma_c = B / p and gamma_e = p / (rho e) + 1 are gamma up to a few
@@ -941,18 +851,6 @@ __device__ __forceinline__ void gam_plm(int qm, int q0, int qp, int odd, int &ql
 }
 #endif
 
-template <int RECON>
-__device__ __forceinline__ void reconstruct(const double *q, double &ql_ip1, double &qr_i) {
-  // q[-2..2] addressable around q[0]
-  if (RECON == RECON_DC) {
-    ql_ip1 = qr_i = q[0];
-  } else if (RECON == RECON_PLM) {
-    plm(q[-1], q[0], q[1], ql_ip1, qr_i);
-  } else {
-    ppm(q[-2], q[-1], q[0], q[1], q[2], ql_ip1, qr_i);
-  }
-}
-
 // ---- Riemann solvers (src/hydro/rsolvers) -------------------------------------------
 // wl, wr: (rho, v_normal, v_t1, v_t2, p).  gl*, gr*: reconstructed (gamma_c, gamma_e).
 // With CONSTG the adiabatic indices are the pack's constants (gc) instead.
@@ -1015,8 +913,9 @@ __device__ __forceinline__ void solve_hlle_exact(const double *wli, const double
 // longer agree with one another.
 // Their plain products take the integer pipe (FaceOps), the same bits: with PLM + HLLE the stage
 // kernel held the FP64 pipe for 67 % of its cycles (PPM + HLLC: 77 %) and the ALU for 6 (12) %.  A
-// step of the 512^2 Kelvin-Helmholtz pack (PPM + HLLC) went from 547 to 479 us with it, of the 512^2
-// rollout's forward and backward from 8.41 to 7.94 ms.
+// step of the 512^2 Kelvin-Helmholtz pack (PLM + HLLE) went from 547 to 479 us with it, of the
+// 512^2 rollout the forward and backward from 8.41 to 7.94 ms (415 us and 6.55 ms with the products
+// of PLM and ConsToPrim there too).
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
 template <class OPS>
