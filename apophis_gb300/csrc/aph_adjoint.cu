@@ -16,6 +16,7 @@
 // APH_ERR_STATE.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/aph_hydro.h"
@@ -285,48 +286,58 @@ __global__ void __launch_bounds__(256, 2) k_adj_pass_ppm(AdjGeom g, const double
   const int tid = threadIdx.x, nth = blockDim.x;
   const Lines<DIR> line(g, l0);
   const Split by_nw(NW, nl), by_n(n, nl), by_w2(W2, nl), by_w3(W3, nl), by_w4(W4, nl);
+  bool tame_ok = true;
   for (int it = tid; it < 5 * nl * NW; it += nth) {
     int v, t;
     const int w = by_nw(it, v, t);
-    W[(v * T + t) * NW + w] = P[v * nc + line(t) + (w - G) * line.stride];
+    const double x = P[v * nc + line(t) + (w - G) * line.stride];
+    W[(v * T + t) * NW + w] = x;
+    tame_ok = tame_ok & tame(x);
   }
   for (int it = tid; it < 5 * nl * n; it += nth) {
     int v, t;
     const int c = by_n(it, v, t);
     MU[(v * T + t) * n + c] = Mu[v * nc + line(t) + c * line.stride];
   }
-  __syncthreads();
+  const bool all_tame = __syncthreads_and(tame_ok);
   auto q = [&](int v, int t, int c) { return W[(v * T + t) * NW + c + G]; };
-  for (int it = tid; it < 5 * nl * W4; it += nth) {  // cells -2..n+1
-    int v, t;
-    const int c = by_w4(it, v, t) - 2;
-    D2[(v * T + t) * W4 + c + 2] = ppm_d2(q(v, t, c - 1), q(v, t, c), q(v, t, c + 1));
-    DD[(v * T + t) * W4 + c + 2] = ppm_dd(q(v, t, c - 1), q(v, t, c), q(v, t, c + 1));
-  }
-  __syncthreads();
-  for (int it = tid; it < 5 * nl * W3; it += nth) {  // faces -1..n+1
-    int v, t;
-    const int f = by_w3(it, v, t) - 1;
-    const size_t o4 = (size_t)(v * T + t) * W4;
-    int code;
-    DPH[(v * T + t) * W3 + f + 1] = ppm_face_code(q(v, t, f - 1), q(v, t, f), DD[o4 + f + 1], DD[o4 + f + 2],
-                                                  D2[o4 + f + 1], D2[o4 + f + 2], code);
-    FB[(v * T + t) * W3 + f + 1] = code;
-  }
-  __syncthreads();
-  for (int it = tid; it < 5 * nl * W2; it += nth) {  // cells -1..n
-    int v, t;
-    const int c = by_w2(it, v, t) - 1;
-    const size_t o4 = (size_t)(v * T + t) * W4, o3 = (size_t)(v * T + t) * W3, o2 = (size_t)(v * T + t) * W2;
-    double ql, qr, rho;
-    int code;
-    ppm_cell_code(q(v, t, c - 2), q(v, t, c - 1), q(v, t, c), q(v, t, c + 1), q(v, t, c + 2), D2[o4 + c + 1],
-                  D2[o4 + c + 2], D2[o4 + c + 3], DPH[o3 + c + 1], DPH[o3 + c + 2], ql, qr, code, rho);
-    SL[o2 + c + 1] = ql;
-    SR[o2 + c + 1] = qr;
-    RHO[o2 + c + 1] = rho;
-    CB[o2 + c + 1] = code;
-  }
+  // face states and the branches taken; tame windows scale on the integer pipe, the same bits
+  // (the blast rollouts, forward and backward: 5.13 -> 4.77 ms)
+  auto states = [&](auto tame_window) {
+    constexpr bool kTame = decltype(tame_window)::value;
+    for (int it = tid; it < 5 * nl * W4; it += nth) {  // cells -2..n+1
+      int v, t;
+      const int c = by_w4(it, v, t) - 2;
+      D2[(v * T + t) * W4 + c + 2] = ppm_d2<kTame>(q(v, t, c - 1), q(v, t, c), q(v, t, c + 1));
+      DD[(v * T + t) * W4 + c + 2] = ppm_dd<kTame>(q(v, t, c - 1), q(v, t, c), q(v, t, c + 1));
+    }
+    __syncthreads();
+    for (int it = tid; it < 5 * nl * W3; it += nth) {  // faces -1..n+1
+      int v, t;
+      const int f = by_w3(it, v, t) - 1;
+      const size_t o4 = (size_t)(v * T + t) * W4;
+      int code;
+      DPH[(v * T + t) * W3 + f + 1] = ppm_face_code<kTame>(q(v, t, f - 1), q(v, t, f), DD[o4 + f + 1], DD[o4 + f + 2],
+                                                    D2[o4 + f + 1], D2[o4 + f + 2], code);
+      FB[(v * T + t) * W3 + f + 1] = code;
+    }
+    __syncthreads();
+    for (int it = tid; it < 5 * nl * W2; it += nth) {  // cells -1..n
+      int v, t;
+      const int c = by_w2(it, v, t) - 1;
+      const size_t o4 = (size_t)(v * T + t) * W4, o3 = (size_t)(v * T + t) * W3, o2 = (size_t)(v * T + t) * W2;
+      double ql, qr, rho;
+      int code;
+      ppm_cell_code<kTame>(q(v, t, c - 2), q(v, t, c - 1), q(v, t, c), q(v, t, c + 1), q(v, t, c + 2), D2[o4 + c + 1],
+                    D2[o4 + c + 2], D2[o4 + c + 3], DPH[o3 + c + 1], DPH[o3 + c + 2], ql, qr, code, rho);
+      SL[o2 + c + 1] = ql;
+      SR[o2 + c + 1] = qr;
+      RHO[o2 + c + 1] = rho;
+      CB[o2 + c + 1] = code;
+    }
+  };
+  if (all_tame) states(std::true_type{});
+  else states(std::false_type{});
   __syncthreads();
   riemann_pass_vjp<DIR, RS>(g.mem[g.blk[b].member], T, nl, n, W2, SL, SR, MU,
                             pass_scale<DIR>(g, b, beta, dt), GL, GR);

@@ -71,20 +71,25 @@ constexpr int PF_OPEN = 0, PF_AVG = 1, PF_D2M = 2, PF_D20 = 3, PF_QA = 4;
 
 // ppm_face (fast arithmetic) returning the branch: OPEN (unlimited), or limited with
 // qd = 0 (AVG), C2 d2(f-1) (D2M), C2 d2(f) (D20), or qa (QA).
+// TAME: every window value tame, the scalings on the integer pipe (the same bits).
+template <bool TAME>
 __device__ __forceinline__ double ppm_face_code(double qm1, double q0, double ddm1, double dd0,
                                                 double d2m1, double d20, int &code) {
-  const double avg = 0.5 * (qm1 + q0);
+  const double s = qm1 + q0;
+  const double avg = TAME ? half_x(s) : 0.5 * s;
   double dph = fma(ddm1 - dd0, 1.0 / 6.0, avg);
-  const double qa = 3.0 * (qm1 + q0 - 2.0 * dph);
   code = PF_OPEN;
   if (strictly_outside(dph, qm1, q0)) {  // the forward's test (ppm_face, fast mode)
+    const double qa_3 = fma(-2.0, dph, s);
+    const double qa = TAME ? mulk_x<3, 0>(qa_3) : 3.0 * qa_3;
     double qd = 0.0;
     code = PF_AVG;
     const bool sa = is_neg(qa);
     if (sa == is_neg(d2m1) && sa == is_neg(d20)) {
       const unsigned long long mb = mag(d2m1), mc = mag(d20);
       const bool pick_c = mc < mb;
-      const unsigned long long mm = mag(PPM_C2 * from_bits(pick_c ? mc : mb)), ma = mag(qa);
+      const double m = from_bits(pick_c ? mc : mb);
+      const unsigned long long mm = mag(TAME ? mulk_x<5, -2>(m) : PPM_C2 * m), ma = mag(qa);
       if (ma < mm) {
         qd = qa;
         code = PF_QA;
@@ -116,19 +121,42 @@ __device__ __forceinline__ void ppm_face_coef(int code, double c[4]) {
 // ppm_cell (fast arithmetic) returning its branch: bit 0 extremum; extremum: bits 1-3 the
 // source of qe (0 none, 1..3 C2 d2 of cell i-1, i, i+1, 4 d2qf), bit 4 the ratio applied;
 // monotone: bit 1 qr steepened, bit 2 ql steepened.  rho: the ratio used.
+template <bool TAME>
 __device__ __forceinline__ void ppm_cell_code(double q_im2, double q_im1, double q_i, double q_ip1,
                                               double q_ip2, double d2m1, double d20, double d2p1,
                                               double dph_lo, double dph_hi, double &ql, double &qr,
                                               int &code, double &rho) {
-  const double d2qf = 6.0 * (dph_lo + dph_hi - 2.0 * q_i);
   qr = dph_lo;
   ql = dph_hi;
   const double dqf_minus = q_i - qr;
   const double dqf_plus = ql - q_i;
   code = 0;
   rho = 0.0;
+  if (TAME) {
+    double f = 2.0, xm = dqf_plus, xp = dqf_minus;
+    bool sub_m = mag(dqf_minus) >= twice_mag(dqf_plus), add_p = mag(dqf_plus) >= twice_mag(dqf_minus);
+    code = (sub_m ? 2 : 0) | (add_p ? 4 : 0);
+    if (!strictly_between(qr, q_i, ql) | !strictly_between(q_im1, q_i, q_ip1)) {
+      const double d2qf = mulk_x<3, 1>(fma(-2.0, q_i, dph_lo + dph_hi));
+      bool guard;
+      int src;
+      const double qe = extremum_qe(d2qf, d2m1, d20, d2p1, q_im2, q_im1, q_i, q_ip1, q_ip2, guard, src);
+      IntOps o;
+      const double q = o.div0(qe, o.den(d2qf));
+      rho = f = guard ? q : 0.0;
+      xm = dqf_minus;
+      xp = dqf_plus;
+      sub_m = add_p = le(f, 1.0 - 1.0e-12);
+      code = 1 | (src << 1) | (sub_m ? 16 : 0);
+    }
+    const double rm = fma(-f, xm, q_i), lp = fma(f, xp, q_i);
+    qr = sub_m ? rm : qr;
+    ql = add_p ? lp : ql;
+    return;
+  }
   if (!strictly_between(qr, q_i, ql) || !strictly_between(q_im1, q_i, q_ip1)) {  // as ppm_cell
     code = 1;
+    const double d2qf = 6.0 * (dph_lo + dph_hi - 2.0 * q_i);
     double qe = 0.0;
     int src = 0;
     const bool sd = is_neg(d2qf);

@@ -646,17 +646,22 @@ __device__ __forceinline__ double ppm_face(double qm1, double q0, double ddm1, d
   return dph;
 }
 
-// The limited curvature of an extremum with d2qf, tame operands; guard: whether d2qf counts.
+// The limited curvature of an extremum with d2qf, tame operands; guard: whether d2qf counts; src:
+// where it comes from (0 nowhere, 1..3 the cell i-1, i, i+1, 4 d2qf itself).
 __device__ __forceinline__ double extremum_qe(double d2qf, double d2m1, double d20, double d2p1, double q_im2,
-                                              double q_im1, double q_i, double q_ip1, double q_ip2, bool &guard) {
+                                              double q_im1, double q_i, double q_ip1, double q_ip2, bool &guard,
+                                              int &src) {
   const bool sd = is_neg(d2qf);
   unsigned long long m = mag(d2m1);
   const unsigned long long m0 = mag(d20), m1 = mag(d2p1), md = mag(d2qf);
+  src = m0 < m ? 2 : 1;
   m = m0 < m ? m0 : m;
+  src = m1 < m ? 3 : src;
   m = m1 < m ? m1 : m;
   const unsigned long long ms = mag(mulk_x<5, -2>(from_bits(m)));
   const bool same = (sd == is_neg(d2m1)) & (sd == is_neg(d20)) & (sd == is_neg(d2p1));
   const double qe = same ? flip_if(from_bits(md < ms ? md : ms), sd) : 0.0;
+  src = same ? (md < ms ? 4 : src) : 0;
   unsigned long long mx = mag(q_im2);
   const unsigned long long a1 = mag(q_im1), a2 = mag(q_i), a3 = mag(q_ip1), a4 = mag(q_ip2);
   mx = a1 > mx ? a1 : mx;
@@ -694,7 +699,8 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
     if (!strictly_between(qr, q_i, ql) | !strictly_between(q_im1, q_i, q_ip1)) {
       const double d2qf = mulk_x<3, 1>((dph_lo + dph_hi) - twice_x(q_i));
       bool guard;
-      const double qe = extremum_qe(d2qf, d2m1, d20, d2p1, q_im2, q_im1, q_i, q_ip1, q_ip2, guard);
+      int src;
+      const double qe = extremum_qe(d2qf, d2m1, d20, d2p1, q_im2, q_im1, q_i, q_ip1, q_ip2, guard, src);
       IntOps o;  // (tame operands: all in range)
       // rho = qe / d2qf with the guard, else +0.  Where it is a zero (of qe's and d2qf's signs with
       // the guard) the steps are signed zeros; where qe is d2qf it is 1 > 1 - 1e-12: the face
@@ -732,7 +738,8 @@ __device__ __forceinline__ void ppm_cell(double q_im2, double q_im1, double q_i,
     if (!strictly_between(qr, q_i, ql) | !strictly_between(q_im1, q_i, q_ip1)) {
       const double d2qf = mulk_x<3, 1>(fma(-2.0, q_i, dph_lo + dph_hi));
       bool guard;
-      const double qe = extremum_qe(d2qf, d2m1, d20, d2p1, q_im2, q_im1, q_i, q_ip1, q_ip2, guard);
+      int src;
+      const double qe = extremum_qe(d2qf, d2m1, d20, d2p1, q_im2, q_im1, q_i, q_ip1, q_ip2, guard, src);
       IntOps o;
       const double rho = o.div0(qe, o.den(d2qf));
       f = guard ? rho : 0.0;
