@@ -207,10 +207,12 @@ void destroy_graph(aph_stepper s) {
   s->graph = nullptr;
 }
 
-// The launch configuration of a new stepper.  A pack whose passes hold several items per SM takes the
-// build for three CTAs per SM in exact mode (KH 192^3: 21.5 against 22.9 ms per RK2 step, refined RT 1.45
-// against 1.69; fast mode is the other way round, KH 512^2 PLM 0.57 against 0.53) and, where a CTA
-// gets more than a few, the dynamic schedule (KH 192^3: 21.2 against 22.4 ms strided).  A smaller pack
+// The launch configuration of a new stepper.  A pack whose passes hold more than two items per SM takes
+// the build for three CTAs per SM (exact: KH 192^3 21.5 against 22.9 ms per RK2 step, refined RT 1.45
+// against 1.69; fast: KH 128^3 PPM + HLLC 4.7 against 5.4, KH 512^2 PLM + HLLE 0.368 against 0.390) and,
+// where the items are more than those CTAs, the dynamic schedule: a strided second round leaves most
+// of them idle (fast KH 320^2, 3.6 items per SM: PLM 0.189 against 0.228 ms, PPM 0.225 against 0.304;
+// exact, PPM, 0.307 against 0.413; 256^2, 2.3 items: 0.142 against 0.136 strided).  A smaller pack
 // never fills an SM twice: registers as needed, no work counter.
 void default_launch(aph_stepper s) {
   int dev = 0, sms = 0;
@@ -231,8 +233,8 @@ void default_launch(aph_stepper s) {
   }
   c.use_graph = 1;
   c.tma = 0;
-  c.reg_cap = s->params.exact && most > 2LL * sms ? 1 : 0;
-  c.schedule = most > 6LL * sms ? 2 : 0;
+  c.reg_cap = most > 2LL * sms ? 1 : 0;
+  c.schedule = most > 3LL * sms ? 2 : 0;
 }
 
 // TMA staging of pass windows (cfg.tma): every block of the same size, laid out back to back
