@@ -66,13 +66,13 @@ BYTES_PER_ZONE_UPDATE = 200.0   # RK2 with 5 FP64 conserved variables
 # FP64 work of the stage kernel per RK2 zone-update on this workload: the DADD + DMUL + DFMA
 # thread instructions the kernel executes (ncu sass counters of one stage launch of each kind
 # on a 128^3 pack of 64^3 blocks, per zone), by arithmetic mode
-FP64_LANE_OPS_PER_ZONE_UPDATE = {"fast": 1981.0, "exact": 2364.0}
+FP64_LANE_OPS_PER_ZONE_UPDATE = {"fast": 789.0, "exact": 752.0}
 FP64_LANES_PER_CLK_PER_SM = 2.0    # DFMA lanes per clock per SM on GB300 (measured)
 # DRAM bytes (read + write) per zone per stage launch, same captures (the 256^3 launches
 # process 8x the blocks of the 128^3 capture, so traffic is scaled by zones)
-TRAFFIC_BYTES_PER_ZONE_LAUNCH = {"fast": 628.3, "exact": 612.7}
-TRAFFIC_LAUNCH = {"fast": "8 lines, dynamic schedule (not the tuned launch)",
-                  "exact": "256 threads, 3 lines, dynamic schedule, 80-register build: the tuned launch"}
+TRAFFIC_BYTES_PER_ZONE_LAUNCH = {"fast": 560.1, "exact": 619.6}
+TRAFFIC_LAUNCH = {"fast": "the default launch: 256 threads, 3 lines, dynamic schedule, 80-register build",
+                  "exact": "the default launch: 256 threads, 3 lines, dynamic schedule, 80-register build"}
 PARITY = {
     "exact": "bit-identical to the oracle (the reference's FP64 CPU path): one step of this "
              "256^3 pack with this launch, 50 steps of 128^3, the refined RT pack over 100 "
@@ -719,8 +719,8 @@ def main():
                                      if traffic else "no capture of this mode's launch",
                      "kernel": "k_stage (batched stage, %s mode)" % args.mode,
                      "stage_ms": stage_ms, "peak_source": peak_kind},
-        "fp64_pipe": {"note": "the FP64 pipe binds this kernel; achieved counts the DADD/DMUL/DFMA "
-                              "it executes (ncu)",
+        "fp64_pipe": {"note": "FP64 issue, integer issue and latencies bind this kernel about evenly; "
+                              "achieved counts the DADD/DMUL/DFMA it executes (ncu)",
                       "peak_source": "2 DFMA lanes/clk/SM x 152 SMs x sampled SM clock"},
         "clocks": clocks,
         "time_check": {"sim_time": status["time"], "ncycle": status["ncycle"]},
