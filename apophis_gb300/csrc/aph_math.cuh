@@ -109,9 +109,11 @@ __device__ __forceinline__ bool tame(double x) {
   const unsigned e = hi >> 20;  // biased exponent
   return (e - (1023u - 200u) <= 400u) | ((hi | (unsigned)__double2loint(x)) == 0u);
 }
-// Zero or 2^-110 <= |x| < 2^111.  From face states in this range the exact Riemann solvers form no
+// Zero or 2^-110 <= |x| < 2^111.  From the face states of such cells the exact Riemann solvers form no
 // product or quotient outside 2^+-1000 as long as their denominators and the few results they
-// check stay within 2^+-400, so their operations need no checks of their own.
+// check stay within 2^+-400, so their other operations need no checks of their own.  The signs of
+// a face's states do not follow from the cells': at a deep trough of positive cells PPM forms
+// negative densities and pressures, whose roots are NaN, so the solvers look at those (positive).
 __device__ __forceinline__ bool snug(double x) {
   const unsigned hi = abs_hi(x);
   return (hi - ((1023u - 110u) << 20) < (221u << 20)) | ((hi | (unsigned)__double2loint(x)) == 0u);
@@ -266,8 +268,9 @@ struct Den {
 
 // Operations of a Riemann solve on the integer pipe, free of branches: far collects the largest
 // distance over the denominators and what else the caller has it see; where that is out of range
-// the solve is taken again with IeeeOps.  Other operands are not checked (snug states).  div0
-// allows a numerator of zero, mul any zeros.
+// the solve is taken again with IeeeOps.  Other operands are not checked (snug states): the caller
+// makes sure that numerators (div) are not zero and radicands are positive.  div0 allows a
+// numerator of zero, mul any zeros.
 struct IntOps {
   static constexpr bool kInt = true;
   unsigned far = 0;
@@ -285,6 +288,13 @@ struct IntOps {
     return is_zero(a) ? __hiloint2double(sg, 0) : q;
   }
   __device__ __forceinline__ double rcp(double b) { return div(1.0, den(b)); }
+  // a value that has to be positive and inside the range, as such and as a denominator
+  __device__ __forceinline__ void positive(double x) { far = max(far, far_of_signed(x)); }
+  __device__ __forceinline__ Den den_positive(double b) {
+    positive(b);
+    return Den{b, rcp_word(significand((unsigned long long)__double_as_longlong(b)))};
+  }
+  __device__ __forceinline__ double rcp_positive(double b) { return div(1.0, den_positive(b)); }
   __device__ __forceinline__ double sqrt(double x) {
     return sqrt_bits((unsigned long long)__double_as_longlong(x));
   }
@@ -356,6 +366,9 @@ struct IeeeOps {
   __device__ __forceinline__ double div(double a, const Den &d) { return __ddiv_rn(a, d.b); }
   __device__ __forceinline__ double div0(double a, const Den &d) { return __ddiv_rn(a, d.b); }
   __device__ __forceinline__ double rcp(double b) { return __drcp_rn(b); }
+  __device__ __forceinline__ void positive(double) {}
+  __device__ __forceinline__ Den den_positive(double b) { return Den{b, 0u}; }
+  __device__ __forceinline__ double rcp_positive(double b) { return __drcp_rn(b); }
   __device__ __forceinline__ double sqrt(double x) { return __dsqrt_rn(x); }
   __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
   __device__ __forceinline__ double half(double x) { return __dmul_rn(0.5, x); }
@@ -866,18 +879,29 @@ __device__ __forceinline__ void gam_plm(int qm, int q0, int qp, int odd, int &ql
 // c-limited sound speed C*sqrt(gamma / (1 + (1/gm1 + rho C^2 / p))) (hydro_hlle.hpp:63-66)
 
 #if APH_EXACT
+// A side's density, pressure and adiabatic indices, all positive with gamma_e above 1: then every
+// radicand of the exact solvers is positive (rho C^2 / p, 1 / (gamma_e - 1) and gamma are; a shock
+// factor is taken where the middle pressure is above p), and no numerator is zero.  Returns
+// 1 / (gamma_e - 1).
 template <class OPS>
-__device__ __forceinline__ double sound_speed(double rho, double p, double gamma, double igm1, OPS &o) {
-  return o.mul(C_LIGHT, o.sqrt(o.div(gamma, o.den(1 + (igm1 + o.div(o.mul(rho, C_LIGHT2), o.den(p)))))));
+__device__ __forceinline__ double see_side(double rho, double gc, double ge, OPS &o) {
+  o.positive(rho);
+  o.positive(gc);
+  return o.rcp_positive(ge - 1);
+}
+template <class OPS>
+__device__ __forceinline__ double sound_speed(double rho, const Den &p, double gamma, double igm1, OPS &o) {
+  return o.mul(C_LIGHT, o.sqrt(o.div(gamma, o.den(1 + (igm1 + o.div(o.mul(rho, C_LIGHT2), p))))));
 }
 
 template <class OPS>
 __device__ __forceinline__ void solve_hlle_exact(const double *wli, const double *wri, double glc,
                                                  double gle, double grc, double gre, double *flxi,
                                                  OPS &o) {
-  const double igm1l = o.rcp(gle - 1), igm1r = o.rcp(gre - 1);
-  const double cl = sound_speed(wli[IDN], wli[IPR], glc, igm1l, o);
-  const double cr = sound_speed(wri[IDN], wri[IPR], grc, igm1r, o);
+  const double igm1l = see_side(wli[IDN], glc, gle, o), igm1r = see_side(wri[IDN], grc, gre, o);
+  const Den pl = o.den_positive(wli[IPR]), pr = o.den_positive(wri[IPR]);
+  const double cl = sound_speed(wli[IDN], pl, glc, igm1l, o);
+  const double cr = sound_speed(wri[IDN], pr, grc, igm1r, o);
   auto energy = [&](const double *w, double igm1) {
     return o.mul(w[IPR], igm1) +
            o.mul(o.half(w[IDN]), o.mul(w[IV1], w[IV1]) + o.mul(w[IV2], w[IV2]) + o.mul(w[IV3], w[IV3]));
@@ -888,9 +912,9 @@ __device__ __forceinline__ void solve_hlle_exact(const double *wli, const double
   const double pmid = o.half(wli[IPR] + wri[IPR] + o.mul(o.mul(wli[IV1] - wri[IV1], rhoa), ca));
   double ql = 1.0, qr = 1.0;
   if (gt(pmid, wli[IPR]))
-    ql = 1.0 + o.mul(o.div(glc + 1, o.den(o.sqrt(o.twice(glc)))), o.div(pmid, o.den(wli[IPR])) - 1.0);
+    ql = 1.0 + o.mul(o.div(glc + 1, o.den(o.sqrt(o.twice(glc)))), o.div(pmid, pl) - 1.0);
   if (gt(pmid, wri[IPR]))
-    qr = 1.0 + o.mul(o.div(grc + 1, o.den(o.sqrt(o.twice(grc)))), o.div(pmid, o.den(wri[IPR])) - 1.0);
+    qr = 1.0 + o.mul(o.div(grc + 1, o.den(o.sqrt(o.twice(grc)))), o.div(pmid, pr) - 1.0);
   const double al = wli[IV1] - o.mul(cl, ql);
   const double ar = wri[IV1] + o.mul(cr, qr);
   const double bp = is_pos(ar) ? ar : 0.0;
@@ -1140,9 +1164,9 @@ __device__ __forceinline__ void solve_hllc_exact(const double *wli, const double
                                                  double gle, double grc, double gre, double *flxi,
                                                  OPS &o) {
   const double gammal = glc, gammar = grc;
-  const double igm1l = o.rcp(gle - 1), igm1r = o.rcp(gre - 1);
+  const double igm1l = see_side(wli[IDN], glc, gle, o), igm1r = see_side(wri[IDN], grc, gre, o);
   // the sound speed and the shock factor divide by the pressures
-  const Den pl = o.den(wli[IPR]), pr = o.den(wri[IPR]);
+  const Den pl = o.den_positive(wli[IPR]), pr = o.den_positive(wri[IPR]);
   const double cl = csound_exact(wli[IDN], pl, gammal, igm1l, o);
   const double cr = csound_exact(wri[IDN], pr, gammar, igm1r, o);
   const double rhoa = o.half(wli[IDN] + wri[IDN]);
