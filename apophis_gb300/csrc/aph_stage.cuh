@@ -295,7 +295,7 @@ __device__ __forceinline__ bool ghost_copy_src(const StageArgs &a, const StepBlo
   if (!p.amr) {  // the uniform block grid's map (ghost_cell)
     bool flip = false;
     const int g = map_index(B.loc[d] * n + c, p.mesh_nx[d], p.bc[d][0], p.bc[d][1], flip);
-    const int sl = quick_div(g, n, B.inv[d][0]);
+    const int sl = wide_div(g, n, B.inv[d][0]);  // (g: an index of the whole mesh)
     int loc[3] = {B.loc[0], B.loc[1], B.loc[2]};
     loc[d] = sl;
     S = &a.blocks[(loc[2] * p.nb[1] + loc[1]) * p.nb[0] + loc[0]];
