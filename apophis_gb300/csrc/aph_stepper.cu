@@ -194,11 +194,21 @@ aph_status upload_items(aph_stepper s, int2 **dst, const std::vector<int2> &v) {
   return e == cudaSuccess ? APH_OK : cuda_fail(e, "stepper items");
 }
 
+// The most shared memory of a stage CTA, and what T lines of n cells take.
+constexpr size_t kStageBytes = 220 * 1024;
+size_t lines_bytes(aph_stepper s, int n, int T) {
+  return s->params.exact ? aph_exact::stage_smem_bytes(s->params.recon, n, T, s->dev.nvar)
+                         : aph_fast::stage_smem_bytes(s->params.recon, n, T, s->dev.nvar);
+}
+
 // Lines of n cells per item: the faces of one round of 256 threads, and two lines where one would
 // leave most of a second line's room empty (2D blocks of 128, exact PPM: 1.46 ms per RK2 step of a
 // 768^2 mesh with two lines, 1.87 with one; at 16 to 96 cells the count for one round is within 2 %
-// of the best).
-int auto_lines(int n) { return n + 2 >= 224 ? 1 : n + 2 >= 128 ? 2 : 256 / (n + 2); }
+// of the best) and two fit (with many scalars they do not).
+int auto_lines(aph_stepper s, int n) {
+  if (n + 2 < 128) return 256 / (n + 2);
+  return n + 2 < 224 && lines_bytes(s, n, 2) <= kStageBytes ? 2 : 1;
+}
 
 void destroy_graph(aph_stepper s) {
   if (s->exec) cudaGraphExecDestroy(s->exec);
@@ -226,7 +236,7 @@ void default_launch(aph_stepper s) {
     c.lines[d] = 0;
     c.order[d] = d + 1;
     if (d >= s->dev.ndim) continue;
-    const int T = auto_lines(s->dev.max_nx[d]);
+    const int T = auto_lines(s, s->dev.max_nx[d]);
     long long items = 0;
     for (const StepBlock &B : s->hblocks) items += (B.nint / B.nx[d] + T - 1) / T;
     most = std::max(most, items);
@@ -307,7 +317,7 @@ size_t stage_lines(aph_stepper s, const int lines[3], bool tma, int T_out[3]) {
   for (int d = 0; d < 3; ++d) T_out[d] = 0;
   for (int d = 0; d < p.ndim; ++d) {
     const int n = p.max_nx[d];
-    int T = lines[d] > 0 ? lines[d] : auto_lines(n);
+    int T = lines[d] > 0 ? lines[d] : auto_lines(s, n);
     int ntr_max = 1;
     for (const StepBlock &B : s->hblocks) {
       const int ntr = d == 0 ? B.nx[1] * B.nx[2] : d == 1 ? B.nx[0] * B.nx[2] : B.nx[0] * B.nx[1];
@@ -319,8 +329,7 @@ size_t stage_lines(aph_stepper s, const int lines[3], bool tma, int T_out[3]) {
     const int nv = p.nvar;
     const size_t need = tma ? (s->params.exact ? aph_exact::stage_smem_bytes_tma(recon, n, T, ext, nv)
                                                : aph_fast::stage_smem_bytes_tma(recon, n, T, ext, nv))
-                            : (s->params.exact ? aph_exact::stage_smem_bytes(recon, n, T, nv)
-                                               : aph_fast::stage_smem_bytes(recon, n, T, nv));
+                            : lines_bytes(s, n, T);
     smem = std::max(smem, need);
   }
   return smem;
@@ -353,11 +362,7 @@ aph_status configure(aph_stepper s) {
   const int nb = p.nblocks;
   // lines per item and shared memory per direction
   const size_t smem = stage_lines(s, s->cfg.lines, s->cfg.tma != 0, s->T);
-  auto smem_of = [&](int n, int T) {
-    return s->params.exact ? aph_exact::stage_smem_bytes(s->params.recon, n, T, p.nvar)
-                           : aph_fast::stage_smem_bytes(s->params.recon, n, T, p.nvar);
-  };
-  if (smem > 220 * 1024)
+  if (smem > kStageBytes)
     return fail(APH_ERR_UNSUPPORTED, "stage needs %zu bytes of shared memory; use fewer lines", smem);
   const int threads = s->cfg.threads;
   int per_sm = stage_residency(s, threads, s->cfg.reg_cap, smem);
@@ -392,7 +397,7 @@ aph_status configure(aph_stepper s) {
       // plain loads: a narrower block takes as many lines per item as the shared memory
       // sized for the widest holds, and its lines are spread evenly over the fewest items
       int Tb = std::min(T, ntr);
-      while (Tb < ntr && Tb + 1 < (1 << kItemLineBits) && smem_of(n, Tb + 1) <= smem) ++Tb;
+      while (Tb < ntr && Tb + 1 < (1 << kItemLineBits) && lines_bytes(s, n, Tb + 1) <= smem) ++Tb;
       const int k = (ntr + Tb - 1) / Tb, base = ntr / k, rem = ntr % k;
       for (int i = 0, l = 0; i < k; ++i) {
         const int lines = base + (i < rem ? 1 : 0);
@@ -1251,7 +1256,7 @@ aph_status aph_stepper_autotune(aph_stepper s, int trial_steps, aph_stepper_conf
         const int lines[3] = {T, T, T};
         int Ts[3];
         const size_t smem = stage_lines(s, lines, tma != 0, Ts);
-        if (smem <= 220 * 1024 && !(tma && tma_unsupported(s, Ts)))
+        if (smem <= kStageBytes && !(tma && tma_unsupported(s, Ts)))
           occ = stage_residency(s, threads, reg_cap, smem);
       }
       if (occ != prev_occ && prev_occ > 0 && prev_occ * threads >= 256) {

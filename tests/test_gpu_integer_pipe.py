@@ -175,3 +175,26 @@ def test_adjoint_outside_the_main_path(recon, rsolver, scale):
     want = adj.step_vjp(u, 2e-3, lam).clone()
     got = adj.step_vjp(u, 2e-3, lam * 2.0 ** scale)
     _same((got * 2.0 ** -scale).cpu().numpy(), want.cpu().numpy())
+
+
+@pytest.mark.parametrize("n,nscalars,exact", [(126, 30, True), (160, 14, True), (200, 10, True), (221, 12, True),
+                                              (221, 12, False)])
+def test_default_lines_with_many_scalars(n, nscalars, exact):
+    """Widths whose default is two lines per item, with more scalars than two lines leave room for: one
+    step equals the oracle (fast mode: it runs)."""
+    from oracle import oracle as O
+    cfg, cons = problems.kh2d(n=n, block=n, ng=3, recon="ppm", rsolver="hllc")
+    cfg, cons = problems.with_tracers(cfg, cons, nscalars)
+    st = Stepper(cfg, cons, exact=exact)
+    st.step(1)
+    sk, sj, si = cfg.interior
+    got = np.ascontiguousarray(st.state()[:, :, sk, sj, si])
+    st.close()
+    ref = O.Mesh(cfg)
+    ref.set_cons(cons)
+    ref.run(nsteps=1)
+    want = np.ascontiguousarray(ref.get()[:, :, sk, sj, si])
+    if exact:
+        _same(got, want)
+    else:
+        assert np.allclose(got, want, rtol=1e-10, atol=1e-10)
