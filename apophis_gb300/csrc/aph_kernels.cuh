@@ -491,12 +491,10 @@ constexpr size_t kSegmentBytes = 200 * 1024;  // the most shared memory of a seg
 template <int DIR, int RECON, int RS, int MINB>
 static cudaError_t launch_segments(const PackDev &p, const BlockDev *blocks, dim3 grid, int nt, size_t smem,
                                    int T, int n, int nseg, cudaStream_t s) {
-  static bool attr_set = false;
-  if (!attr_set) {
+  if (smem > 48 * 1024) {  // the attribute belongs to the device and its context: not kept from one call for the next
     cudaError_t e = cudaFuncSetAttribute(k_fluxes<DIR, RECON, RS, MINB>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSegmentBytes);
     if (e != cudaSuccess) return e;
-    attr_set = true;
   }
   k_fluxes<DIR, RECON, RS, MINB><<<grid, nt, smem, s>>>(p, blocks, T, n, nseg);
   return cudaGetLastError();
