@@ -270,7 +270,7 @@ __device__ __forceinline__ SoundSpeed sound_speed_d(double rho, double p, double
   const double N = o.mul(gc.c2g, p);
   const double D = fma(p, gc.one_igm1, o.mul(rho, C_LIGHT2));
   SoundSpeed s;
-  s.c = o.mul(N, rsqrt(o.mul(N, D)));
+  s.c = o.mul(N, o.rsqrt(o.mul(N, D)));
   const double iD = o.mul(o.mul(s.c, s.c), o.mul(ip, ic2g));
   const double hc = o.half(s.c);
   s.dc_dp = o.mul(hc, fma(-gc.one_igm1, iD, ip));
@@ -403,8 +403,8 @@ __device__ __forceinline__ void hllc_vjp(const double *wl, const double *wr, con
   const bool bl = gt(pstar, pl), br = gt(pstar, pr);
   const double argl = bl ? fma(k, fma(pstar, ipl, -1.0), 1.0) : 1.0;
   const double argr = br ? fma(k, fma(pstar, ipr, -1.0), 1.0) : 1.0;
-  const double iql = bl ? rsqrt(argl) : 1.0;  // q = arg / sqrt(arg), 1/q kept for the reverse
-  const double iqr = br ? rsqrt(argr) : 1.0;
+  const double iql = bl ? o.rsqrt(argl) : 1.0;  // q = arg / sqrt(arg), 1/q kept for the reverse
+  const double iqr = br ? o.rsqrt(argr) : 1.0;
   const double ql = bl ? o.mul(argl, iql) : 1.0;
   const double qr = br ? o.mul(argr, iqr) : 1.0;
   const double sl = fma(-cl, ql, ul);

@@ -350,9 +350,15 @@ struct CheckedOps : IntOps {
   }
 };
 // The fast solvers': an operand of a product is a state value the solver has seen, a product, a
-// quotient or a sum of those, so it is finite and zero or normal, and the exponent of the product
-// tells whether the result is.
+// quotient, a reciprocal root (seen: that of a zero is infinite, and a product with zero would hide
+// it) or a sum of those, so it is finite and zero or normal, and the exponent of the product tells
+// whether the result is.
 struct FaceOps : CheckedOps {
+  __device__ __forceinline__ double rsqrt(double x) {
+    const double r = ::rsqrt(x);
+    far = max(far, far_of(r));
+    return r;
+  }
   __device__ __forceinline__ double mul(double a, double b) {
     unsigned e;
     const double r = product(a, b, e);
@@ -370,6 +376,7 @@ struct IeeeOps {
   __device__ __forceinline__ Den den_positive(double b) { return Den{b, 0u}; }
   __device__ __forceinline__ double rcp_positive(double b) { return __drcp_rn(b); }
   __device__ __forceinline__ double sqrt(double x) { return __dsqrt_rn(x); }
+  __device__ __forceinline__ double rsqrt(double x) { return ::rsqrt(x); }
   __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
   __device__ __forceinline__ double half(double x) { return __dmul_rn(0.5, x); }
   __device__ __forceinline__ double twice(double x) { return __dadd_rn(x, x); }
@@ -960,7 +967,7 @@ __device__ __forceinline__ void sound_parts(double rho, double p, double gamma, 
                                             const GasConsts &gc, double &num, double &root, OPS &o) {
   num = CONSTG ? o.mul(gc.c2g, p) : o.mul(o.mul(C_LIGHT2, gamma), p);
   const double den = fma(p, CONSTG ? gc.one_igm1 : add(1.0, igm1), o.mul(rho, C_LIGHT2));
-  root = rsqrt(o.mul(num, den));  // the speed is num * root
+  root = o.rsqrt(o.mul(num, den));  // the speed is num * root
 }
 template <bool CONSTG, class OPS>
 __device__ __forceinline__ double sound_speed(double rho, double p, double gamma, double igm1,
@@ -1003,8 +1010,8 @@ __device__ __forceinline__ void solve_hlle(const double *wl, const double *wr, d
   const bool bl = gt(pmid, wl[IPR]), br = gt(pmid, wr[IPR]);
   if (bl || br) {
     const double ipp = o.rcp(o.mul(wl[IPR], wr[IPR]));  // shared reciprocal
-    const double kl = CONSTG ? gc.hlle_k : o.mul(add(gl, 1), rsqrt(o.twice(gl)));
-    const double kr = CONSTG ? gc.hlle_k : o.mul(add(gr, 1), rsqrt(o.twice(gr)));
+    const double kl = CONSTG ? gc.hlle_k : o.mul(add(gl, 1), o.rsqrt(o.twice(gl)));
+    const double kr = CONSTG ? gc.hlle_k : o.mul(add(gr, 1), o.rsqrt(o.twice(gr)));
     if (bl) ql = fma(kl, fma(o.mul(pmid, wr[IPR]), ipp, -1.0), 1.0);
     if (br) qr = fma(kr, fma(o.mul(pmid, wl[IPR]), ipp, -1.0), 1.0);
   }

@@ -131,3 +131,87 @@ def test_exact_faces_of_positive_cells_with_troughs(exact, solver):
     got, wrong, first = _count(exact.faces, solver, s)
     assert wrong == 0, (got, wrong, first)
     assert got >= (s[:, [0, 4, 5, 9]] > 0).all(axis=1).sum() * 0.999
+
+
+FAST = COUNT + r"""
+static GasConsts gas() {
+  const double gm1 = 0.4, g = gm1 + 1.0;
+  return GasConsts{gm1, 1.0 / gm1, g, C_LIGHT2 * g, 1.0 + 1.0 / gm1, (g + 1.0) / std::sqrt(2.0 * g), (g + 1.0) / (2.0 * g)};
+}
+template <int RS, bool CONSTG>
+static void run(const double *s, long long n, long long *res) {
+  const GasConsts gc = gas();
+  count<14, 5>(s, n, res, [&](const double *w, double *got, double *want) {
+    const double *g = w + 10;
+    FaceOps o;
+    riemann<RS, CONSTG>(w, w + 5, g[0], g[1], g[2], g[3], gc, got, o);
+    IeeeOps i;
+    riemann<RS, CONSTG>(w, w + 5, g[0], g[1], g[2], g[3], gc, want, i);
+    return o.ok();
+  });
+}
+extern "C" void faces(int rs, const double *s, long long n, long long *res) {
+  if (rs == RS_HLLE) run<RS_HLLE, false>(s, n, res);
+  else if (rs == RS_HLLC) run<RS_HLLC, false>(s, n, res);
+  else run<RS_LHLLC, false>(s, n, res);
+}
+extern "C" void gas_faces(int rs, const double *s, long long n, long long *res) {
+  if (rs == RS_HLLE) run<RS_HLLE, true>(s, n, res);
+  else if (rs == RS_HLLC) run<RS_HLLC, true>(s, n, res);
+  else run<RS_LHLLC, true>(s, n, res);
+}
+// the reverse of a face: states, then the adjoint of its fluxes
+extern "C" void adjoints(int rs, const double *s, long long n, long long *res) {
+  const GasConsts gc = gas();
+  count<15, 10>(s, n, res, [&](const double *w, double *got, double *want) {
+    FaceOps o;
+    IeeeOps i;
+    for (int k = 0; k < 10; ++k) o.see(w[k]);
+    for (int k = 10; k < 15; ++k) o.see(w[k]);
+    if (rs == RS_HLLE) hlle_vjp(w, w + 5, gc, 1.0 / gc.c2g, w + 10, got, got + 5, o), hlle_vjp(w, w + 5, gc, 1.0 / gc.c2g, w + 10, want, want + 5, i);
+    else hllc_vjp(w, w + 5, gc, 1.0 / gc.c2g, w + 10, got, got + 5, o), hllc_vjp(w, w + 5, gc, 1.0 / gc.c2g, w + 10, want, want + 5, i);
+    return o.ok();
+  });
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def fast(tmp_path_factory):
+    return ctypes.CDLL(host_math.build(tmp_path_factory.mktemp("fast"), 0, FAST, ("aph_math.cuh", "aph_adjoint_math.cuh")))
+
+
+def _any_sign(rng, s, col):
+    """One or more of the columns negative, zero or lowered by 1 in each row."""
+    n = len(s)
+    pick = rng.integers(0, 2, (n, col.size)) & rng.integers(0, 2, (n, col.size))
+    pick[np.arange(n), rng.integers(0, col.size, n)] = 1
+    x = s[:, col]
+    s[:, col] = np.where(pick == 1, np.choose(rng.integers(0, 5, x.shape), [-x, -x * 2.0 ** -4, 0.0 * x, -0.0 * x, x - 1.0]), x)
+    rest = rng.integers(0, 4, n) == 0
+    s[rest, 1:4] = s[rest, 6:9] = 0.0
+    return s
+
+
+@pytest.mark.parametrize("which", ["faces", "gas_faces"])
+@pytest.mark.parametrize("solver", [HLLE, HLLC, LHLLC])
+def test_fast_faces_of_any_sign(fast, solver, which):
+    """Zero pressures above all: 0 x rsqrt(0) is NaN."""
+    rng = np.random.default_rng(420 + solver)
+    n = 200_000
+    fn = getattr(fast, which)
+    s = _states(rng, n, 3)
+    assert _count(fn, solver, s)[:2] == (n, 0)
+    col = np.array([0, 4, 5, 9, 10, 11, 12, 13] if which == "faces" else [0, 4, 5, 9])
+    got, wrong, first = _count(fn, solver, _any_sign(rng, s, col))
+    assert wrong == 0, (got, wrong, first)
+
+
+@pytest.mark.parametrize("solver", [HLLE, HLLC])
+def test_adjoint_faces_of_any_sign(fast, solver):
+    rng = np.random.default_rng(430 + solver)
+    n = 200_000
+    s = np.concatenate([_states(rng, n, 3)[:, :10], rng.normal(0.0, 1.0, (n, 5))], axis=1)
+    assert _count(fast.adjoints, solver, s)[:2] == (n, 0)
+    got, wrong, first = _count(fast.adjoints, solver, _any_sign(rng, s, np.array([0, 4, 5, 9])))
+    assert wrong == 0, (got, wrong, first)
