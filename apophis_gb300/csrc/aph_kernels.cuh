@@ -91,12 +91,13 @@ struct Segment {
 };
 
 // How a segment is solved: exact build, gamma offsets (kFluxMain), then double slabs on tame windows
-// (kFluxSlabs); fast build, kFluxSlabs; last, any window with the IEEE instructions.  Returns false
-// where the window or an operand is out of range (nothing but fluxes to be rewritten was stored).
-constexpr int kFluxMain = 0, kFluxSlabs = 1, kFluxIeee = 2;
+// (kFluxSlabs); fast build, kFluxSlabs; last, any window with the IEEE instructions.  Returns kFluxDone,
+// or how to take the segment instead where the window or an operand is out of range (nothing but
+// fluxes to be rewritten was stored): kFluxSlabs where only the adiabatic indices are.
+constexpr int kFluxMain = 0, kFluxSlabs = 1, kFluxIeee = 2, kFluxDone = 3;
 
 template <int DIR, int RECON, int RS, int HOW>
-__device__ __forceinline__ bool flux_segment(const PackDev &p, const BlockDev &B, const Segment &g, int T,
+__device__ __forceinline__ int flux_segment(const PackDev &p, const BlockDev &B, const Segment &g, int T,
                                              const unsigned *inv, double *sm) {
   constexpr int G = Halo<RECON>::G;
   constexpr bool kTame = (APH_EXACT || RECON == RECON_PPM) && HOW != kFluxIeee, kOffsets = HOW == kFluxMain;
@@ -105,7 +106,7 @@ __device__ __forceinline__ bool flux_segment(const PackDev &p, const BlockDev &B
   const long long nc = B.ncell;
   const long long stride = DIR == 1 ? 1 : DIR == 2 ? B.ni : (long long)B.ni * B.nj;
   const Window w = window_regions<RECON>(sm, n, T, V, nvar);
-  bool tame_ok = true;
+  bool tame_ok = true, offset_ok = true;
 #if APH_EXACT
   const long long gbase = __double_as_longlong(p.gamma);
   const int odd = (int)gbase & 1;
@@ -136,7 +137,7 @@ __device__ __forceinline__ bool flux_segment(const PackDev &p, const BlockDev &B
 #if APH_EXACT
     if (kOffsets) {
       const long long kc = __double_as_longlong(gc) - gbase, ke = __double_as_longlong(ge) - gbase;
-      tame_ok = tame_ok & gam_near(kc) & gam_near(ke);
+      offset_ok = offset_ok & gam_near(kc) & gam_near(ke);
       w.GW[t * NW + x0] = gam_pack((int)kc, (int)ke);
     }
 #endif
@@ -147,10 +148,10 @@ __device__ __forceinline__ bool flux_segment(const PackDev &p, const BlockDev &B
     }
   }
 #if APH_EXACT
-  if (kOffsets) tame_ok = tame_ok && gamma_inside(p.gamma);
+  if (kOffsets) offset_ok = offset_ok && gamma_inside(p.gamma);
 #endif
   if (kTame) {
-    if (!__syncthreads_and(tame_ok)) return false;
+    if (!__syncthreads_and(tame_ok & offset_ok)) return kOffsets && __syncthreads_and(tame_ok) ? kFluxSlabs : kFluxIeee;
   } else {
     __syncthreads();
   }
@@ -197,21 +198,22 @@ __device__ __forceinline__ bool flux_segment(const PackDev &p, const BlockDev &B
     for (int v = NHYDRO; v < nvar; ++v)
       out[v * fn] = flx[IDN] * (!is_neg(flx[IDN]) ? w.SL[v * vs + oL] : w.SR[v * vs + oL + 1]);
   }
-  return HOW == kFluxIeee || __syncthreads_and(in_range);
+  return HOW == kFluxIeee || __syncthreads_and(in_range) ? kFluxDone : kFluxIeee;
 }
 
 // A segment whose window left the first arithmetic's range, in chunks of lines that fit the slabs of
 // the adiabatic indices (out of line: it is rare).
 template <int DIR, int RECON, int RS>
 static __device__ __noinline__ void flux_general(const PackDev &p, const BlockDev &B, Segment g, int T,
-                                                 const unsigned *inv, double *sm) {
+                                                 const unsigned *inv, double *sm, int how) {
   const int l0 = g.l0, nl = g.nl;
   const int Tc = APH_EXACT ? max(1, p.nvar * T / (p.nvar + 2)) : T;
   for (int o = 0; o < nl; o += Tc) {
     g.l0 = l0 + o;
     g.nl = min(Tc, nl - o);
     __syncthreads();
-    if (APH_EXACT && flux_segment<DIR, RECON, RS, kFluxSlabs>(p, B, g, Tc, inv, sm)) continue;
+    if (APH_EXACT && how == kFluxSlabs && flux_segment<DIR, RECON, RS, kFluxSlabs>(p, B, g, Tc, inv, sm) == kFluxDone)
+      continue;
     __syncthreads();
     flux_segment<DIR, RECON, RS, kFluxIeee>(p, B, g, Tc, inv, sm);
   }
@@ -234,8 +236,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_fluxes(const __grid_constant
   g.last = g.c0 + g.n == N;
   if (threadIdx.x < 7) inv[threadIdx.x] = 0xffffffffu / (unsigned)(g.n + threadIdx.x) + 1u;
   __syncthreads();
-  if (!flux_segment<DIR, RECON, RS, APH_EXACT ? kFluxMain : kFluxSlabs>(p, B, g, T, inv, sm))
-    flux_general<DIR, RECON, RS>(p, B, g, T, inv, sm);
+  const int how = flux_segment<DIR, RECON, RS, APH_EXACT ? kFluxMain : kFluxSlabs>(p, B, g, T, inv, sm);
+  if (how != kFluxDone) flux_general<DIR, RECON, RS>(p, B, g, T, inv, sm, how);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -447,6 +447,11 @@ __device__ __forceinline__ void line_of(const StepBlock &B, int ndim, int ng, in
 //   ARITH_IEEE   any window: the IEEE instructions
 // An item whose window or operands leave ARITH_MAIN's range is taken again with one of the
 // others, in chunks of lines that fit the two more slabs (split_lines).
+// What that costs (KH 1024^2, RK2, ms a step; in brackets all on the FP64 pipe with tame forms): PPM +
+// HLLC 2.29 with every item ARITH_MAIN [9.18], 4.09 where a velocity tail takes a quarter of the cells
+// through 2^-110 .. 2^-200 [9.21], 7.61 where all cells lie there [9.19]; PLM + HLLE 1.88 [4.82], 2.64
+// [4.87], 3.94 [4.87].  The per-kernel fluxes go the same way (per-kernel step, PLM + HLLE: 1.78 [3.70],
+// 2.48 [3.73], 3.71 [3.74]).
 constexpr int ARITH_MAIN = 0, ARITH_SLABS = 1, ARITH_IEEE = 2;
 constexpr int ITEM_DONE = 0, ITEM_TIMEOUT = 1, ITEM_SLABS = 2, ITEM_IEEE = 3;
 
@@ -615,7 +620,8 @@ __device__ __forceinline__ int pass_item(const StageArgs &a, const StepBlock &B,
   }
 #if APH_EXACT
   if (kOffsets) {
-    if (!__syncthreads_and(tame_ok && offset_ok && gamma_inside(gc.gamma))) return ITEM_SLABS;
+    if (!__syncthreads_and(tame_ok && offset_ok && gamma_inside(gc.gamma)))
+      return __syncthreads_and(tame_ok) ? ITEM_SLABS : ITEM_IEEE;  // (slabs of doubles help the indices only)
   } else if (kTame) {
     if (!__syncthreads_and(tame_ok)) return ITEM_IEEE;
   } else {
