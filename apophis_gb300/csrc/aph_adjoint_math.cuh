@@ -257,8 +257,8 @@ __device__ __forceinline__ void ppm_cell_vjp(double q_i, double dph_lo, double d
 // The adjoint passes are bound by the FP64 pipe, so the reverse forms neither the fluxes (their
 // products with the adjoint are sums it needs anyway) nor a factor twice, and its plain products
 // take the integer pipe (OPS = FaceOps); every fused one is named.  The PLM + HLLE pass held the
-// FP64 pipe for 384 instructions a zone, 78 % of its cycles, before; the forward and backward of
-// a 512^2 rollout with it went from 7.94 to 7.18 ms.
+// FP64 pipe for 384 warp instructions per 32 zones, 78 % of its cycles, before (now 245 and 66 %); the
+// forward and backward of a 512^2 rollout with it went from 7.94 to 7.18 ms.
 struct SoundSpeed {
   double c, dc_dp, dc_drho;
 };
